@@ -262,6 +262,12 @@ __global__ void k_colgrad_sq(const double* c, const double* b, int m, double* ou
 
 }  // namespace
 
+}  // namespace regot
+
+#include "bcd_scaled.cuh"
+
+namespace regot {
+
 void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int max_iter,
                       const regot_opts& o, regot_result* res) {
     cudaStream_t st = ctx->stream;
@@ -290,21 +296,54 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
     BcdState* S = dst.get();
     double* mx = scratch.get();
 
+    // FP64: sweeps on the stored plan (bcd_scaled.cuh), where its launch and
+    // its memory (the size of M once more) fit.
+    const long long ldk = ((long long)m + 1) & ~1LL;
+    ScaledPlan sp;
+    DBuf<double> K, spart, sbuf;
+    bool scaled = !mixed && (double)n * ldk * sizeof(double) <= kScaledMaxBytes;
+    for (int i = 0; scaled && i < n; ++i) scaled = P->ha[i] >= kMinMarginal;
+    for (int j = 0; scaled && j < m; ++j) scaled = P->hb[j] >= kMinMarginal;
+    if (scaled) {
+        sp = scaled_plan(n, m, ldk);
+        scaled = sp.ok;
+    }
+    if (scaled) {
+        try {
+            K.alloc((size_t)n * ldk, st);
+            spart.alloc((size_t)sp.blocks * ldk, st);
+            // v, red, blast, redf, count
+            sbuf.alloc((size_t)ldk + 5 * (size_t)sp.blocks + 4, st);
+        } catch (const Error&) {  // no room for a second matrix: the passes below
+            cudaGetLastError();
+            K.release();
+            spart.release();
+            scaled = false;
+        }
+    }
+
     // Initial value (sinkhorn_bcd.cpp:38-47).
     const bool has_x0 = o.x0 && o.x0_len == n + m - 1;
+    const bool scaled_start = scaled && !has_x0;
     if (has_x0) {
         std::vector<double> hb(m, 0.0);
         std::copy(o.x0 + n, o.x0 + n + m - 1, hb.begin());
         h2d(alpha.get(), o.x0, n * sizeof(double), st);
         h2d(beta.get(), hb.data(), m * sizeof(double), st);
+    } else if (scaled_start) {
+        // beta's sums are the first products of the sweep kernel
+        alpha.zero();
+        ops.col_anchor(alpha.get(), beta.get(), mx);
     } else {
         alpha.zero();
         ops.optimal_beta(alpha.get(), beta.get(), mx);
     }
     // Timer starts after the initial value (sinkhorn_bcd.cpp:49-51).
-    k_bcd_init<<<std::min(cdiv((long long)n + m, 256), 64), 256, 0, st>>>(
-        P->b, alpha.get(), n, beta.get(), m, parts.get(), S);
-    count_launch();
+    if (!scaled_start) {
+        k_bcd_init<<<std::min(cdiv((long long)n + m, 256), 64), 256, 0, st>>>(
+            P->b, alpha.get(), n, beta.get(), m, parts.get(), S);
+        count_launch();
+    }
     if (has_x0) {
         // With a user x0 the beta part of the first gradient is not zero.
         ops.row_col_sums(alpha.get(), beta.get(), rsum.get(), csum.get(), mx);
@@ -335,6 +374,133 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
     };
     const int gn = cdiv(n, kFinItems), gm = cdiv(m, kFinItems), gnm = cdiv(std::max(n, m), 256);
 
+    // ---- general path's pieces: split before each pass, commit after each sweep ----
+    PassParams p1 = ops.base_params();
+    p1.grid = &S->maxabs;
+    p1.done = &S->done;
+    PassParams p2 = p1;
+    // K1: anchor alpha_k, column dual beta_k
+    p1.ra = alpha.get();
+    p1.cb = beta.get();
+    // K2: row dual alpha_{k+1}, anchor beta_k
+    p2.ra = alpha_next.get();
+    p2.cb = beta.get();
+
+    auto launch_row = [&](const double* anc, int robust) {
+        if (mixed)
+            k_bcd_row<float, true><<<gn, kFinBlock, 0, st>>>(
+                (const float*)ops.buf().rowpart.get(), sh.nslabs, n, anc, alpha.get(), P->a,
+                ops.loga(), reg, ops.sum_a(), ops.sum_bt(), alpha_next.get(), hobj, hmar,
+                htime, parts.get(), S, robust, SplitOut());
+        else
+            k_bcd_row<double, false><<<gn, kFinBlock, 0, st>>>(
+                (const double*)ops.buf().rowpart.get(), sh.nslabs, n, anc, alpha.get(), P->a,
+                ops.loga(), reg, ops.sum_a(), ops.sum_bt(), alpha_next.get(), hobj, hmar,
+                htime, parts.get(), S, robust, SplitOut());
+        count_launch();
+    };
+    auto launch_col = [&](const double* anc, int robust) {
+        if (mixed)
+            k_bcd_col<float, true><<<gm, kFinBlock, 0, st>>>(
+                (const float*)ops.buf().colpart.get(), sh.nrb, m, anc, ops.logb(), P->b, reg,
+                beta_next.get(), parts.get(), S, robust, SplitOut(), 0);
+        else
+            k_bcd_col<double, false><<<gm, kFinBlock, 0, st>>>(
+                (const double*)ops.buf().colpart.get(), sh.nrb, m, anc, ops.logb(), P->b,
+                reg, beta_next.get(), parts.get(), S, robust, SplitOut(), 0);
+        count_launch();
+    };
+    auto launch_commit = [&]() {
+        k_bcd_commit<<<gnm, 256, 0, st>>>(n, m, alpha.get(), alpha_next.get(), beta.get(),
+                                          beta_next.get(), S);
+        count_launch();
+    };
+    auto sweep = [&]() {
+        ops.pass(OP_E_ROW, p1);
+        launch_row(alpha.get(), 0);
+        ops.pass(OP_E_COL, p2);
+        launch_col(beta.get(), 0);
+        launch_commit();
+    };
+    // Robust redo of the half-sweep that left the safe range.
+    auto robust = [&](int which) {
+        const int zero = 0;
+        h2d(&S->bad, &zero, sizeof(int), st);
+        h2d(&S->done, &zero, sizeof(int), st);
+        PassParams pr = ops.base_params();
+        pr.grid = &S->maxabs;
+        if (which & 1) {
+            // alpha_{k+1} with an explicit max anchor, then the row sums of
+            // iterate k measured against it.
+            ops.optimal_alpha(beta.get(), anchor.get(), mx);
+            ops.maxabs(anchor.get(), n, beta.get(), m, &S->maxabs);
+            pr.ra = anchor.get();
+            pr.cb = beta.get();
+            ops.pass(OP_E_ROW, pr);
+            launch_row(anchor.get(), 1);
+            ops.maxabs(alpha_next.get(), n, beta.get(), m, &S->maxabs);
+            ops.pass(OP_E_COL, p2);
+            launch_col(beta.get(), 0);
+            launch_commit();
+        } else {
+            // beta_{k+1} with an explicit max anchor.
+            ops.optimal_beta(alpha_next.get(), anchor.get(), mx);
+            ops.maxabs(alpha_next.get(), n, anchor.get(), m, &S->maxabs);
+            pr.ra = alpha_next.get();
+            pr.cb = anchor.get();
+            ops.pass(OP_E_COL, pr);
+            launch_col(anchor.get(), 1);
+            launch_commit();
+        }
+        REGOT_CHECK_LAUNCH();
+        read_state();
+        if (hs.bad) throw Error(REGOT_ERR_NONFINITE, "non-finite row or column sums in BCD");
+    };
+
+    // ---- FP64: sweeps on the stored plan ----
+    if (scaled) {
+        ScaledParams q{};
+        q.K = K.get();
+        q.ldk = ldk;
+        q.n = n;
+        q.m = m;
+        q.a = P->a;
+        q.b = P->b;
+        q.alpha = alpha.get();
+        q.beta = beta.get();
+        q.alpha_next = alpha_next.get();
+        q.reg = reg;
+        q.sum_a = ops.sum_a();
+        q.sum_bt = ops.sum_bt();
+        q.part = spart.get();
+        q.red = sbuf.get();
+        q.vbuf = q.red + 4 * (size_t)sp.blocks;
+        q.blast = q.vbuf + ldk;
+        q.redf = reinterpret_cast<int*>(q.blast + 1);
+        q.count = reinterpret_cast<unsigned*>(q.blast + 3 + sp.blocks / 2);
+        q.err = ops.err_flag();
+        q.st = S;
+        q.hobj = hobj;
+        q.hmar = hmar;
+        q.htime = htime;
+        q.first_col = scaled_start ? 1 : 0;
+        // Every launch advances at least one sweep, and so does every robust
+        // half-sweep, so the loop ends with the iterations.
+        for (long long launched = 0; !hs.done; ++launched) {
+            if (launched > 2LL * max_iter + 64)
+                throw Error(REGOT_ERR_NUMERIC, "BCD did not terminate");
+            launch_plan64(static_cast<const double*>(P->M), P->ldm, n, m, alpha.get(), beta.get(),
+                          reg, K.get(), ldk, q.count, st);
+            launch_scaled(sp, q, st);
+            REGOT_CHECK_LAUNCH();
+            read_state();
+            if (hs.done) break;
+            ops.check_err();
+            q.first_col = 0;
+            if (hs.bad) robust(hs.bad);
+        }
+    }
+
     // ---- ping-pong path: 4 kernels per sweep ----
     // The duals alternate between (alpha, beta) for even iterates and
     // (alpha_next, beta_next) for odd ones, so no commit kernel is needed, and
@@ -345,7 +511,7 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
     // general path below, which re-splits before every pass.
     int pending = 0;  // robust column half-sweep owed to the general path
     bool finished = false;
-    {
+    if (!scaled) {
         // The grid comes from the initial duals on the device, so the graph
         // below is captured while the initialisation still runs.
         float4* rs = const_cast<float4*>(ops.rsplit());
@@ -459,89 +625,8 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
         }
     }
 
-    // ---- general path: split before each pass, commit after each sweep ----
-    if (!finished) {
-        PassParams p1 = ops.base_params();
-        p1.grid = &S->maxabs;
-        p1.done = &S->done;
-        PassParams p2 = p1;
-        // K1: anchor alpha_k, column dual beta_k
-        p1.ra = alpha.get();
-        p1.cb = beta.get();
-        // K2: row dual alpha_{k+1}, anchor beta_k
-        p2.ra = alpha_next.get();
-        p2.cb = beta.get();
-
-        auto launch_row = [&](const double* anc, int robust) {
-            if (mixed)
-                k_bcd_row<float, true><<<gn, kFinBlock, 0, st>>>(
-                    (const float*)ops.buf().rowpart.get(), sh.nslabs, n, anc, alpha.get(), P->a,
-                    ops.loga(), reg, ops.sum_a(), ops.sum_bt(), alpha_next.get(), hobj, hmar,
-                    htime, parts.get(), S, robust, SplitOut());
-            else
-                k_bcd_row<double, false><<<gn, kFinBlock, 0, st>>>(
-                    (const double*)ops.buf().rowpart.get(), sh.nslabs, n, anc, alpha.get(), P->a,
-                    ops.loga(), reg, ops.sum_a(), ops.sum_bt(), alpha_next.get(), hobj, hmar,
-                    htime, parts.get(), S, robust, SplitOut());
-            count_launch();
-        };
-        auto launch_col = [&](const double* anc, int robust) {
-            if (mixed)
-                k_bcd_col<float, true><<<gm, kFinBlock, 0, st>>>(
-                    (const float*)ops.buf().colpart.get(), sh.nrb, m, anc, ops.logb(), P->b, reg,
-                    beta_next.get(), parts.get(), S, robust, SplitOut(), 0);
-            else
-                k_bcd_col<double, false><<<gm, kFinBlock, 0, st>>>(
-                    (const double*)ops.buf().colpart.get(), sh.nrb, m, anc, ops.logb(), P->b,
-                    reg, beta_next.get(), parts.get(), S, robust, SplitOut(), 0);
-            count_launch();
-        };
-        auto launch_commit = [&]() {
-            k_bcd_commit<<<gnm, 256, 0, st>>>(n, m, alpha.get(), alpha_next.get(), beta.get(),
-                                              beta_next.get(), S);
-            count_launch();
-        };
-        auto sweep = [&]() {
-            ops.pass(OP_E_ROW, p1);
-            launch_row(alpha.get(), 0);
-            ops.pass(OP_E_COL, p2);
-            launch_col(beta.get(), 0);
-            launch_commit();
-        };
-        // Robust redo of the half-sweep that left the safe range.
-        auto robust = [&](int which) {
-            const int zero = 0;
-            h2d(&S->bad, &zero, sizeof(int), st);
-            h2d(&S->done, &zero, sizeof(int), st);
-            PassParams pr = ops.base_params();
-            pr.grid = &S->maxabs;
-            if (which & 1) {
-                // alpha_{k+1} with an explicit max anchor, then the row sums of
-                // iterate k measured against it.
-                ops.optimal_alpha(beta.get(), anchor.get(), mx);
-                ops.maxabs(anchor.get(), n, beta.get(), m, &S->maxabs);
-                pr.ra = anchor.get();
-                pr.cb = beta.get();
-                ops.pass(OP_E_ROW, pr);
-                launch_row(anchor.get(), 1);
-                ops.maxabs(alpha_next.get(), n, beta.get(), m, &S->maxabs);
-                ops.pass(OP_E_COL, p2);
-                launch_col(beta.get(), 0);
-                launch_commit();
-            } else {
-                // beta_{k+1} with an explicit max anchor.
-                ops.optimal_beta(alpha_next.get(), anchor.get(), mx);
-                ops.maxabs(alpha_next.get(), n, anchor.get(), m, &S->maxabs);
-                pr.ra = alpha_next.get();
-                pr.cb = anchor.get();
-                ops.pass(OP_E_COL, pr);
-                launch_col(anchor.get(), 1);
-                launch_commit();
-            }
-            REGOT_CHECK_LAUNCH();
-            read_state();
-            if (hs.bad) throw Error(REGOT_ERR_NONFINITE, "non-finite row or column sums in BCD");
-        };
+    // ---- general path ----
+    if (!scaled && !finished) {
         if (pending) robust(pending);
 
         cudaGraph_t graph = nullptr;

@@ -1,4 +1,5 @@
 // EROT building blocks (see erot_ops.cuh).
+#include <algorithm>
 #include <cmath>
 
 #include "erot_ops.cuh"
@@ -91,7 +92,57 @@ __global__ void k_sum_totals(const double* totpart, int nblocks, int nt, double*
     out[t] = acc;
 }
 
+// out_ij = exp((alpha_i + beta_j - M_ij) / reg), row stride ldo, zero in the
+// columns m .. ldo - 1; *zero = 0 (the counter of a barrier that a later
+// kernel uses). One FP64 exponential an entry (about twenty FP64 operations at
+// two a clock and SM) bounds it, so the entries are spread over all SMs
+// whatever the shape: the tiles of the dense pass give 64 x 256 entries to one
+// SM, 190 us at 1000 x 800, of which this kernel needs a quarter. VEC: pairs of
+// columns, where out and the rows of both matrices start on 16 bytes.
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_plan64(const double* __restrict__ M, long long ldm, int n,
+                                                int m, const double* __restrict__ alpha,
+                                                const double* __restrict__ beta, double kexp,
+                                                double* out, long long ldo, unsigned* zero) {
+    constexpr int W = VEC ? 2 : 1;
+    if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;
+    const long long per_row = ldo / W, total = n * per_row;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
+         t += (long long)gridDim.x * blockDim.x) {
+        const long long i = t / per_row;
+        const int j = W * (int)(t - i * per_row);
+        const double al = alpha[i];
+        const double* src = M + i * ldm + j;
+        if constexpr (VEC) {
+            double2 q = make_double2(0.0, 0.0);
+            if (j < m) {  // ldm is even: the second column may be padding
+                const double2 c = *reinterpret_cast<const double2*>(src);
+                q.x = exp(((al + beta[j]) - c.x) * kexp);
+                if (j + 1 < m) q.y = exp(((al + beta[j + 1]) - c.y) * kexp);
+            }
+            *reinterpret_cast<double2*>(out + i * ldo + j) = q;
+        } else {
+            out[i * ldo + j] = j < m ? exp(((al + beta[j]) - *src) * kexp) : 0.0;
+        }
+    }
+}
+
 }  // namespace
+
+void launch_plan64(const double* M, long long ldm, int n, int m, const double* alpha,
+                   const double* beta, double reg, double* out, long long ldo, unsigned* zero,
+                   cudaStream_t st) {
+    const bool vec = ldo % 2 == 0 && ldm % 2 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(M)) & 15) == 0;
+    const long long items = (long long)n * (vec ? ldo / 2 : ldo);
+    const int blocks = (int)std::min<long long>((items + 255) / 256, 8LL * device_sm_count());
+    if (vec)
+        k_plan64<true><<<blocks, 256, 0, st>>>(M, ldm, n, m, alpha, beta, 1.0 / reg, out, ldo, zero);
+    else
+        k_plan64<false><<<blocks, 256, 0, st>>>(M, ldm, n, m, alpha, beta, 1.0 / reg, out, ldo, zero);
+    count_launch();
+    REGOT_CHECK_LAUNCH();
+}
 
 ErotOps::ErotOps(regot_dproblem* P, double reg, cudaStream_t st)
     : P_(P), st_(st), n_(P->n), m_(P->m), mixed_(P->prec == REGOT_PREC_MIXED), reg_(reg) {
@@ -196,14 +247,21 @@ void ErotOps::merge_cols(int nc, double* out) {
 // sinkhorn_problem_bcd.cpp:149-174: beta_j = reg (log b_j - LSE_i (alpha_i - M_ij)/reg),
 // evaluated as anchor_j + reg (log b_j - log sum_i exp((alpha_i + anchor_j - M_ij)/reg))
 // with anchor_j = -max_i (alpha_i - M_ij), so no term exceeds 1.
-void ErotOps::optimal_beta(const double* alpha, double* beta, double* mx) {
+void ErotOps::col_anchor(const double* alpha, double* anchor, double* mx) {
     PassParams p = base_params();
     p.ra = alpha;
     maxabs(alpha, n_, nullptr, 0, mx);
     p.grid = mx;
     pass(OP_E_COLMAX, p);
     // mx = max(|alpha|, |anchor|): the anchor kernel raises max |alpha|
-    REGOT_LAUNCH_ACC(k_col_anchor, m_, buf_.colpart.get(), buf_.shape.nrb, m_, anchor_.get(), mx);
+    REGOT_LAUNCH_ACC(k_col_anchor, m_, buf_.colpart.get(), buf_.shape.nrb, m_, anchor, mx);
+}
+
+void ErotOps::optimal_beta(const double* alpha, double* beta, double* mx) {
+    col_anchor(alpha, anchor_.get(), mx);
+    PassParams p = base_params();
+    p.ra = alpha;
+    p.grid = mx;
     p.cb = anchor_.get();
     pass(OP_E_COL, p);
     REGOT_LAUNCH_ACC(k_col_lse, m_, buf_.colpart.get(), buf_.shape.nrb, m_, anchor_.get(),
@@ -290,6 +348,11 @@ void ErotOps::avg_plan(const double* alpha, const double* beta, void* X, double 
 }
 
 void ErotOps::plan(const double* alpha, const double* beta, double* out, double* mx) {
+    if (!mixed_) {
+        launch_plan64(static_cast<const double*>(P_->M), P_->ldm, n_, m_, alpha, beta, reg_, out, m_,
+                      nullptr, st_);
+        return;
+    }
     PassParams p = base_params();
     p.ra = alpha;
     p.cb = beta;

@@ -26,6 +26,12 @@ struct PassBuffers {
     }
 };
 
+// FP64 plan exp((alpha_i + beta_j - M_ij) / reg) into out (row stride ldo >= m,
+// the columns from m on zero); *zero = 0 when zero is not null.
+void launch_plan64(const double* M, long long ldm, int n, int m, const double* alpha,
+                   const double* beta, double reg, double* out, long long ldo, unsigned* zero,
+                   cudaStream_t st);
+
 // Engine bound to one device problem and one regularisation value.
 class ErotOps {
 public:
@@ -68,6 +74,8 @@ public:
     // Maximum of |x| over up to two device vectors, into *out (device).
     void maxabs(const double* x, int nx, const double* y, int ny, double* out);
 
+    // anchor_j = -max_i (alpha_i - M_ij); *maxabs_scratch = max |alpha|, |anchor|.
+    void col_anchor(const double* alpha, double* anchor, double* maxabs_scratch);
     // beta = optimal_beta(alpha) (robust: column max anchor, then sums).
     void optimal_beta(const double* alpha, double* beta, double* maxabs_scratch);
     // alpha = optimal_alpha(beta).

@@ -1,0 +1,70 @@
+// Barrier of a kernel whose blocks wait on one another: all blocks of a
+// cooperative launch (one counter in global memory), or the blocks of one
+// thread-block cluster (the hardware's cluster barrier). Both order global
+// memory: what a block wrote before it arrived is seen, through L2 (__ldcg),
+// by every block after it waited.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace regot {
+
+// Polls of the grid barrier before it gives up (each a round trip to L2,
+// about a microsecond: some seconds in all).
+constexpr unsigned kGridSpins = 1u << 22;
+
+template <bool CLUSTER>
+struct GridBarrier;
+
+// count starts at 0 and only grows; generation g is complete at g * gridDim.x
+// arrivals. *err is set when a wait gives up; every later wait returns false
+// at once then, so all blocks leave within one limit.
+template <>
+struct GridBarrier<false> {
+    unsigned* count;
+    int* err;
+    unsigned target;
+    int* s_ok;  // one int of shared memory
+
+    __device__ GridBarrier(unsigned* c, int* e, int* s) : count(c), err(e), target(0), s_ok(s) {}
+    __device__ void arrive() {
+        __syncthreads();
+        target += gridDim.x;
+        if (threadIdx.x == 0)
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    }
+    __device__ bool wait() {
+        if (threadIdx.x == 0) {
+            int ok = 0;
+            for (unsigned s = 0; s < kGridSpins; ++s) {
+                unsigned c;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+                if ((int)(c - target) >= 0) {
+                    ok = 1;
+                    break;
+                }
+                if ((s & 1023u) == 1023u && *(volatile int*)err) break;
+            }
+            if (!ok) atomicOr(err, 1);
+            *s_ok = ok;
+        }
+        __syncthreads();
+        return *s_ok != 0;
+    }
+};
+
+template <>
+struct GridBarrier<true> {
+    __device__ GridBarrier(unsigned*, int*, int*) {}
+    __device__ void arrive() {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    __device__ bool wait() {
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
+};
+
+}  // namespace regot
