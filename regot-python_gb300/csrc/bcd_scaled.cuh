@@ -27,7 +27,6 @@ namespace {
 constexpr int kScaleLim = 100;   // scalings stay within 2^-100 .. 2^100
 constexpr int kSumLim = 896;     // sums within 2^-896 .. 2^896 are exact enough
 constexpr double kMinMarginal = 1e-150;
-constexpr double kScaledMaxBytes = 32.0 * (1ULL << 30);
 
 struct ScaledParams {
     const double* K;
@@ -280,82 +279,29 @@ __global__ void __launch_bounds__(kResThreads, 1) k_bcd_scaled(const ScaledParam
         p.beta[j] += p.reg * log(colbad ? s_vp[j - j0] : s_v[j]);
 }
 
-// Launch shape of the sweeps: one cluster of 16 blocks for problems whose
-// products are short against a barrier of the whole grid, else a block an SM.
+// Launch shape of the sweeps: one cluster for problems whose products are
+// short against a barrier of the whole grid, else a block an SM.
 struct ScaledPlan {
     bool ok = false, cluster = false;
     int blocks = 0;
     size_t smem = 0;
 };
 
-// Problems of at most this many entries run in one cluster.
-constexpr long long kClusterEntries = 64 * 1024;
-
 inline ScaledPlan scaled_plan(int n, int m, long long ldk) {
     ScaledPlan s;
-    int dev = 0, optin = 0, coop = 0;
-    REGOT_CUDA(cudaGetDevice(&dev));
-    REGOT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    REGOT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if ((long long)n * m <= kClusterEntries) {
-        s.smem = scaled_smem(n, ldk, m, 16);
-        if (s.smem + 1024 <= (size_t)optin &&
-            cudaFuncSetAttribute(k_bcd_scaled<true>, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                 1) == cudaSuccess &&
-            cudaFuncSetAttribute(k_bcd_scaled<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)s.smem) == cudaSuccess) {
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 16;
-            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-            cfg.gridDim = dim3(16);
-            cfg.blockDim = dim3(kResThreads);
-            cfg.dynamicSmemBytes = s.smem;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, k_bcd_scaled<true>, &cfg) == cudaSuccess &&
-                clusters > 0) {
-                s.ok = s.cluster = true;
-                s.blocks = 16;
-                return s;
-            }
-        }
-        cudaGetLastError();
-    }
+    s.blocks = 16;
+    s.smem = scaled_smem(n, ldk, m, s.blocks);
+    s.ok = s.cluster = resident_cluster(k_bcd_scaled<true>, (long long)n * m, s.smem);
+    if (s.ok) return s;
     s.blocks = n < device_sm_count() ? n : device_sm_count();
     s.smem = scaled_smem(n, ldk, m, s.blocks);
-    if (!coop || s.smem + 1024 > (size_t)optin) return s;
-    REGOT_CUDA(cudaFuncSetAttribute(k_bcd_scaled<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)s.smem));
-    int occ = 0;
-    REGOT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bcd_scaled<false>, kResThreads,
-                                                             s.smem));
-    s.ok = occ >= 1;
+    s.ok = resident_grid(k_bcd_scaled<false>, s.smem);
     return s;
 }
 
-inline void launch_scaled(const ScaledPlan& s, ScaledParams& p, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    if (s.cluster) {
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)s.blocks;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    } else {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-    }
-    cfg.gridDim = dim3(s.blocks);
-    cfg.blockDim = dim3(kResThreads);
-    cfg.dynamicSmemBytes = s.smem;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (s.cluster) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_bcd_scaled<true>, p));
-    else REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_bcd_scaled<false>, p));
-    count_launch();
+inline void launch_scaled(const ScaledPlan& s, const ScaledParams& p, cudaStream_t st) {
+    launch_resident(s.cluster ? k_bcd_scaled<true> : k_bcd_scaled<false>, s.cluster, s.blocks, s.smem,
+                    st, p);
 }
 
 }  // namespace

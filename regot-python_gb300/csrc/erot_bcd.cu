@@ -301,7 +301,7 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
     const long long ldk = ((long long)m + 1) & ~1LL;
     ScaledPlan sp;
     DBuf<double> K, spart, sbuf;
-    bool scaled = !mixed && (double)n * ldk * sizeof(double) <= kScaledMaxBytes;
+    bool scaled = !mixed && (double)n * ldk * sizeof(double) <= kPlanMaxBytes;
     for (int i = 0; scaled && i < n; ++i) scaled = P->ha[i] >= kMinMarginal;
     for (int j = 0; scaled && j < m; ++j) scaled = P->hb[j] >= kMinMarginal;
     if (scaled) {

@@ -249,6 +249,91 @@ __global__ void k_ls_totals(const double* totpart, int nblocks, int nsteps, doub
 
 }  // namespace
 
+}  // namespace regot
+
+#include "newton_plan.cuh"
+
+namespace regot {
+
+namespace {
+
+// The FP64 solver on the stored plan: gradient, CG and full-step line search
+// of an iterate are launched together and read back once.
+void newton_on_plan(regot_ctx* ctx, regot_dproblem* P, ErotOps& ops, PlanCgLaunch& L, double tol,
+                    int max_iter, double cg_tol, double* gamma, const regot_opts& o, double* hist,
+                    int hist_cap, double* parts, NewtonState* S, int* niter, int* hist_len,
+                    long long* passes) {
+    cudaStream_t st = ctx->stream;
+    const int n = P->n, m = P->m, N = n + m;
+    constexpr double theta = 0.5, kappa = 0.5;  // sinkhorn_newton.cpp:29-30
+    constexpr int nlinesearch = 20;
+    DBuf<double> g(N, st), x(N, st), lsout(4, st);
+    x.zero();
+    L.p.gamma = gamma;
+    L.p.rhs = nullptr;
+    L.p.grad_tol = tol;
+    L.p.cg_tol = cg_tol;
+    L.p.g = g.get();
+    L.p.x = x.get();
+    const int gv = cdiv(N, kVecThreads);
+    const double full[4] = {1.0, 0.0, 0.0, 0.0};
+    NewtonState hs{};
+    int i = 0;
+    for (;; i++) {
+        L.p.hobj = hist + i;
+        L.p.hmar = hist + hist_cap + i;
+        L.p.htime = hist + 2 * (size_t)hist_cap + i;
+        // at max_iter the iterate is recorded and not left again
+        if (i == max_iter) L.p.grad_tol = INFINITY;
+        L.form_plan(P, gamma, st);
+        L.solve(st);
+        k_dir_dots<<<gv, kVecThreads, 0, st>>>(n, m, g.get(), x.get(), P->a, P->b, parts, S);
+        count_launch();
+        L.line_search(x.get(), full, 1, lsout.get(), st);
+        double tots[4];
+        d2h(tots, lsout.get(), sizeof(double), st);
+        read_small(ctx, &hs, S, sizeof(hs), st);
+        if (!hs.cg_done) ops.check_err();
+        *passes += 1;
+        if (i == max_iter) break;
+        if (o.verbose >= 1)
+            std::printf("iter = %d, objval = %g, ||grad|| = %g\n", i, hs.f, hs.gnorm);
+        if (hs.cg_done == 2) break;  // sinkhorn_newton.cpp:87-88
+        *passes += hs.cg_it + 1;
+        const double thresh = theta * hs.gtd;
+        double step = 1.0, accepted = -1.0;
+        for (int k0 = 0; k0 < nlinesearch && accepted < 0.0;) {
+            const int ns = std::min(k0 == 0 ? 1 : 4, nlinesearch - k0);
+            double steps[4] = {0, 0, 0, 0};
+            for (int s = 0; s < ns; ++s) steps[s] = step * std::pow(kappa, s);
+            if (k0 > 0) {  // the full step alone is evaluated already
+                L.line_search(x.get(), steps, ns, lsout.get(), st);
+                ++*passes;
+                d2h(tots, lsout.get(), ns * sizeof(double), st);
+                sync(st);
+            }
+            k0 += ns;
+            for (int s = 0; s < ns; ++s) {
+                const double df = steps[s] * hs.gtd + ops.reg() * tots[s];
+                if (df <= steps[s] * thresh) {  // newf <= f + step * thresh
+                    accepted = steps[s];
+                    break;
+                }
+            }
+            step = steps[ns - 1] * kappa;
+        }
+        // Without an acceptable step the reference keeps the last trial
+        // (step = kappa^19).
+        if (accepted < 0.0) accepted = std::pow(kappa, nlinesearch - 1);
+        k_axpy_gamma<<<gv, kVecThreads, 0, st>>>(N, accepted, x.get(), gamma, S);
+        count_launch();
+    }
+    *niter = i;
+    *hist_len = i + 1;
+}
+
+}  // namespace
+
 void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int max_iter,
                          const regot_opts& o, regot_result* res) {
     cudaStream_t st = ctx->stream;
@@ -296,6 +381,20 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
     k_newton_start<<<1, 1, 0, st>>>(S);
     count_launch();
     ops.maxabs(gamma.get(), N, nullptr, 0, &S->maxabs);
+
+    if (!mixed) {
+        PlanCgLaunch L;
+        L.init(P, reg, S, ops.err_flag(), st);
+        if (L.ok) {
+            int niter = 0, len = 0;
+            long long np = 0;
+            newton_on_plan(ctx, P, ops, L, tol, max_iter, cg_tol, gamma.get(), o, hist.get(),
+                           hist_cap, parts.get(), S, &niter, &len, &np);
+            finish_erot_result(ops, gamma.get(), hobj, hmar, htime, nullptr, len, hist_cap, niter, np,
+                               o, res);
+            return;
+        }
+    }
 
     // f, g at gamma (one fused row+column pass).
     PassParams pg = ops.base_params();
@@ -480,6 +579,23 @@ void erot_hess_solve_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, const do
         std::copy(rhs_h, rhs_h + n + m - 1, h.begin());
         h[N - 1] = 0.0;
         h2d(rhs.get(), h.data(), N * sizeof(double), st);
+    }
+    if (!mixed) {
+        PlanCgLaunch L;
+        L.init(P, reg, S, ops.err_flag(), st);
+        if (L.ok) {
+            L.p.rhs = rhs.get();
+            L.p.cg_tol = tol;
+            L.p.x = x.get();
+            L.form_plan(P, gamma.get(), st);
+            L.solve(st);
+            NewtonState hs{};
+            read_small(ctx, &hs, S, sizeof(hs), st);
+            if (!hs.cg_done) ops.check_err();
+            read_small(ctx, x_h, x.get(), (size_t)(n + m - 1) * sizeof(double), st);
+            if (iters) *iters = hs.cg_it;
+            return;
+        }
     }
     ops.maxabs(gamma.get(), N, nullptr, 0, &S->maxabs);
     PassParams pg = ops.base_params();

@@ -127,6 +127,34 @@ __global__ void __launch_bounds__(256) k_plan64(const double* __restrict__ M, lo
     }
 }
 
+// FP64 column sums of exp((ra_i + cb_j - M_ij) / reg) over blocks of kRB rows,
+// colpart[rb][j] as the dense pass leaves them: 32 columns and 64 rows a
+// block, for the same reason as k_plan64 (a dense-pass tile holds one SM for
+// 190 us; this takes 12 us at 100 x 80).
+__global__ void __launch_bounds__(256) k_colsum64(const double* __restrict__ M, long long ldm, int n,
+                                                  int m, const double* __restrict__ ra,
+                                                  const double* __restrict__ cb, double kexp,
+                                                  double* colpart) {
+    __shared__ double s_c[8][32];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + tx, r0 = blockIdx.y * kRB;
+    double c = 0.0;
+    if (j < m) {
+        const double be = cb[j];
+        for (int u = ty; u < kRB; u += 8) {
+            const int i = r0 + u;
+            if (i < n) c += exp(((ra[i] + be) - M[(long long)i * ldm + j]) * kexp);
+        }
+    }
+    s_c[ty][tx] = c;
+    __syncthreads();
+    if (ty == 0 && j < m) {
+#pragma unroll
+        for (int q = 1; q < 8; ++q) c += s_c[q][tx];
+        colpart[(long long)blockIdx.y * m + j] = c;
+    }
+}
+
 }  // namespace
 
 void launch_plan64(const double* M, long long ldm, int n, int m, const double* alpha,
@@ -263,7 +291,16 @@ void ErotOps::optimal_beta(const double* alpha, double* beta, double* mx) {
     p.ra = alpha;
     p.grid = mx;
     p.cb = anchor_.get();
-    pass(OP_E_COL, p);
+    const int nrb = cdiv(n_, kRB);
+    if (!mixed_ && nrb <= 65535) {
+        k_colsum64<<<dim3(cdiv(m_, 32), nrb), 256, 0, st_>>>(
+            static_cast<const double*>(P_->M), P_->ldm, n_, m_, alpha, anchor_.get(), 1.0 / reg_,
+            reinterpret_cast<double*>(buf_.colpart.get()));
+        count_launch();
+        REGOT_CHECK_LAUNCH();
+    } else {
+        pass(OP_E_COL, p);
+    }
     REGOT_LAUNCH_ACC(k_col_lse, m_, buf_.colpart.get(), buf_.shape.nrb, m_, anchor_.get(),
                      P_->logb, reg_, beta);
 }

@@ -176,4 +176,77 @@ __device__ __forceinline__ void merge_columns(const double* part, long long ldk,
     else merge_columns_w<4>(part, ldk, G, j0, j1, warp, warps, use);
 }
 
+// ---- launches: one cluster of 16 blocks for small problems, else a block an SM ----
+
+// Problems of at most this many entries run in one cluster.
+constexpr long long kClusterEntries = 64 * 1024;
+// A stored plan doubles the memory of the cost matrix; beyond this size the
+// solvers keep to the dense passes.
+constexpr double kPlanMaxBytes = 32.0 * (1ULL << 30);
+
+inline size_t max_block_smem() {
+    int dev = 0, optin = 0;
+    REGOT_CUDA(cudaGetDevice(&dev));
+    REGOT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    return (size_t)optin - 1024;  // static shared memory of the kernels
+}
+
+inline cudaLaunchConfig_t resident_config(cudaLaunchAttribute* at, bool cluster, int blocks,
+                                          size_t smem, cudaStream_t st) {
+    if (cluster) {
+        at->id = cudaLaunchAttributeClusterDimension;
+        at->val.clusterDim.x = (unsigned)blocks;
+        at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    } else {
+        at->id = cudaLaunchAttributeCooperative;
+        at->val.cooperative = 1;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kResThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Whether `kernel` runs n m = entries entries in one cluster of 16 blocks.
+template <typename P>
+bool resident_cluster(void (*kernel)(P), long long entries, size_t smem) {
+    if (entries > kClusterEntries || smem > max_block_smem()) return false;
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = resident_config(at, true, 16, smem, nullptr);
+    int clusters = 0;
+    const bool ok =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+            cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+// Whether a cooperative launch of `kernel` holds one block on every SM.
+template <typename P>
+bool resident_grid(void (*kernel)(P), size_t smem) {
+    int dev = 0, coop = 0, occ = 0;
+    REGOT_CUDA(cudaGetDevice(&dev));
+    REGOT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop || smem > max_block_smem()) return false;
+    REGOT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    REGOT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kResThreads, smem));
+    return occ >= 1;
+}
+
+template <typename P>
+void launch_resident(void (*kernel)(P), bool cluster, int blocks, size_t smem, cudaStream_t st,
+                     const P& params) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = resident_config(at, cluster, blocks, smem, st);
+    REGOT_CUDA(cudaLaunchKernelEx(&cfg, kernel, params));
+    count_launch();
+}
+
 }  // namespace regot
