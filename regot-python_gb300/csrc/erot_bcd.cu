@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <vector>
 
 #include "device_util.cuh"
@@ -312,8 +313,8 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
         try {
             K.alloc((size_t)n * ldk, st);
             spart.alloc((size_t)sp.blocks * ldk, st);
-            // v, red, blast, redf, count
-            sbuf.alloc((size_t)ldk + 5 * (size_t)sp.blocks + 4, st);
+            // red, v, blast, fin, redf, count
+            sbuf.alloc((size_t)ldk + 6 * (size_t)sp.blocks + 8, st);
         } catch (const Error&) {  // no room for a second matrix: the passes below
             cudaGetLastError();
             K.release();
@@ -472,12 +473,14 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
         q.reg = reg;
         q.sum_a = ops.sum_a();
         q.sum_bt = ops.sum_bt();
+        q.stop2 = largest_square_below(tol);
         q.part = spart.get();
         q.red = sbuf.get();
         q.vbuf = q.red + 4 * (size_t)sp.blocks;
         q.blast = q.vbuf + ldk;
-        q.redf = reinterpret_cast<int*>(q.blast + 1);
-        q.count = reinterpret_cast<unsigned*>(q.blast + 3 + sp.blocks / 2);
+        q.fin = q.blast + 1;
+        q.redf = reinterpret_cast<int*>(q.fin + sp.blocks + 1);
+        q.count = reinterpret_cast<unsigned*>(q.redf + sp.blocks);
         q.err = ops.err_flag();
         q.st = S;
         q.hobj = hobj;

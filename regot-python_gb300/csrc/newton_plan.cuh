@@ -38,15 +38,15 @@ struct PlanCgParams {
 
 inline size_t plan_cg_smem(int n, long long ldk, int m, int G) {
     const size_t R = (size_t)(n + G - 1) / G + 1, C = (size_t)(m + G - 1) / G + 1;
-    return sizeof(double) * ((size_t)ldk + 2 * kResThreads + 2 * R + (R > kResWarps ? R : kResWarps) +
-                             6 * (R + C) + 4 * kResWarps);
+    return sizeof(double) * ((size_t)ldk + 2 * kResThreads + 2 * R + rows_part_size((int)R) +
+                             7 * (R + C) + 4 * kResWarps);
 }
 
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p) {
     extern __shared__ __align__(16) double s_dyn[];
-    __shared__ int s_ok;
-    __shared__ double s_tot[4];
+    __shared__ int s_ok, s_stop;
+    __shared__ double s_sc;  // beta, then alpha, of the step
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = blockIdx.x, G = gridDim.x;
     const int n = p.n, m = p.m;
@@ -60,15 +60,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     double* s_sum = s_u + Rm;             // [Rm]
     double* s_part = s_sum + Rm;
     // own items: rows 0 .. R - 1, columns R .. R + C - 1
-    double* s_h = s_part + (Rm > kResWarps ? Rm : kResWarps);  // diag(H)
-    double* s_p = s_h + Im;
+    double* s_h = s_part + rows_part_size(Rm);  // diag(H)
+    double* s_ih = s_h + Im;                    // 1 / diag(H)
+    double* s_p = s_ih + Im;
     double* s_xs = s_p + Im;  // the solution
     double* s_r = s_xs + Im;
     double* s_z = s_r + Im;
-    double* s_y = s_z + Im;   // T p / T' p
+    double* s_y = s_z + Im;   // (T'p)_j of the own columns, at R + j
     double* s_w = s_y + Im;   // [4][kResWarps]
     GridBarrier<CLUSTER> bar(p.count, p.err, &s_ok);
     const double reg = p.reg;
+    const int S = row_segments((int)(ldk >> 1), R);
     const int items = R + C, iwarps = (items + 31) / 32 < kResWarps ? (items + 31) / 32 : kResWarps;
 
     // Sums of v[0..K) over the block's item threads into red[slot][b]: called by
@@ -76,29 +78,25 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     auto publish = [&](int slot, const double* v, int K) {
         if (warp < iwarps) {
             for (int q = 0; q < K; ++q) {
-                const double s = warp_sum_d(v[q]);
+                const double s = warp_sum_low(v[q]);
                 if (lane == 0) s_w[q * kResWarps + warp] = s;
             }
         }
         __syncthreads();
         if (tid < K) {
-            double s = 0.0;
-            for (int w = 0; w < iwarps; ++w) s += s_w[tid * kResWarps + w];
+            double s = iwarps > 0 ? s_w[tid * kResWarps] : 0.0;
+            for (int w = 1; w < iwarps; ++w) s += s_w[tid * kResWarps + w];
             __stcg(p.red + ((size_t)slot * G + b) * 4 + tid, s);
         }
     };
-    // After a barrier: the totals over all blocks into s_tot, the same bits in
-    // every block; warp q sums value q. The caller synchronises.
-    auto total = [&](int slot, int K) {
-        if (warp < K) {
-            double s = 0.0;
-            for (int g = lane; g < G; g += 32) s += __ldcg(p.red + ((size_t)slot * G + g) * 4 + warp);
-            s = warp_sum_d(s);
-            if (lane == 0) s_tot[warp] = s;
-        }
+    // After a barrier, in warp 0: the total of value q over all blocks (in
+    // lane 0; the same bits in every block).
+    auto total = [&](int slot, int q) {
+        return warp_sum_strided(p.red + (size_t)slot * G * 4 + q, G, 4);
     };
+    // Beside it, in the other warps: the own columns' products.
     auto merge = [&]() {
-        merge_columns(p.part, ldk, G, j0, j1, warp, kResWarps,
+        merge_columns(p.part, ldk, G, j0, j1, warp - 1, kResWarps - 1,
                       [&](int j, double c) { s_y[R + j - j0] = c; });
     };
     auto publish_z = [&]() {
@@ -110,11 +108,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     for (int j = tid; j < ldk; j += kResThreads) s_x[j] = j < m ? 1.0 : 0.0;
     for (int r = tid; r < R; r += kResThreads) s_u[r] = 1.0;
     __syncthreads();
-    rows_dot(p.T, ldk, r0, R, s_x, s_part, s_sum);
+    rows_dot(p.T, ldk, r0, R, S, s_x, s_part, s_sum);
     cols_dot(p.T, ldk, r0, R, s_u, p.part + (long long)b * ldk, s_q);
     bar.arrive();
     if (!bar.wait()) return;
-    merge();
+    if (warp > 0) merge();
     __syncthreads();
     {
         double v[4] = {0.0, 0.0, 0.0, 0.0};  // rr, rz, sum r, sum gamma (a, b)
@@ -137,8 +135,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
                 p.g[gi] = 0.0;
             }
             const double h = last ? 1.0 : s / reg;
-            const double z = ri / h;
+            const double ih = 1.0 / h, z = ri * ih;
             s_h[t] = h;
+            s_ih[t] = ih;
             s_r[t] = ri;
             s_z[t] = z;
             s_p[t] = z;
@@ -152,33 +151,42 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     }
     bar.arrive();
     if (!bar.wait()) return;
-    total(0, 4);
-    __syncthreads();
-    const double rr0 = s_tot[0];
-    double rz = s_tot[1];
-    const double thresh2 = fmax(p.cg_tol * p.cg_tol * rr0, 2.2250738585072014e-308);
-    bool stop = rr0 == 0.0 || rr0 < thresh2;
-    if (!p.rhs) {
-        const double f = reg * s_tot[2] - s_tot[3], gnorm = sqrt(rr0);
-        if (b == 0 && tid == 0) {
-            p.st->f = f;
-            p.st->gnorm = gnorm;
-            *p.hobj = f;
-            *p.hmar = gnorm;
-            *p.htime = (double)(globaltimer_ns() - p.st->t0) * 1e-6;
-        }
-        if (gnorm < p.grad_tol || !isfinite(f)) {  // the caller stops here
-            if (b == 0 && tid == 0) p.st->cg_done = 2;
-            return;
-        }
-    }
+    // scalars of the iteration: lane 0 of warp 0, broadcast through s_sc
+    double rz = 0.0, thresh2 = 0.0;
     const int cg_max = p.st->cg_max;
+    if (warp == 0) {
+        const double rr0 = total(0, 0);
+        rz = total(0, 1);
+        const double sr = total(0, 2), sg = total(0, 3);
+        if (lane == 0) {
+            thresh2 = fmax(p.cg_tol * p.cg_tol * rr0, 2.2250738585072014e-308);
+            int stop = rr0 == 0.0 || rr0 < thresh2 ? 1 : 0;
+            if (!p.rhs) {
+                const double f = reg * sr - sg, gnorm = sqrt(rr0);
+                if (gnorm < p.grad_tol || !isfinite(f)) stop = 2;  // the caller stops here
+                if (b == 0) {
+                    p.st->f = f;
+                    p.st->gnorm = gnorm;
+                    *p.hobj = f;
+                    *p.hmar = gnorm;
+                    *p.htime = (double)(globaltimer_ns() - p.st->t0) * 1e-6;
+                    if (stop == 2) p.st->cg_done = 2;
+                }
+            }
+            s_stop = stop;
+            s_sc = 0.0;
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (s_stop == 2) return;
+    const double inv_reg = 1.0 / reg;
     int it = 0;
-    double beta = 0.0;
 
 #pragma unroll 1
-    while (!stop) {
+    while (!s_stop) {
         // the direction: p_beta whole, p_alpha of the own rows
+        const double beta = s_sc;
         for (int j = tid; j < m - 1; j += kResThreads) {
             const double z = __ldcg(p.zbuf + j);
             s_x[j] = it == 0 ? z : fma(beta, s_x[j], z);
@@ -189,36 +197,42 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
             for (int t = tid; t < items; t += kResThreads) s_p[t] = fma(beta, s_p[t], s_z[t]);
         }
         __syncthreads();
-        rows_dot(p.T, ldk, r0, R, s_x, s_part, s_sum);
+        rows_dot(p.T, ldk, r0, R, S, s_x, s_part, s_sum);
         __syncthreads();
         {
             double v = 0.0;
             for (int t = tid; t < items; t += kResThreads) {
                 const double pt = s_p[t];
                 double y = s_h[t] * pt;
-                if (t < R) y = fma(2.0 / reg, s_sum[t], y);
+                if (t < R) y = fma(2.0 * inv_reg, s_sum[t], y);
                 v = fma(pt, y, v);
             }
+            __syncwarp();
             publish(0, &v, 1);
         }
         cols_dot(p.T, ldk, r0, R, s_p, p.part + (long long)b * ldk, s_q);
         bar.arrive();
         if (!bar.wait()) return;
-        total(0, 1);
-        merge();
+        if (warp == 0) {
+            const double pap = total(0, 0);
+            if (lane == 0) s_sc = rz / pap;
+            __syncwarp();
+        } else {
+            merge();
+        }
         __syncthreads();
-        const double alpha = rz / s_tot[0];
         {
+            const double alpha = s_sc;
             double v[2] = {0.0, 0.0};
             for (int t = tid; t < items; t += kResThreads) {
                 const bool last = t >= R && j0 + (t - R) == m - 1;
                 const double tp = t < R ? s_sum[t] : s_y[t];
                 const double pt = s_p[t];
-                const double y = last ? 0.0 : fma(s_h[t], pt, tp / reg);
+                const double y = last ? 0.0 : fma(s_h[t], pt, tp * inv_reg);
                 s_xs[t] = fma(alpha, pt, s_xs[t]);
                 const double ri = fma(-alpha, y, s_r[t]);
                 s_r[t] = ri;
-                const double z = ri / s_h[t];
+                const double z = ri * s_ih[t];
                 s_z[t] = z;
                 v[0] = fma(ri, ri, v[0]);
                 v[1] = fma(ri, z, v[1]);
@@ -229,14 +243,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
         }
         bar.arrive();
         if (!bar.wait()) return;
-        total(1, 2);
-        __syncthreads();
         ++it;
-        const double rr = s_tot[0], rzn = s_tot[1];
-        if (rr < thresh2 || it >= cg_max || !(rr == rr)) stop = true;
-        beta = rzn / rz;
-        rz = rzn;
-        // s_tot is written again after two more barriers of the block
+        if (warp == 0) {
+            const double rr = total(1, 0), rzn = total(1, 1);
+            if (lane == 0) {
+                s_sc = rzn / rz;
+                rz = rzn;
+                if (rr < thresh2 || it >= cg_max || !(rr == rr)) s_stop = 1;
+            }
+            __syncwarp();
+        }
+        __syncthreads();
     }
     for (int t = tid; t < items; t += kResThreads) {
         const int gi = t < R ? r0 + t : n + j0 + (t - R);

@@ -4,11 +4,14 @@
 // vector, then its part of the column products, and after a barrier of all
 // blocks merges a run of columns over the blocks.
 //
-// FP64 issue bounds these kernels, not memory: a GB300 SM starts two FP64
-// operations a clock, so a warp's FP64 instruction holds its quarter of the
-// SM for 64 clocks whatever the number of active lanes. Hence the layouts:
-// full warps, few reduction levels (they cost as much as full-width work),
-// and no FP64 comparison where a look at the exponent bits will do.
+// FP64 issue bounds these kernels, not memory: on a GB300 an FP64 instruction
+// holds its quarter of the SM for 64 to 77 clocks, whether one of the warp's
+// lanes is active or all (measured: dependent or not, 71 clocks an addition,
+// 630 a division, 2150 a logarithm, 610 a five-level shuffle sum). Hence: as
+// few FP64 instructions as possible, packed into full warps - divisions of a
+// block's rows or columns together in one warp, lane sums of several rows
+// added side by side - and no FP64 comparison where a look at the exponent
+// bits will do.
 #pragma once
 
 #include "device_util.cuh"
@@ -30,53 +33,126 @@ __device__ __forceinline__ bool exponent_within(double x, int lim) {
     return e >= -lim && e <= lim;
 }
 
+// Sum over the lanes congruent modulo `keep`, valid in lanes 0 .. keep - 1.
+__device__ __forceinline__ double warp_sum_low(double v, int keep = 1) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (o < keep) break;
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    return v;
+}
+
+// Sum of p[g * stride], g < G, over the warp (valid in lane 0): five loads a
+// lane under way together.
+__device__ __forceinline__ double warp_sum_strided(const double* p, int G, int stride) {
+    const int lane = threadIdx.x & 31;
+    double s = 0.0;
+    for (int g = lane; g < G; g += 160) {
+        double v[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            v[k] = g + 32 * k < G ? __ldcg(p + (long long)(g + 32 * k) * stride) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            if (g + 32 * k < G) s += v[k];
+    }
+    __syncwarp();
+    return warp_sum_low(s);
+}
+
 // s_sum[r] = sum_j K[r0 + r][j] s_x[j], r < R. s_x: ldk entries in shared
-// memory. Whole rows a warp; with fewer rows than warps, equal column
-// segments of a row. Synchronises the block before the segments are added;
-// the caller synchronises before it reads s_sum.
+// memory. A warp takes a row, or one of S equal column segments of it, with S
+// as it leaves the fewest FP64 instructions on a quarter of the SM. The lanes'
+// sums of up to kRowUnits segments go through shared memory, so that several
+// rows are added side by side; beyond that many a warp adds its own.
+// Synchronises the block before the last additions; the caller synchronises
+// before it reads s_sum. s_part: rows_part_size(R) doubles.
+constexpr int kRowUnits = 64;
+__host__ __device__ constexpr int rows_part_size(int R) {
+    return R > kRowUnits * 33 ? R : kRowUnits * 33;
+}
+__device__ __forceinline__ int row_segments(int P, int R) {
+    int best = 1, cost = 1 << 30;
+    for (int S = 1; S <= 16; S <<= 1) {
+        if (S > 1 && (R * S > kRowUnits || P < 64 * S)) break;
+        const int c = ((R * S + 3) / 4) * (2 * ((P + 32 * S - 1) / (32 * S)) + 4);
+        if (c < cost) {
+            cost = c;
+            best = S;
+        }
+    }
+    return best;
+}
 __device__ __forceinline__ void rows_dot(const double* __restrict__ K, long long ldk, int r0, int R,
-                                         const double* s_x, double* s_part, double* s_sum) {
+                                         int S, const double* s_x, double* s_part, double* s_sum) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int P = (int)(ldk >> 1);
-    int S = 1;
-    if (R > 0 && R < kResWarps) {
-        const int by_width = P / 64 > 0 ? P / 64 : 1;
-        S = kResWarps / R < by_width ? kResWarps / R : by_width;
-    }
     const double2* x2 = reinterpret_cast<const double2*>(s_x);
-    for (int unit = warp; unit < R * S; unit += kResWarps) {
-        const int row = unit / S, seg = unit - row * S;
+    const int units = R * S, len = (P + S - 1) / S;
+    const bool own = units > kRowUnits;  // then S == 1
+    for (int unit = warp; unit < units; unit += kResWarps) {
+        const int row = S == 1 ? unit : unit / S, seg = unit - row * S;
         const double2* k2 = reinterpret_cast<const double2*>(K + (long long)(r0 + row) * ldk);
-        const int p1 = (int)((long long)P * (seg + 1) / S);
-        int p = (int)((long long)P * seg / S) + lane;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        for (; p + 96 < p1; p += 128) {
-            const double2 q0 = __ldg(k2 + p), q1 = __ldg(k2 + p + 32), q2 = __ldg(k2 + p + 64),
-                          q3 = __ldg(k2 + p + 96);
-            const double2 y0 = x2[p], y1 = x2[p + 32], y2 = x2[p + 64], y3 = x2[p + 96];
-            a0 = fma(q0.x, y0.x, a0);
-            a1 = fma(q0.y, y0.y, a1);
-            a2 = fma(q1.x, y1.x, a2);
-            a3 = fma(q1.y, y1.y, a3);
-            a0 = fma(q2.x, y2.x, a0);
-            a1 = fma(q2.y, y2.y, a1);
-            a2 = fma(q3.x, y3.x, a2);
-            a3 = fma(q3.y, y3.y, a3);
-        }
-        for (; p < p1; p += 32) {
-            const double2 q0 = __ldg(k2 + p);
+        const int p1 = (seg + 1) * len < P ? (seg + 1) * len : P;
+        int p = seg * len + lane;
+        double a0 = 0.0, a1 = 0.0;
+        // the next loads are under way while these are multiplied
+        double2 q[4];
+        auto load = [&](int at) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                q[k] = at + 32 * k < p1 ? __ldg(k2 + at + 32 * k) : make_double2(0.0, 0.0);
+        };
+        load(p);
+        for (; p < p1; p += 128) {
+            const double2 c0 = q[0], c1 = q[1], c2 = q[2], c3 = q[3];
+            load(p + 128);
             const double2 y0 = x2[p];
-            a0 = fma(q0.x, y0.x, a0);
-            a1 = fma(q0.y, y0.y, a1);
+            a0 = fma(c0.x, y0.x, a0);
+            a1 = fma(c0.y, y0.y, a1);
+            if (p + 32 < p1) {
+                const double2 y1 = x2[p + 32];
+                a0 = fma(c1.x, y1.x, a0);
+                a1 = fma(c1.y, y1.y, a1);
+            }
+            if (p + 64 < p1) {
+                const double2 y2 = x2[p + 64];
+                a0 = fma(c2.x, y2.x, a0);
+                a1 = fma(c2.y, y2.y, a1);
+            }
+            if (p + 96 < p1) {
+                const double2 y3 = x2[p + 96];
+                a0 = fma(c3.x, y3.x, a0);
+                a1 = fma(c3.y, y3.y, a1);
+            }
         }
-        const double v = warp_sum_d((a0 + a1) + (a2 + a3));
-        if (lane == 0) s_part[unit] = v;
+        __syncwarp();
+        const double v = a0 + a1;
+        if (own) {
+            const double t = warp_sum_low(v);
+            if (lane == 0) s_sum[row] = t;
+        } else {
+            s_part[unit * 33 + lane] = v;
+        }
     }
     __syncthreads();
-    for (int r = threadIdx.x; r < R; r += kResThreads) {
-        double v = s_part[r * S];
-        for (int k = 1; k < S; ++k) v += s_part[r * S + k];
-        s_sum[r] = v;
+    if (own) return;
+    // eight threads a row: four lane sums of each of its segments, then a tree
+    for (int g = threadIdx.x; g < ((8 * R + 31) & ~31); g += kResThreads) {
+        const int row = g >> 3, e = g & 7;
+        double v = 0.0;
+        if (row < R) {
+            const double* src = s_part + row * S * 33 + e;
+            v = (src[0] + src[8]) + (src[16] + src[24]);
+            for (int k = 1; k < S; ++k) {
+                src += 33;
+                v += (src[0] + src[8]) + (src[16] + src[24]);
+            }
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (e == 0 && row < R) s_sum[row] = v;
     }
 }
 
@@ -136,43 +212,39 @@ __device__ __forceinline__ void cols_dot(const double* __restrict__ K, long long
 }
 
 // Columns [j0, j1) summed over the G rows of part (stride ldk), one warp for
-// CPW adjacent columns and 32 / CPW groups of rows: use(j, sum) in one lane
-// per column. Called by `warps` whole warps, this one being number `warp`.
+// CPW adjacent columns and 32 / CPW groups of rows, five loads a lane under
+// way together: use(j, sum) in one lane per column. Called by `warps` whole
+// warps, this one being number `warp`.
 template <int CPW, typename F>
 __device__ __forceinline__ void merge_columns_w(const double* part, long long ldk, int G, int j0,
                                                 int j1, int warp, int warps, F&& use) {
     const int lane = threadIdx.x & 31;
     const int c = lane % CPW, g0 = lane / CPW;
-    constexpr int GS = 32 / CPW;
+    constexpr int GS = 32 / CPW, NL = 5;
     for (int jb = j0 + warp * CPW; jb < j1; jb += warps * CPW) {
         const int j = jb + c;
         const bool ok = j < j1;
-        double s0 = 0.0, s1 = 0.0;
-        if (ok) {
-            int g = g0;
-            for (; g + 3 * GS < G; g += 4 * GS) {
-                double v[4];
+        double s = 0.0;
+        for (int g = g0; g < G; g += NL * GS) {
+            double v[NL];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) v[k] = __ldcg(part + (long long)(g + k * GS) * ldk + j);
-                s0 += v[0];
-                s1 += v[1];
-                s0 += v[2];
-                s1 += v[3];
-            }
-            for (; g < G; g += GS) s0 += __ldcg(part + (long long)g * ldk + j);
+            for (int k = 0; k < NL; ++k)
+                v[k] = ok && g + k * GS < G ? __ldcg(part + (long long)(g + k * GS) * ldk + j) : 0.0;
+#pragma unroll
+            for (int k = 0; k < NL; ++k)
+                if (g + k * GS < G) s += v[k];
         }
-        double s = s0 + s1;
-#pragma unroll
-        for (int o = 16; o >= CPW; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        __syncwarp();
+        s = warp_sum_low(s, CPW);
         if (ok && g0 == 0) use(j, s);
     }
 }
-// Few columns a block: two a warp, so that the chain of additions is short;
+// Few columns a block: one a warp, so that the chain of additions is short;
 // many: four, whose loads fill whole 32-byte sectors.
 template <typename F>
 __device__ __forceinline__ void merge_columns(const double* part, long long ldk, int G, int j0,
                                               int j1, int warp, int warps, F&& use) {
-    if (j1 - j0 <= 2 * warps) merge_columns_w<2>(part, ldk, G, j0, j1, warp, warps, use);
+    if (j1 - j0 <= 2 * warps) merge_columns_w<1>(part, ldk, G, j0, j1, warp, warps, use);
     else merge_columns_w<4>(part, ldk, G, j0, j1, warp, warps, use);
 }
 
