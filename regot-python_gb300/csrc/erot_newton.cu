@@ -238,13 +238,15 @@ __global__ void k_newton_time(NewtonState* st, double* out) {
     *out = (double)(globaltimer_ns() - st->t0) * 1e-6;
 }
 
-// Sum of the per-CTA line-search totals of `nsteps` step sizes.
+// Sum of the per-CTA line-search totals of `nsteps` step sizes, a warp each
+// (one thread adding 304 values in a row took 20 us).
 __global__ void k_ls_totals(const double* totpart, int nblocks, int nsteps, double* out) {
-    const int s = threadIdx.x;
+    const int s = threadIdx.y;
     if (s >= nsteps) return;
     double acc = 0.0;
-    for (int k = 0; k < nblocks; ++k) acc += totpart[(size_t)s * nblocks + k];
-    out[s] = acc;
+    for (int k = threadIdx.x; k < nblocks; k += 32) acc += totpart[(size_t)s * nblocks + k];
+    acc = warp_sum_d(acc);
+    if (threadIdx.x == 0) out[s] = acc;
 }
 
 }  // namespace
@@ -252,6 +254,7 @@ __global__ void k_ls_totals(const double* totpart, int nblocks, int nsteps, doub
 }  // namespace regot
 
 #include "newton_plan.cuh"
+#include "newton_plan32.cuh"
 
 namespace regot {
 
@@ -441,10 +444,14 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
         k_cg_c<<<gv, kVecThreads, 0, st>>>(N, n, z.get(), pv.get(), S, rs_mut, cs_mut);
         count_launch(3);
     };
+    // The whole CG in one launch on the stored plan, where that fits; else the
+    // captured step.
+    PlanCg32 L32;
+    if (mixed) L32.init(P, ops, S, st);
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     long long graph_kernels = 0;
-    {
+    if (!L32.ok) {
         long long* saved = g_launch_counter;
         g_launch_counter = &graph_kernels;
         REGOT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -480,15 +487,20 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
             std::printf("iter = %d, objval = %g, ||grad|| = %g\n", i, hs.f, hs.gnorm);
         if (hs.gnorm < tol || !std::isfinite(hs.f)) break;  // sinkhorn_newton.cpp:87-88
 
-        // Newton direction: H x = -g by preconditioned CG.
-        k_cg_init<<<gv, kVecThreads, 0, st>>>(N, g.get(), -1.0, hdiag.get(), cg_tol, x.get(),
-                                              r.get(), z.get(), pv.get(), parts.get(), S);
-        count_launch();
-        // the split of gamma (and of p = z) for the CG's HVP passes
-        ops.maxabs(gamma.get(), N, nullptr, 0, &S->maxabs);
-        ops.split(ph);
-        int batch = 8;
-        for (;;) {
+        // Newton direction: H x = -g by preconditioned CG, on the split of gamma
+        // (and of p = z for the HVP passes).
+        if (L32.ok) {
+            ops.maxabs(gamma.get(), N, nullptr, 0, &S->maxabs);
+            ops.split(pg);
+            L32.solve(ops.rsplit(), ops.csplit(), g.get(), -1.0, hdiag.get(), cg_tol, x.get(), st);
+        } else {
+            k_cg_init<<<gv, kVecThreads, 0, st>>>(N, g.get(), -1.0, hdiag.get(), cg_tol, x.get(),
+                                                  r.get(), z.get(), pv.get(), parts.get(), S);
+            count_launch();
+            ops.maxabs(gamma.get(), N, nullptr, 0, &S->maxabs);
+            ops.split(ph);
+        }
+        for (int batch = 8; !L32.ok;) {
             for (int q = 0; q < batch; ++q) REGOT_CUDA(cudaGraphLaunch(exec, st));
             count_launch(graph_kernels * batch);
             int done = 0, it = 0;
@@ -502,14 +514,30 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
             batch = std::min(batch * 2, 64);
         }
 
-        // Armijo backtracking on exact objective differences.
+        // Armijo backtracking on exact objective differences. The first pass
+        // tries the full step alone and is read back with the direction.
         k_dir_dots<<<gv, kVecThreads, 0, st>>>(n, m, g.get(), x.get(), P->a, P->b, parts.get(), S);
         count_launch();
+        double tots[4];
+        auto try_steps = [&](const double* steps, int ns) {
+            PassParams q = pl;
+            for (int s = 0; s < 4; ++s) q.steps[s] = s < ns ? steps[s] : 0.0;
+            q.nsteps = ns;
+            ops.pass(OP_E_LS, q);
+            ++passes;
+            k_ls_totals<<<1, dim3(32, 4), 0, st>>>(ops.buf().totpart.get(), ls_blocks, ns, lsout.get());
+            count_launch();
+            d2h(tots, lsout.get(), ns * sizeof(double), st);
+        };
+        const double full = 1.0;
+        try_steps(&full, 1);
         read_small(ctx, &hs, S, sizeof(hs), st);
+        if (!hs.cg_done) ops.check_err();
+        if (L32.ok) passes += hs.cg_it;
         const double thresh = theta * hs.gtd;
         double step = 1.0, accepted = -1.0;
-        // The first pass tries the full step alone (accepted in most Newton
-        // iterations; one phi per entry instead of four), later passes four
+        // The first pass tried the full step alone (accepted in most Newton
+        // iterations; one phi per entry instead of four), later passes try four
         // steps at a time. The accepted step is the reference's first
         // acceptable one either way.
         for (int k0 = 0; k0 < nlinesearch && accepted < 0.0;) {
@@ -517,16 +545,10 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
             k0 += ns;
             double steps[4] = {0, 0, 0, 0};
             for (int s = 0; s < ns; ++s) steps[s] = step * std::pow(kappa, s);
-            PassParams q = pl;
-            for (int s = 0; s < 4; ++s) q.steps[s] = steps[s];
-            q.nsteps = ns;
-            ops.pass(OP_E_LS, q);
-            ++passes;
-            k_ls_totals<<<1, 32, 0, st>>>(ops.buf().totpart.get(), ls_blocks, ns, lsout.get());
-            count_launch();
-            double tots[4];
-            d2h(tots, lsout.get(), ns * sizeof(double), st);
-            sync(st);
+            if (k0 > ns) {  // the full step is tried already
+                try_steps(steps, ns);
+                sync(st);
+            }
             for (int s = 0; s < ns; ++s) {
                 const double df = steps[s] * hs.gtd + reg * tots[s];
                 if (df <= steps[s] * thresh) {  // newf <= f + step * thresh
@@ -545,8 +567,8 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
         ++passes;
         record();
     }
-    cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
     finish_erot_result(ops, gamma.get(), hobj, hmar, htime, nullptr, hist_len, hist_cap, i,
                        passes, o, res);
 }
@@ -613,10 +635,23 @@ void erot_hess_solve_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, const do
             (const double*)ops.buf().rowpart.get(), sh.nslabs,
             (const double*)ops.buf().colpart.get(), sh.nrb, n, m, gamma.get(), P->a, P->b, reg,
             g.get(), hdiag.get(), parts.get(), S);
+    count_launch();
+    REGOT_CHECK_LAUNCH();
+    PlanCg32 L32;
+    if (mixed) L32.init(P, ops, S, st);
+    if (L32.ok) {  // the split of the pass above is gamma's
+        L32.solve(ops.rsplit(), ops.csplit(), rhs.get(), 1.0, hdiag.get(), tol, x.get(), st);
+        NewtonState done{};
+        read_small(ctx, &done, S, sizeof(done), st);
+        if (!done.cg_done) ops.check_err();
+        read_small(ctx, x_h, x.get(), (size_t)(n + m - 1) * sizeof(double), st);
+        if (iters) *iters = done.cg_it;
+        ops.check_err();
+        return;
+    }
     k_cg_init<<<gv, kVecThreads, 0, st>>>(N, rhs.get(), 1.0, hdiag.get(), tol, x.get(), r.get(),
                                           z.get(), pv.get(), parts.get(), S);
-    count_launch(2);
-    REGOT_CHECK_LAUNCH();
+    count_launch();
     PassParams ph = pg;
     ph.rx = pv.get();
     ph.cx = pv.get() + n;

@@ -59,3 +59,37 @@ def test_optimal_beta_fp64_shapes(n, m):
     np.testing.assert_allclose(P.erot_optimal_beta(0.02, alpha),
                                O.erot_optimal_beta(M, b, 0.02, alpha), rtol=0, atol=1e-13)
     P.close()
+
+
+SHAPES32 = [(1, 5), (5, 1), (63, 511), (64, 512), (65, 513), (129, 1030), (300, 260), (2100, 1000),
+            (40, 4200), (4200, 40)]
+
+
+@pytest.mark.parametrize("n,m", SHAPES32)
+def test_mixed_hessian_solve_on_the_plan(n, m):
+    # T carries a few 1e-7 relative and the FP32 tile sums some 1e-7 more, so a
+    # product errs by less than 5e-7 of H |x|; the residual that CG updates
+    # drifts from the true one by a few products' errors: four of them, and
+    # the solve's own tolerance
+    reg = 0.05
+    M, a, b = erot_points(n, m, seed=n + m, dtype=np.float32)
+    Mq = M.astype(np.float64)
+    gamma = O.sinkhorn_bcd(Mq, a, b, reg, tol=1e-5, max_iter=200, plan=False).dual
+    rhs = np.random.default_rng(0).standard_normal(n + m - 1)
+    P = regot.Problem(M, a, b, precision="mixed")
+    x, steps = P.erot_hess_solve(reg, gamma, rhs, tol=1e-7)
+    assert steps > 0
+    res = O.erot_hvp(Mq, a, b, reg, gamma, x) - rhs
+    size = O.erot_hvp(Mq, a, b, reg, gamma, np.abs(x))
+    assert np.linalg.norm(res) < 2e-6 * np.linalg.norm(size) + 1e-7 * np.linalg.norm(rhs)
+    P.close()
+
+
+@pytest.mark.parametrize("n,m", [(65, 513), (700, 1100)])
+def test_mixed_newton_on_the_plan_agrees_with_fp64(n, m):
+    reg = 0.05
+    M, a, b = erot_points(n, m, seed=n + m, dtype=np.float32)
+    r = regot.sinkhorn_newton(M, a, b, reg, tol=1e-6, max_iter=50, precision="mixed")
+    o = regot.sinkhorn_newton(M.astype(np.float64), a, b, reg, tol=1e-6, max_iter=50)
+    assert r.mar_errs[-1] < 1e-6
+    np.testing.assert_allclose(r.dual, o.dual, rtol=0, atol=1e-6)
