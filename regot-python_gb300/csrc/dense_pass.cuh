@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
 
     // Constants prepared on the host (no FP64 arithmetic in this kernel:
     // FP64 throughput on this part is a small fraction of FP32).
-    const TM kexp = MIXED ? (TM)p.kexp_f : (TM)p.kexp_d;
+    const TM kexp = MIXED ? (TM)p.kexp_f : (TM)0;  // FP64: p.exp64
     const TM inv_reg = MIXED ? (TM)p.inv_reg_f : (TM)p.inv_reg_d;
     const TM init = ISMAX ? (TM)(-INFINITY) : (TM)0;
     TM steps[4];
@@ -771,7 +771,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
                                 const TM s = (rh + ch[q]) - mval;
                                 T = ex2_approx(fmaf(s, kexp, rlk + clk[q]));
                             } else {
-                                T = exp(((rh + ch[q]) - mval) * kexp);
+                                T = exp_scaled((rh + ch[q]) - mval, p.exp64);
                             }
                             if constexpr (OP == OP_E_ROW) {
                                 racc[0] += T;

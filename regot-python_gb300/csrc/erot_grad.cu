@@ -34,7 +34,8 @@ constexpr int kTyyD = 64;
 template <bool COLS>
 __global__ void __launch_bounds__(256) k_tyy64(const double* __restrict__ M, long long ldm, int n,
                                                int m, const double* __restrict__ gamma,
-                                               double inv_reg, const double* __restrict__ u,
+                                               double inv_reg, const Exp64 ex,
+                                               const double* __restrict__ u,
                                                const double* __restrict__ W,
                                                const double* __restrict__ Y, int ldy, int d,
                                                double* __restrict__ sums, double* __restrict__ Z,
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__(256) k_tyy64(const double* __restrict__ M, lon
             const int i = COLS ? k : o, j = COLS ? o : k;
             double g = 0.0;
             if (o < nown && k < K) {
-                const double T = exp(((gamma[i] + gamma[n + j]) - M[(long long)i * ldm + j]) * inv_reg);
+                const double T = exp_scaled((gamma[i] + gamma[n + j]) - M[(long long)i * ldm + j], ex);
                 if (u) {
                     const double w = W ? W[(long long)i * m + j] : 0.0;
                     g = T * (u[i] + u[n + j] - w) * inv_reg;
@@ -193,11 +194,11 @@ void erot_contract_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, const doub
         const double* Y = d_Y ? d_Y + k0 : nullptr;
         if (cols)
             k_tyy64<true><<<blocks, 256, 0, st>>>(static_cast<const double*>(P->M), P->ldm, n, m,
-                                                  d_gamma, 1.0 / reg, d_u, d_W, Y, d, dk, sums, Z,
+                                                  d_gamma, 1.0 / reg, exp64_for(reg), d_u, d_W, Y, d, dk, sums, Z,
                                                   d);
         else
             k_tyy64<false><<<blocks, 256, 0, st>>>(static_cast<const double*>(P->M), P->ldm, n, m,
-                                                   d_gamma, 1.0 / reg, d_u, d_W, Y, d, dk, sums,
+                                                   d_gamma, 1.0 / reg, exp64_for(reg), d_u, d_W, Y, d, dk, sums,
                                                    Z, d);
         count_launch();
         REGOT_CHECK_LAUNCH();

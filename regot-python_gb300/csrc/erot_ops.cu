@@ -94,22 +94,22 @@ __global__ void k_sum_totals(const double* totpart, int nblocks, int nt, double*
 
 // out_ij = exp((alpha_i + beta_j - M_ij) / reg), row stride ldo, zero in the
 // columns m .. ldo - 1; *zero = 0 (the counter of a barrier that a later
-// kernel uses). One FP64 exponential an entry (about twenty FP64 operations at
-// two a clock and SM) bounds it, so the entries are spread over all SMs
-// whatever the shape: the tiles of the dense pass give 64 x 256 entries to one
-// SM, 190 us at 1000 x 800, of which this kernel needs a quarter. VEC: pairs of
+// kernel uses). One FP64 exponential an entry bounds it, so the entries are
+// spread over all SMs whatever the shape: the tiles of the dense pass give
+// 64 x 256 entries to one SM, 190 us at 1000 x 800. VEC: pairs of
 // columns, where out and the rows of both matrices start on 16 bytes.
 template <bool VEC>
 __global__ void __launch_bounds__(256) k_plan64(const double* __restrict__ M, long long ldm, int n,
                                                 int m, const double* __restrict__ alpha,
-                                                const double* __restrict__ beta, double kexp,
+                                                const double* __restrict__ beta, const Exp64 ex,
                                                 double* out, long long ldo, unsigned* zero) {
     constexpr int W = VEC ? 2 : 1;
     if (zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0u;
-    const long long per_row = ldo / W, total = n * per_row;
+    const unsigned per_row = (unsigned)(ldo / W);
+    const long long total = (long long)n * per_row;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const long long i = t / per_row;
+        const long long i = total <= 0xffffffffLL ? (long long)((unsigned)t / per_row) : t / per_row;
         const int j = W * (int)(t - i * per_row);
         const double al = alpha[i];
         const double* src = M + i * ldm + j;
@@ -117,12 +117,12 @@ __global__ void __launch_bounds__(256) k_plan64(const double* __restrict__ M, lo
             double2 q = make_double2(0.0, 0.0);
             if (j < m) {  // ldm is even: the second column may be padding
                 const double2 c = *reinterpret_cast<const double2*>(src);
-                q.x = exp(((al + beta[j]) - c.x) * kexp);
-                if (j + 1 < m) q.y = exp(((al + beta[j + 1]) - c.y) * kexp);
+                q.x = exp_scaled((al + beta[j]) - c.x, ex);
+                if (j + 1 < m) q.y = exp_scaled((al + beta[j + 1]) - c.y, ex);
             }
             *reinterpret_cast<double2*>(out + i * ldo + j) = q;
         } else {
-            out[i * ldo + j] = j < m ? exp(((al + beta[j]) - *src) * kexp) : 0.0;
+            out[i * ldo + j] = j < m ? exp_scaled((al + beta[j]) - *src, ex) : 0.0;
         }
     }
 }
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(256) k_plan64(const double* __restrict__ M, lo
 // 190 us; this takes 12 us at 100 x 80).
 __global__ void __launch_bounds__(256) k_colsum64(const double* __restrict__ M, long long ldm, int n,
                                                   int m, const double* __restrict__ ra,
-                                                  const double* __restrict__ cb, double kexp,
+                                                  const double* __restrict__ cb, const Exp64 ex,
                                                   double* colpart) {
     __shared__ double s_c[8][32];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) k_colsum64(const double* __restrict__ M, 
         const double be = cb[j];
         for (int u = ty; u < kRB; u += 8) {
             const int i = r0 + u;
-            if (i < n) c += exp(((ra[i] + be) - M[(long long)i * ldm + j]) * kexp);
+            if (i < n) c += exp_scaled((ra[i] + be) - M[(long long)i * ldm + j], ex);
         }
     }
     s_c[ty][tx] = c;
@@ -163,11 +163,13 @@ void launch_plan64(const double* M, long long ldm, int n, int m, const double* a
     const bool vec = ldo % 2 == 0 && ldm % 2 == 0 &&
                      ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(M)) & 15) == 0;
     const long long items = (long long)n * (vec ? ldo / 2 : ldo);
-    const int blocks = (int)std::min<long long>((items + 255) / 256, 8LL * device_sm_count());
+    // one item a thread: a grid of resident blocks would leave most SMs idle in
+    // its last round (45 against 30 us at 1000 x 800)
+    const int blocks = (int)std::min<long long>((items + 255) / 256, 1 << 20);
     if (vec)
-        k_plan64<true><<<blocks, 256, 0, st>>>(M, ldm, n, m, alpha, beta, 1.0 / reg, out, ldo, zero);
+        k_plan64<true><<<blocks, 256, 0, st>>>(M, ldm, n, m, alpha, beta, exp64_for(reg), out, ldo, zero);
     else
-        k_plan64<false><<<blocks, 256, 0, st>>>(M, ldm, n, m, alpha, beta, 1.0 / reg, out, ldo, zero);
+        k_plan64<false><<<blocks, 256, 0, st>>>(M, ldm, n, m, alpha, beta, exp64_for(reg), out, ldo, zero);
     count_launch();
     REGOT_CHECK_LAUNCH();
 }
@@ -294,7 +296,7 @@ void ErotOps::optimal_beta(const double* alpha, double* beta, double* mx) {
     const int nrb = cdiv(n_, kRB);
     if (!mixed_ && nrb <= 65535) {
         k_colsum64<<<dim3(cdiv(m_, 32), nrb), 256, 0, st_>>>(
-            static_cast<const double*>(P_->M), P_->ldm, n_, m_, alpha, anchor_.get(), 1.0 / reg_,
+            static_cast<const double*>(P_->M), P_->ldm, n_, m_, alpha, anchor_.get(), exp64_for(reg_),
             reinterpret_cast<double*>(buf_.colpart.get()));
         count_launch();
         REGOT_CHECK_LAUNCH();

@@ -111,9 +111,9 @@ __device__ __forceinline__ float t_mixed(float mv, float4 r, float4 c, float kex
     return ex2_approx_f(z);
 }
 
-__device__ __forceinline__ double t_plain(double mv, double ra, double cb, double kexp,
+__device__ __forceinline__ double t_plain(double mv, double ra, double cb, const Exp64& ex,
                                           bool& zero64) {
-    const double t = exp(((ra + cb) - mv) * kexp);
+    const double t = exp_scaled((ra + cb) - mv, ex);
     zero64 = (t == 0.0);
     return t;
 }
@@ -371,7 +371,7 @@ struct DenseArgs {
     const float4* cs;  // mixed: column split
     float kexp_f;
     const double* gamma;  // plain: duals (beta at gamma + n)
-    double kexp_d;
+    Exp64 ex;  // FP64 storage
 };
 
 template <typename TM>
@@ -384,7 +384,7 @@ __device__ __forceinline__ float t_at<float>(const DenseArgs& a, int i, int j, f
 template <>
 __device__ __forceinline__ double t_at<double>(const DenseArgs& a, int i, int j, double mv,
                                                bool& z64) {
-    return t_plain(mv, a.gamma[i], a.gamma[a.n + j], a.kexp_d, z64);
+    return t_plain(mv, a.gamma[i], a.gamma[a.n + j], a.ex, z64);
 }
 
 // T' (rows j < m - 1 of length n, stride ldt) and the count of FP64 zeros.
@@ -1738,7 +1738,7 @@ public:
         a.cs = ops_.csplit();
         a.kexp_f = (float)(1.4426950408889634 / reg_);
         a.gamma = gamma_.get();
-        a.kexp_d = 1.0 / reg_;
+        a.ex = exp64_for(reg_);
         return a;
     }
 

@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "exp64.cuh"
 #include "regot_gb300.h"
 
 namespace regot {
@@ -120,7 +121,8 @@ struct PassParams {
     const float* cdsplit = nullptr;  // per column: cd
     // Filled by launch_pass from reg.
     float kexp_f = 0.f, inv_kexp_f = 0.f, inv_reg_f = 0.f;
-    double kexp_d = 0.0, inv_reg_d = 0.0;
+    double inv_reg_d = 0.0;
+    Exp64 exp64{};                 // FP64 passes
     void* rowpart = nullptr;       // [NR][nslabs][n] (Acc)
     void* colpart = nullptr;       // [NC][nrb][m]   (Acc)
     double* totpart = nullptr;     // [NT][nblocks]

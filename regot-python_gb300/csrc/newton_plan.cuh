@@ -29,7 +29,7 @@ struct PlanCgParams {
     double *g, *x;    // gradient (gradient mode) and solution, n + m (last 0)
     double* part;     // [G][ldk]
     double* zbuf;     // [ldk]
-    double* red;      // [2][G][4]
+    double* red;      // [3][G][2]: pairs of block sums
     unsigned* count;
     int* err;
     NewtonState* st;
@@ -67,32 +67,34 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     double* s_r = s_xs + Im;
     double* s_z = s_r + Im;
     double* s_y = s_z + Im;   // (T'p)_j of the own columns, at R + j
-    double* s_w = s_y + Im;   // [4][kResWarps]
+    double* s_w = s_y + Im;   // [2][kResWarps]
     GridBarrier<CLUSTER> bar(p.count, p.err, &s_ok);
     const double reg = p.reg;
     const int S = row_segments((int)(ldk >> 1), R);
     const int items = R + C, iwarps = (items + 31) / 32 < kResWarps ? (items + 31) / 32 : kResWarps;
 
-    // Sums of v[0..K) over the block's item threads into red[slot][b]: called by
-    // all threads (the warps without items only synchronise).
-    auto publish = [&](int slot, const double* v, int K) {
+    // Pairs (v0, v1) summed over the block's item threads into red[slot][b]:
+    // called by all threads (the warps without items only synchronise).
+    auto publish = [&](int slot, double v0, double v1) {
         if (warp < iwarps) {
-            for (int q = 0; q < K; ++q) {
-                const double s = warp_sum_low(v[q]);
-                if (lane == 0) s_w[q * kResWarps + warp] = s;
-            }
+            const bool upper = (lane & 16) != 0;
+            const double send = upper ? v0 : v1;
+            double s = (upper ? v1 : v0) + __shfl_xor_sync(0xffffffffu, send, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if ((lane & 15) == 0) s_w[(lane >> 4) * kResWarps + warp] = s;
         }
         __syncthreads();
-        if (tid < K) {
+        if (tid < 2) {
             double s = iwarps > 0 ? s_w[tid * kResWarps] : 0.0;
             for (int w = 1; w < iwarps; ++w) s += s_w[tid * kResWarps + w];
-            __stcg(p.red + ((size_t)slot * G + b) * 4 + tid, s);
+            __stcg(p.red + ((size_t)slot * G + b) * 2 + tid, s);
         }
     };
-    // After a barrier, in warp 0: the total of value q over all blocks (in
-    // lane 0; the same bits in every block).
-    auto total = [&](int slot, int q) {
-        return warp_sum_strided(p.red + (size_t)slot * G * 4 + q, G, 4);
+    // After a barrier, in one warp: the totals over all blocks (the same bits
+    // in every block).
+    auto total = [&](int slot) {
+        return warp_sum_pairs(reinterpret_cast<const double2*>(p.red) + (size_t)slot * G, G);
     };
     // Beside it, in the other warps: the own columns' products.
     auto merge = [&]() {
@@ -147,7 +149,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
         }
         __syncthreads();
         publish_z();
-        publish(0, v, 4);
+        publish(0, v[0], v[1]);
+        __syncthreads();
+        publish(2, v[2], v[3]);
     }
     bar.arrive();
     if (!bar.wait()) return;
@@ -155,9 +159,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     double rz = 0.0, thresh2 = 0.0;
     const int cg_max = p.st->cg_max;
     if (warp == 0) {
-        const double rr0 = total(0, 0);
-        rz = total(0, 1);
-        const double sr = total(0, 2), sg = total(0, 3);
+        const double2 q0 = total(0), q2 = total(2);
+        const double rr0 = q0.x, sr = q2.x, sg = q2.y;
+        rz = q0.y;
         if (lane == 0) {
             thresh2 = fmax(p.cg_tol * p.cg_tol * rr0, 2.2250738585072014e-308);
             int stop = rr0 == 0.0 || rr0 < thresh2 ? 1 : 0;
@@ -208,13 +212,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
                 v = fma(pt, y, v);
             }
             __syncwarp();
-            publish(0, &v, 1);
+            publish(0, v, 0.0);
         }
         cols_dot(p.T, ldk, r0, R, s_p, p.part + (long long)b * ldk, s_q);
         bar.arrive();
         if (!bar.wait()) return;
         if (warp == 0) {
-            const double pap = total(0, 0);
+            const double pap = total(0).x;
             if (lane == 0) s_sc = rz / pap;
             __syncwarp();
         } else {
@@ -239,13 +243,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
             }
             __syncthreads();
             publish_z();
-            publish(1, v, 2);
+            publish(1, v[0], v[1]);
         }
         bar.arrive();
         if (!bar.wait()) return;
         ++it;
         if (warp == 0) {
-            const double rr = total(1, 0), rzn = total(1, 1);
+            const double2 q = total(1);
+            const double rr = q.x, rzn = q.y;
             if (lane == 0) {
                 s_sc = rzn / rz;
                 rz = rzn;
@@ -266,8 +271,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
 }
 
 // totals[s] = sum_ij T_ij phi(steps[s] w_ij), w = (d_i + d_j) / reg,
-// phi(x) = e^x - 1 - x, for the line search; about twenty FP64 operations an
-// entry and step bound it.
+// phi(x) = e^x - 1 - x, for the line search; FP64 issue bounds it (about twenty
+// instructions an entry and step).
 struct PlanLsParams {
     const double* T;
     long long ldk;
@@ -279,50 +284,31 @@ struct PlanLsParams {
     double* parts;  // [grid][4]
     double* out;    // [4]
     NewtonState* st;
+    Exp64 ex;
 };
-
-__device__ __forceinline__ double phi64(double x) {
-    if (fabs(x) < 0.5) {  // x^2 sum_k x^k / (k + 2)!, to x^17
-        double q = 2.8114572543455206e-15;
-        q = fma(q, x, 4.7794773323873853e-14);
-        q = fma(q, x, 7.6471637318198164e-13);
-        q = fma(q, x, 1.1470745597729725e-11);
-        q = fma(q, x, 1.6059043836821613e-10);
-        q = fma(q, x, 2.0876756987868099e-09);
-        q = fma(q, x, 2.5052108385441720e-08);
-        q = fma(q, x, 2.7557319223985888e-07);
-        q = fma(q, x, 2.7557319223985893e-06);
-        q = fma(q, x, 2.4801587301587302e-05);
-        q = fma(q, x, 1.9841269841269841e-04);
-        q = fma(q, x, 1.3888888888888889e-03);
-        q = fma(q, x, 8.3333333333333333e-03);
-        q = fma(q, x, 4.1666666666666667e-02);
-        q = fma(q, x, 1.6666666666666667e-01);
-        q = fma(q, x, 0.5);
-        return (x * x) * q;
-    }
-    return expm1(x) - x;
-}
 
 __global__ void __launch_bounds__(256) k_plan_ls(const PlanLsParams p) {
     if (p.st->cg_done == 2) return;  // the gradient already met the tolerance
-    const long long per_row = p.ldk >> 1, total = p.n * per_row;
+    const unsigned per_row = (unsigned)(p.ldk >> 1);
+    const long long total = (long long)p.n * per_row;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const long long i = t / per_row;
+        const long long i = total <= 0xffffffffLL ? (long long)((unsigned)t / per_row) : t / per_row;
         const int j = 2 * (int)(t - i * per_row);
         const double2 q = __ldg(reinterpret_cast<const double2*>(p.T + i * p.ldk + j));
         const double di = p.d[i];
         const double w0 = (di + p.d[p.n + j]) * p.inv_reg;
         const bool two = j + 1 < p.m;
         const double w1 = two ? (di + p.d[p.n + j + 1]) * p.inv_reg : 0.0;
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            if (s < p.nsteps) {
-                v[s] = fma(q.x, phi64(p.steps[s] * w0), v[s]);
-                if (two) v[s] = fma(q.y, phi64(p.steps[s] * w1), v[s]);
-            }
+#pragma unroll 1
+        for (int s = 0; s < p.nsteps; ++s) {
+            double a = q.x * phi_tabled(p.steps[s] * w0, p.ex);
+            if (two) a = fma(q.y, phi_tabled(p.steps[s] * w1, p.ex), a);
+            if (s == 0) v[0] += a;
+            else if (s == 1) v[1] += a;
+            else if (s == 2) v[2] += a;
+            else v[3] += a;
         }
     }
     double out[4];
@@ -356,7 +342,7 @@ struct PlanCgLaunch {
             T.alloc((size_t)n * ldk, st);
             part.alloc((size_t)blocks * ldk, st);
             buf.alloc((size_t)ldk + 8 * (size_t)blocks + 8, st);
-            lsparts.alloc(4 * (size_t)ls_blocks(), st);
+            lsparts.alloc(4 * (size_t)(8 * device_sm_count()), st);
         } catch (const Error&) {  // no room for a second matrix
             cudaGetLastError();
             T.release();
@@ -377,7 +363,13 @@ struct PlanCgLaunch {
         p.st = S;
         ok = true;
     }
-    static int ls_blocks() { return 4 * device_sm_count(); }
+    // Blocks of the line search: at most eight an SM, with the items dealt out
+    // evenly over their rounds.
+    int ls_blocks() const {
+        const long long need = ((long long)p.n * (ldk / 2) + 255) / 256, cap = 8LL * device_sm_count();
+        const long long rounds = (need + cap - 1) / cap;
+        return (int)((need + rounds - 1) / rounds);
+    }
     void form_plan(regot_dproblem* P, const double* gamma, cudaStream_t st) {
         launch_plan64(static_cast<const double*>(P->M), P->ldm, p.n, p.m, gamma, gamma + p.n, p.reg,
                       T.get(), ldk, p.count, st);
@@ -400,6 +392,7 @@ struct PlanCgLaunch {
         q.parts = lsparts.get();
         q.out = out;
         q.st = p.st;
+        q.ex = exp64_for(p.reg);
         k_plan_ls<<<ls_blocks(), 256, 0, st>>>(q);
         count_launch();
         REGOT_CHECK_LAUNCH();

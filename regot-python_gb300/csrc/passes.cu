@@ -12,6 +12,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <vector>
 
 #include "internal.h"
 
@@ -151,6 +152,38 @@ void ensure_loaded() {
 int size_class(int n, int m) { return (int)std::floor(std::log2((double)n * (double)m)); }
 }  // namespace
 
+Exp64 exp64_for(double reg) {
+    static std::mutex mutex;
+    static const double* tables[64] = {};  // 4096 doubles, then 6144 pairs
+    int dev = 0;
+    REGOT_CUDA(cudaGetDevice(&dev));
+    require(dev < 64, "device index out of range");
+    std::lock_guard<std::mutex> lock(mutex);
+    if (!tables[dev]) {
+        std::vector<double> h(4096 + 2 * 6144);
+        const long double c = 0.693147180559945309417232121458176568L / 4096.0L;
+        for (int i = 0; i < 4096; ++i) h[i] = (double)std::exp2((long double)i / 4096.0L);
+        for (int i = 0; i < 6144; ++i) {
+            // phi by its series (no cancellation; |x| < 0.52, so 20 terms)
+            const long double x = (i - 3072) * c;
+            long double term = x * x / 2.0L, phi = 0.0L;
+            for (int k = 3; k < 23; ++k) {
+                phi += term;
+                term *= x / k;
+            }
+            h[4096 + 2 * i] = (double)phi;
+            h[4096 + 2 * i + 1] = (double)(phi + x);
+        }
+        double* d = nullptr;
+        REGOT_CUDA(cudaMalloc(&d, h.size() * sizeof(double)));
+        const cudaError_t e = cudaMemcpy(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) cudaFree(d);
+        REGOT_CUDA(e);
+        tables[dev] = d;
+    }
+    return Exp64{tables[dev], reinterpret_cast<const double2*>(tables[dev] + 4096), 1.0 / reg};
+}
+
 long long wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
 long long set_wait_limit(long long spins) {
     return g_wait_limit.exchange(spins < 0 ? kDefaultWaitSpins : spins);
@@ -267,7 +300,7 @@ void launch_pass(int op, const PassParams& p, cudaStream_t st) {
     q.kexp_f = (float)(1.4426950408889634 / p.reg);
     q.inv_kexp_f = 1.0f / q.kexp_f;
     q.inv_reg_f = (float)(1.0 / p.reg);
-    q.kexp_d = 1.0 / p.reg;
+    if (!std::is_same<TM, float>::value) q.exp64 = exp64_for(p.reg);
     q.inv_reg_d = 1.0 / p.reg;
     q.wait_limit = wait_limit();
     constexpr bool mixed = std::is_same<TM, float>::value;

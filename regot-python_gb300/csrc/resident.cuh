@@ -61,6 +61,33 @@ __device__ __forceinline__ double warp_sum_strided(const double* p, int G, int s
     return warp_sum_low(s);
 }
 
+// Sums of p[g].x and p[g].y, g < G, over the warp, in every lane: each half
+// of the warp finishes one of the two.
+__device__ __forceinline__ double2 warp_sum_pairs(const double2* p, int G) {
+    const int lane = threadIdx.x & 31;
+    double a = 0.0, b = 0.0;
+    for (int g = lane; g < G; g += 160) {
+        double2 v[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+            v[k] = g + 32 * k < G ? __ldcg(p + g + 32 * k) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            if (g + 32 * k < G) {
+                a += v[k].x;
+                b += v[k].y;
+            }
+        }
+    }
+    __syncwarp();
+    const bool upper = (lane & 16) != 0;
+    const double send = upper ? a : b;
+    double s = (upper ? b : a) + __shfl_xor_sync(0xffffffffu, send, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return make_double2(__shfl_sync(0xffffffffu, s, 0), __shfl_sync(0xffffffffu, s, 16));
+}
+
 // s_sum[r] = sum_j K[r0 + r][j] s_x[j], r < R. s_x: ldk entries in shared
 // memory. A warp takes a row, or one of S equal column segments of it, with S
 // as it leaves the fewest FP64 instructions on a quarter of the SM. The lanes'
