@@ -67,7 +67,7 @@ inline size_t scaled_smem(int n, long long ldk, int m, int G) {
 // (some 5000 clocks a sweep) while the others work.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kResThreads, 1) k_bcd_scaled(const ScaledParams p) {
-    extern __shared__ __align__(16) double s_dyn[];
+    extern __shared__ __align__(16) double s_dyn_b[];
     __shared__ int s_ok, s_exit, s_flags, s_colflags;
     __shared__ double s_bl, s_rec[4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_bcd_scaled(const ScaledParam
     const int j0 = recorder ? m : own_begin(m, b, W), j1 = recorder ? m : own_begin(m, b + 1, W);
     const int C = j1 - j0, Rm = (n + W - 1) / W + 1, Cm = (m + W - 1) / W + 1;
     const int S = row_segments((int)(ldk >> 1), R);
-    double* s_v = s_dyn;                  // [ldk] column scalings of the current iterate
+    double* s_v = s_dyn_b;                  // [ldk] column scalings of the current iterate
     double* s_q = s_v + ldk;              // [2 kResThreads]
     double* s_u = s_q + 2 * kResThreads;  // [Rm] row scalings of the current iterate
     double* s_un = s_u + Rm;              // [Rm] ... of the next

@@ -25,6 +25,7 @@
 
 #include "device_util.cuh"
 #include "erot_ops.cuh"
+#include "newton_state.h"
 #include "solvers.h"
 
 namespace regot {
@@ -32,24 +33,6 @@ namespace regot {
 namespace {
 
 constexpr int kVecThreads = 64;
-
-struct NewtonState {
-    int cg_done;
-    int cg_it;
-    int cg_max;
-    unsigned counter;
-    double rz;       // r' z of the current CG residual
-    double alpha;    // CG step
-    double beta;     // CG direction update
-    double thresh2;  // stop when ||r||^2 < thresh2
-    double rnorm2;
-    double f;        // objective at gamma
-    double gnorm;
-    double gtd;      // g' d
-    double ad;       // a' d_alpha + b~' d_beta~
-    double maxabs;   // bound on |gamma|, |d| for the hi/lo split
-    unsigned long long t0;
-};
 
 // Vectors of length n + m hold (alpha part, beta part) with beta_{m-1} = 0.
 
@@ -292,7 +275,7 @@ void newton_on_plan(regot_ctx* ctx, regot_dproblem* P, ErotOps& ops, PlanCgLaunc
         L.solve(st);
         k_dir_dots<<<gv, kVecThreads, 0, st>>>(n, m, g.get(), x.get(), P->a, P->b, parts, S);
         count_launch();
-        L.line_search(x.get(), full, 1, lsout.get(), st);
+        L.line_search(x.get(), full, 1, lsout.get(), true, st);
         double tots[4];
         d2h(tots, lsout.get(), sizeof(double), st);
         read_small(ctx, &hs, S, sizeof(hs), st);
@@ -310,7 +293,7 @@ void newton_on_plan(regot_ctx* ctx, regot_dproblem* P, ErotOps& ops, PlanCgLaunc
             double steps[4] = {0, 0, 0, 0};
             for (int s = 0; s < ns; ++s) steps[s] = step * std::pow(kappa, s);
             if (k0 > 0) {  // the full step alone is evaluated already
-                L.line_search(x.get(), steps, ns, lsout.get(), st);
+                L.line_search(x.get(), steps, ns, lsout.get(), true, st);
                 ++*passes;
                 d2h(tots, lsout.get(), ns * sizeof(double), st);
                 sync(st);

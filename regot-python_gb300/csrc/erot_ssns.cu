@@ -63,6 +63,7 @@
 
 #include "device_util.cuh"
 #include "erot_ops.cuh"
+#include "newton_state.h"
 #include "solvers.h"
 #include "wolfe.h"
 
@@ -372,6 +373,7 @@ struct DenseArgs {
     float kexp_f;
     const double* gamma;  // plain: duals (beta at gamma + n)
     Exp64 ex;  // FP64 storage
+    bool stored = false;  // FP64: M is the plan itself (formed by grad())
 };
 
 template <typename TM>
@@ -384,6 +386,10 @@ __device__ __forceinline__ float t_at<float>(const DenseArgs& a, int i, int j, f
 template <>
 __device__ __forceinline__ double t_at<double>(const DenseArgs& a, int i, int j, double mv,
                                                bool& z64) {
+    if (a.stored) {
+        z64 = mv == 0.0;
+        return mv;
+    }
     return t_plain(mv, a.gamma[i], a.gamma[a.n + j], a.ex, z64);
 }
 
@@ -1493,6 +1499,12 @@ __global__ void k_ssns_grad(const Acc* rp, int nslabs, const Acc* cp, int nrb, i
     }
 }
 
+// The objective and gradient norm that the stored plan's gradient left.
+__global__ void k_ssns_take(const NewtonState* ns, SsnState* st) {
+    st->f = ns->f;
+    st->gnorm = ns->gnorm;
+}
+
 __global__ void k_ssns_move(int N, double s, const double* d, double* gamma) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < N) gamma[t] += s * d[t];
@@ -1600,6 +1612,15 @@ __global__ void k_topk_finish(const TopK* tk, int m1, TM* xcol) {
     xcol[j] = j == 0 ? (TM)0 : thr;
 }
 
+}  // namespace
+}  // namespace regot
+
+#include "newton_plan.cuh"
+#include "schur_plan.cuh"
+
+namespace regot {
+namespace {
+
 template <typename TM>
 class SsnsEngine {
 public:
@@ -1678,6 +1699,12 @@ public:
         S_.inv_reg = 1.0 / reg;
         S_.u2 = S_.p2 = S_.x2 = S_.d2 = nullptr;
         S_.w32 = nullptr;
+        if (!mixed_) {
+            ns_.alloc(1, st_);
+            ns_.zero();
+            plan_.init(P, reg, ns_.get(), ops_.err_flag(), st_);
+            schur_.init(S_, state_.get(), ops_.err_flag(), st_);
+        }
         if (mixed_) {
             u2_.alloc(n_, st_);
             d2_.alloc(n_, st_);
@@ -1703,8 +1730,18 @@ public:
         return hs;
     }
 
-    // f, g, h at gamma; leaves the FP32 split of gamma in the ops (mixed).
+    // f, g, h at gamma; leaves the FP32 split of gamma in the ops (mixed) or the
+    // plan in plan_ (FP64, where it fits).
     void grad() {
+        if (plan_.ok) {
+            plan_.form_plan(P_, gamma_.get(), st_);
+            plan_.gradient(gamma_.get(), g_.get(), h_.get(), st_);
+            k_ssns_take<<<1, 1, 0, st_>>>(ns_.get(), state_.get());
+            count_launch();
+            REGOT_CHECK_LAUNCH();
+            ++passes_;
+            return;
+        }
         const PassShape sh = ops_.buf().shape;
         ops_.maxabs(gamma_.get(), n_ + m_, nullptr, 0, &state_.get()->maxabs);
         PassParams p = ops_.base_params();
@@ -1739,6 +1776,11 @@ public:
         a.kexp_f = (float)(1.4426950408889634 / reg_);
         a.gamma = gamma_.get();
         a.ex = exp64_for(reg_);
+        if (plan_.ok) {
+            a.M = plan_.T.get();
+            a.ldm = plan_.ldk;
+            a.stored = true;
+        }
         return a;
     }
 
@@ -1802,7 +1844,7 @@ public:
     void row_stage(const DenseArgs& a, double delta2, int keep_row0) {
         if (rpath()) {
             constexpr int W = VecOf<TM>::W;
-            const int vec = (reinterpret_cast<uintptr_t>(P_->M) % 16 == 0 && P_->ldm % W == 0)
+            const int vec = (reinterpret_cast<uintptr_t>(a.M) % 16 == 0 && a.ldm % W == 0)
                                 ? 1 : 0;
             r_dispatch<TM>(r_vpt<TM>(m1_), [&](auto c) {
                 constexpr int V = decltype(c)::value;
@@ -1850,6 +1892,10 @@ public:
         const double* gsrc = gv ? gv : g_.get();
         cg_tol_ = jac ? tol_direct_ : 1e-8;
         const int maxit = jac ? max_direct_ : max_cg_;
+        if (schur_.ok) {
+            schur_.solve(gsrc, g_.get(), h_.get(), shift, cg_tol_, maxit, jac, dir_.get(), st_);
+            return;
+        }
         if (maxit != cg_max_) {
             cg_max_ = maxit;
             REGOT_CUDA(cudaMemcpyAsync(&S->max_it, &cg_max_, sizeof(int), cudaMemcpyHostToDevice,
@@ -1898,6 +1944,7 @@ public:
 
     // g'd and d'H_s d into the state.
     void dir_dots() {
+        if (schur_.ok) return;  // direction() left them there
         const int bt = 32 * kSpWarps;
         const int gr = cdiv((long long)n_ * 32, bt);
         const int gc = cdiv((long long)std::max(m1_, 1) * 32, bt);
@@ -1911,6 +1958,13 @@ public:
 
     // reg * sum T phi(s w) for up to four steps s (one dense pass).
     void ls_pass(const double* steps, int ns, double* tots) {
+        if (plan_.ok) {
+            plan_.line_search(dir_.get(), steps, ns, lsout_.get(), false, st_);
+            ++passes_;
+            d2h(tots, lsout_.get(), ns * sizeof(double), st_);
+            sync(st_);
+            return;
+        }
         ops_.maxabs(gamma_.get(), n_ + m_, dir_.get(), n_ + m_, &state_.get()->maxabs);
         PassParams p = ops_.base_params();
         p.ra = gamma_.get();
@@ -2110,6 +2164,9 @@ private:
     DBuf<TopK> topk_;
     DBuf<unsigned> hist_;
     DBuf<SsnState> state_;
+    DBuf<NewtonState> ns_;  // FP64: of plan_'s gradient
+    PlanCgLaunch plan_;
+    SchurCg schur_;
     DBuf<unsigned long long> zeros_;
     long long ldt_ = 0, lds_ = 0;
     DBuf<TM> tt_, xcol_, yrow_, rvals_, cvals_, row_scratch_;
@@ -2182,6 +2239,7 @@ void run_ssns(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int max
         E.direction(shift);
         E.dir_dots();
         hs = E.read_state();
+        if (!hs.done) ops.check_err();  // the CG's launch gave up a wait
         const double gtd = hs.gtd, dhd = hs.dhd;
         // line_selection: first candidate below f, else the best. The full
         // step is evaluated alone first (one series per entry instead of

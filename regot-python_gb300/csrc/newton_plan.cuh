@@ -14,6 +14,8 @@
 //     z_beta, so the new direction needs no third barrier.
 #pragma once
 
+#include "erot_ops.cuh"
+#include "newton_state.h"
 #include "resident.cuh"
 
 namespace regot {
@@ -33,7 +35,8 @@ struct PlanCgParams {
     unsigned* count;
     int* err;
     NewtonState* st;
-    double *hobj, *hmar, *htime;  // gradient mode: this iterate's record
+    double *hobj, *hmar, *htime;  // gradient mode: this iterate's record (or null)
+    double* hdiag;                // gradient alone: diag(H) [n + m] out, no solve
 };
 
 inline size_t plan_cg_smem(int n, long long ldk, int m, int G) {
@@ -44,7 +47,7 @@ inline size_t plan_cg_smem(int n, long long ldk, int m, int G) {
 
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p) {
-    extern __shared__ __align__(16) double s_dyn[];
+    extern __shared__ __align__(16) double s_dyn_n[];
     __shared__ int s_ok, s_stop;
     __shared__ double s_sc;  // beta, then alpha, of the step
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -54,7 +57,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     const int r0 = own_begin(n, b, G), R = own_begin(n, b + 1, G) - r0;
     const int j0 = own_begin(m, b, G), j1 = own_begin(m, b + 1, G), C = j1 - j0;
     const int Rm = (n + G - 1) / G + 1, Cm = (m + G - 1) / G + 1, Im = Rm + Cm;
-    double* s_x = s_dyn;                  // [ldk] p_beta (ones at first)
+    double* s_x = s_dyn_n;                  // [ldk] p_beta (ones at first)
     double* s_q = s_x + ldk;              // [2 kResThreads]
     double* s_u = s_q + 2 * kResThreads;  // [Rm] p_alpha of the own rows (ones at first)
     double* s_sum = s_u + Rm;             // [Rm]
@@ -140,6 +143,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
             const double ih = 1.0 / h, z = ri * ih;
             s_h[t] = h;
             s_ih[t] = ih;
+            if (p.hdiag) p.hdiag[gi] = h;
             s_r[t] = ri;
             s_z[t] = z;
             s_p[t] = z;
@@ -167,13 +171,16 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
             int stop = rr0 == 0.0 || rr0 < thresh2 ? 1 : 0;
             if (!p.rhs) {
                 const double f = reg * sr - sg, gnorm = sqrt(rr0);
-                if (gnorm < p.grad_tol || !isfinite(f)) stop = 2;  // the caller stops here
+                // the caller stops here
+                if (gnorm < p.grad_tol || !isfinite(f) || p.hdiag) stop = 2;
                 if (b == 0) {
                     p.st->f = f;
                     p.st->gnorm = gnorm;
-                    *p.hobj = f;
-                    *p.hmar = gnorm;
-                    *p.htime = (double)(globaltimer_ns() - p.st->t0) * 1e-6;
+                    if (p.hobj) {
+                        *p.hobj = f;
+                        *p.hmar = gnorm;
+                        *p.htime = (double)(globaltimer_ns() - p.st->t0) * 1e-6;
+                    }
                     if (stop == 2) p.st->cg_done = 2;
                 }
             }
@@ -284,11 +291,12 @@ struct PlanLsParams {
     double* parts;  // [grid][4]
     double* out;    // [4]
     NewtonState* st;
+    int skip;       // nothing to do where the last gradient stopped the solve
     Exp64 ex;
 };
 
 __global__ void __launch_bounds__(256) k_plan_ls(const PlanLsParams p) {
-    if (p.st->cg_done == 2) return;  // the gradient already met the tolerance
+    if (p.skip && p.st->cg_done == 2) return;  // the gradient already met the tolerance
     const unsigned per_row = (unsigned)(p.ldk >> 1);
     const long long total = (long long)p.n * per_row;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -379,7 +387,16 @@ struct PlanCgLaunch {
         if (cluster) launch_resident(k_plan_cg<true>, true, blocks, smem, st, p);
         else launch_resident(k_plan_cg<false>, false, blocks, smem, st, p);
     }
-    void line_search(const double* d, const double* steps, int nsteps, double* out, cudaStream_t st) {
+    // The gradient, objective and diag(H) alone, right after form_plan.
+    void gradient(const double* gamma, double* g, double* h, cudaStream_t st) {
+        p.gamma = gamma;
+        p.rhs = nullptr;
+        p.g = g;
+        p.hdiag = h;
+        solve(st);
+    }
+    void line_search(const double* d, const double* steps, int nsteps, double* out, bool skip,
+                     cudaStream_t st) {
         PlanLsParams q{};
         q.T = p.T;
         q.ldk = ldk;
@@ -392,6 +409,7 @@ struct PlanCgLaunch {
         q.parts = lsparts.get();
         q.out = out;
         q.st = p.st;
+        q.skip = skip ? 1 : 0;
         q.ex = exp64_for(p.reg);
         k_plan_ls<<<ls_blocks(), 256, 0, st>>>(q);
         count_launch();
