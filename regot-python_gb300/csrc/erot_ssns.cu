@@ -1661,6 +1661,8 @@ public:
         xcol_.alloc(mm, st_);
         yrow_.alloc(n_, st_);
         rcount_.alloc(n_, st_);
+        // m = 1: nothing is sparsified, the products read empty rows
+        if (m1_ <= 0) rcount_.zero();
         rcols_.alloc((size_t)n_ * m1_, st_);
         rvals_.alloc((size_t)n_ * m1_, st_);
         ccount_.alloc(mm, st_);
