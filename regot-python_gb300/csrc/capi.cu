@@ -297,6 +297,7 @@ int regot_ctx_create(int device, regot_ctx** out) {
     regot_ctx* ctx = new regot_ctx();
     ctx->device = device;
     const int rc = guarded(ctx, [&] {
+        exp64_for(1.0);  // the tables, while no stream is being captured
         REGOT_CUDA(cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking));
         ctx->stream = ctx->own_stream;
     });

@@ -154,15 +154,19 @@ int size_class(int n, int m) { return (int)std::floor(std::log2((double)n * (dou
 
 Exp64 exp64_for(double reg) {
     static std::mutex mutex;
-    static const double* tables[64] = {};  // 4096 doubles, then 6144 pairs
+    static const double2* tables[64] = {};  // 4096 pairs, then 6144 pairs
     int dev = 0;
     REGOT_CUDA(cudaGetDevice(&dev));
     require(dev < 64, "device index out of range");
     std::lock_guard<std::mutex> lock(mutex);
     if (!tables[dev]) {
-        std::vector<double> h(4096 + 2 * 6144);
+        std::vector<double2> h(4096 + 6144);
         const long double c = 0.693147180559945309417232121458176568L / 4096.0L;
-        for (int i = 0; i < 4096; ++i) h[i] = (double)std::exp2((long double)i / 4096.0L);
+        for (int i = 0; i < 4096; ++i) {
+            const long double v = std::exp2((long double)i / 4096.0L);
+            h[i].x = (double)v;
+            h[i].y = (double)((v - h[i].x) / h[i].x);
+        }
         for (int i = 0; i < 6144; ++i) {
             // phi by its series (no cancellation; |x| < 0.52, so 20 terms)
             const long double x = (i - 3072) * c;
@@ -171,17 +175,16 @@ Exp64 exp64_for(double reg) {
                 phi += term;
                 term *= x / k;
             }
-            h[4096 + 2 * i] = (double)phi;
-            h[4096 + 2 * i + 1] = (double)(phi + x);
+            h[4096 + i] = make_double2((double)phi, (double)(phi + x));
         }
-        double* d = nullptr;
-        REGOT_CUDA(cudaMalloc(&d, h.size() * sizeof(double)));
-        const cudaError_t e = cudaMemcpy(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+        double2* d = nullptr;
+        REGOT_CUDA(cudaMalloc(&d, h.size() * sizeof(double2)));
+        const cudaError_t e = cudaMemcpy(d, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) cudaFree(d);
         REGOT_CUDA(e);
         tables[dev] = d;
     }
-    return Exp64{tables[dev], reinterpret_cast<const double2*>(tables[dev] + 4096), 1.0 / reg};
+    return Exp64{tables[dev], tables[dev] + 4096, 1.0 / reg};
 }
 
 long long wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
