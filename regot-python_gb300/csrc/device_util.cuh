@@ -373,15 +373,16 @@ __device__ __forceinline__ double max_2d(const Acc* p, int count, size_t stride,
     return (double)r;
 }
 
-// Grid-wide sum of K values when one full warp of each block holds them (the
-// other warps of the block take no part). Returns true in every lane of that
+// Grid-wide sum of K values when one full warp of each of the grid's first
+// `blocks` blocks (0: all) holds them (the other warps take no part). Returns true in every lane of that
 // warp of the last block to finish, with the totals in out[]. The last warp
 // sums the per-block partials lane l taking blocks l, l + 32, ... in order,
 // then a fixed butterfly, so the result does not depend on which block
 // finishes last.
 template <int K>
 __device__ bool warp_grid_reduce(const double (&vals)[K], double* block_parts, unsigned* counter,
-                                 double (&out)[K]) {
+                                 double (&out)[K], unsigned blocks = 0) {
+    if (blocks == 0) blocks = gridDim.x;
     const int lane = threadIdx.x & 31;
     unsigned last = 0;
     double s[K];
@@ -391,7 +392,7 @@ __device__ bool warp_grid_reduce(const double (&vals)[K], double* block_parts, u
 #pragma unroll
         for (int k = 0; k < K; ++k) block_parts[(size_t)blockIdx.x * K + k] = s[k];
         __threadfence();
-        last = atomicAdd(counter, 1u) == gridDim.x - 1 ? 1u : 0u;
+        last = atomicAdd(counter, 1u) == blocks - 1 ? 1u : 0u;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
     if (!last) return false;
@@ -399,7 +400,7 @@ __device__ bool warp_grid_reduce(const double (&vals)[K], double* block_parts, u
     double part[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) part[k] = 0.0;
-    for (unsigned b = lane; b < gridDim.x; b += 32) {
+    for (unsigned b = lane; b < blocks; b += 32) {
 #pragma unroll
         for (int k = 0; k < K; ++k) part[k] += __ldcg(&block_parts[(size_t)b * K + k]);
     }

@@ -62,7 +62,7 @@ struct QState {
     int cg_it;
     int cg_max;
     int changed;
-    int pad;
+    unsigned counter_p;  // of the primal value's merges
     double dot_ab;   // alpha' a + beta' b
     double sum_a;    // 1' alpha
     double sum_b;    // 1' beta
@@ -71,25 +71,51 @@ struct QState {
     double alpha;
     double beta;
     double thresh2;
-    double prim[6];  // primal-value scalars
+    double prim[7];  // primal-value scalars
     double maxabs;
     double mu;       // shift of the Schur CG (read by its captured steps)
     int root_rounds; // Newton rounds of the last optimal_alpha / optimal_beta
     int root_unconverged;
 };
 
+// Sum of one row of per-CTA totals into *out, by a whole block of 256 threads.
+__device__ void block_total(const double* totpart, int nblocks, double* out) {
+    __shared__ double s[8];
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    double v = 0.0;
+    for (int k = tid; k < nblocks; k += 256) v += totpart[k];
+    v = warp_sum_d(v);
+    if ((tid & 31) == 0) s[tid >> 5] = v;
+    __syncthreads();
+    if (tid == 0) {
+        double r = 0.0;
+        for (int w = 0; w < 8; ++w) r += s[w];
+        *out = r;
+    }
+    __syncthreads();
+}
+
 // ---- gradient / objective merge ----
 // Blocks of (32, 8) threads: the first cdiv(n, 32) blocks own 32 rows each,
-// the rest 32 columns each; the eight threads of a row or column merge its
-// partials together (merge_2d), then warp 0 carries on.
+// the next cdiv(m, 32) 32 columns each; the eight threads of a row or column
+// merge its partials together (merge_2d), then warp 0 carries on. nt blocks
+// more sum the pass's totals beside them (into tot): a launch and its gap less
+// for each, 3 to 4 us. xr: the row scalings min(a_i / (rowsum_i / reg), 1) of the
+// primal value, if wanted.
 template <typename Acc>
 __global__ void __launch_bounds__(256) k_q_grad(const Acc* rp, int nslabs, const Acc* cp, int nrb,
                                                int n, int m, int with_counts,
                                                const double* gamma, const double* a,
                                                const double* b, double reg, double* grad,
                                                double* h1, double* h2, double* parts,
-                                               QState* st) {
-    const int nbr = (n + 31) / 32;
+                                               QState* st, const double* totpart, int nblocks,
+                                               double* tot, double* xr) {
+    const int nbr = (n + 31) / 32, nb = nbr + (m + 31) / 32;
+    if ((int)blockIdx.x >= nb) {
+        const int q = (int)blockIdx.x - nb;
+        block_total(totpart + (size_t)q * nblocks, nblocks, tot + q);
+        return;
+    }
     const bool rows = (int)blockIdx.x < nbr;
     const int t = (rows ? (int)blockIdx.x : (int)blockIdx.x - nbr) * 32 + threadIdx.x;
     const bool valid = rows ? t < n : t < m;
@@ -112,6 +138,7 @@ __global__ void __launch_bounds__(256) k_q_grad(const Acc* rp, int nslabs, const
     if (valid && rows) {
         grad[t] = sum - reg * a[t];
         if (with_counts) h1[t] = cnt;
+        if (xr) xr[t] = fmin(a[t] / (sum / reg), 1.0);
         v[0] = gamma[t] * a[t];
         v[1] = gamma[t];
     } else if (valid) {
@@ -122,25 +149,10 @@ __global__ void __launch_bounds__(256) k_q_grad(const Acc* rp, int nslabs, const
     }
     double out[3];
     __threadfence();
-    if (warp_grid_reduce<3>(v, parts, &st->counter, out) && threadIdx.x == 0) {
+    if (warp_grid_reduce<3>(v, parts, &st->counter, out, nb) && threadIdx.x == 0) {
         st->dot_ab = out[0];
         st->sum_a = out[1];
         st->sum_b = out[2];
-    }
-}
-
-// Sum of one row of per-CTA totals into *out (single block).
-__global__ void k_sum_totals(const double* totpart, int nblocks, double* out) {
-    double v = 0.0;
-    for (int k = threadIdx.x; k < nblocks; k += blockDim.x) v += totpart[k];
-    __shared__ double s[32];
-    v = warp_sum_d(v);
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += s[w];
-        *out = r;
     }
 }
 
@@ -204,6 +216,10 @@ __global__ void k_root_loop(QState* st, int cap, cudaGraphConditionalHandle h) {
 }
 
 // ---- primal value (approx_proj) ----
+// The merges use blocks of (32, 8) threads, 32 rows or columns a block, whose
+// partials eight threads merge together (merge_2d): one thread a row or column
+// was bound by the latency of its chain of loads and additions (17 and 15 us at
+// 4096 x 4096, where the three passes take 58).
 // P1 merge: x_i = min(a_i / (rowsum(D)_i / reg), 1)
 template <typename Acc>
 __global__ void k_prim1(const Acc* rp, int nslabs, int n, const double* a, double reg,
@@ -217,12 +233,15 @@ __global__ void k_prim1(const Acc* rp, int nslabs, int n, const double* a, doubl
 }
 // P2 merge: c_j = colsum(D x)/reg; y_j = min(b_j / c_j, 1); f_j = b_j - y_j c_j
 template <typename Acc>
-__global__ void k_prim2(const Acc* cp, int nrb, int m, const double* b, double reg, double* yc,
-                        double* fc, double* parts, QState* st, float4* cs) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_prim2(const Acc* cp, int nrb, int m, const double* b,
+                                               double reg, double* yc, double* fc, double* parts,
+                                               QState* st, float4* cs) {
+    const int j = blockIdx.x * 32 + threadIdx.x;
+    const double sum = merge_2d(cp + j, nrb, (size_t)m, j < m);
+    if (threadIdx.y != 0) return;
     double v[1] = {0.0};
     if (j < m) {
-        const double c = merge_strided(cp + j, nrb, (size_t)m) / reg;
+        const double c = sum / reg;
         const double y = fmin(b[j] / c, 1.0);
         const double f = b[j] - y * c;
         yc[j] = y;
@@ -235,27 +254,43 @@ __global__ void k_prim2(const Acc* cp, int nrb, int m, const double* b, double r
     }
     double out[1];
     __threadfence();
-    if (grid_reduce<1>(v, parts, &st->counter, out)) st->prim[0] = out[0];  // ||f||^2
+    if (warp_grid_reduce<1>(v, parts, &st->counter_p, out) && threadIdx.x == 0)
+        st->prim[0] = out[0];  // ||f||^2
 }
-// P3 merge: e_i = a_i - x_i A_i; sums |e|, e . Cc, x e B, e^2
+// P3 merge: e_i = a_i - x_i A_i; sums |e|, e . Cc, x e B, e^2. Two blocks more
+// sum the pass's totals into tot.
 template <typename Acc>
-__global__ void k_prim3(const Acc* rp, int nslabs, int n, const double* a, const double* xr,
-                        double reg, double* parts, QState* st) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_prim3(const Acc* rp, int nslabs, int n, const double* a,
+                                               const double* xr, double reg, double* parts,
+                                               QState* st, const double* totpart, int nblocks,
+                                               double* tot) {
+    const int nb = (n + 31) / 32;
+    if ((int)blockIdx.x >= nb) {
+        const int q = (int)blockIdx.x - nb;
+        block_total(totpart + (size_t)q * nblocks, nblocks, tot + q);
+        return;
+    }
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    double s[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        s[q] = merge_2d(rp + (size_t)q * nslabs * n + i, nslabs, (size_t)n, i < n);
+        __syncthreads();
+    }
+    if (threadIdx.y != 0) return;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
     if (i < n) {
-        const double A = merge_strided(rp + i, nslabs, (size_t)n) / reg;
-        const double B = merge_strided(rp + (size_t)nslabs * n + i, nslabs, (size_t)n) / reg;
-        const double Cc = merge_strided(rp + 2 * (size_t)nslabs * n + i, nslabs, (size_t)n);
+        const double A = s[0] / reg;
+        const double B = s[1] / reg;
         const double e = a[i] - xr[i] * A;
         v[0] = fabs(e);
-        v[1] = e * Cc;
+        v[1] = e * s[2];
         v[2] = xr[i] * e * B;
         v[3] = e * e;
     }
     double out[4];
     __threadfence();
-    if (grid_reduce<4>(v, parts, &st->counter, out)) {
+    if (warp_grid_reduce<4>(v, parts, &st->counter_p, out, nb) && threadIdx.x == 0) {
         st->prim[1] = out[0];
         st->prim[2] = out[1];
         st->prim[3] = out[2];
@@ -1551,11 +1586,10 @@ __global__ void k_time(unsigned long long t0, unsigned long long* out) {
 }  // namespace
 
 // --------------------------------------------------------------- engine --
-// Scalars of a primal value: the two P3 totals and the merged primal
-// scalars of the state.
+// Scalars of a primal value: the merged primal scalars of the state and the
+// two P3 totals.
 struct PrimRaw {
-    double tot[2];
-    double prim[5];
+    double prim[7];
 };
 
 class QrotEngine {
@@ -1569,8 +1603,8 @@ public:
         h_.alloc(N, st);
         vec_.alloc(6 * (size_t)std::max(n_, m_), st);
         // block partials of the merge kernels: up to 6 per 64-thread block,
-        // 3 per (32, 8) block of 32 rows or columns
-        parts_.alloc(std::max(6 * (size_t)cdiv(N, kVT), 3 * (size_t)(cdiv(n_, 32) + cdiv(m_, 32))),
+        // 4 per (32, 8) block of 32 rows or columns
+        parts_.alloc(std::max(6 * (size_t)cdiv(N, kVT), 4 * (size_t)(cdiv(n_, 32) + cdiv(m_, 32))),
                      st);
         state_.alloc(1, st);
         QState z{};
@@ -1602,19 +1636,20 @@ public:
         p.bitmask = mask ? bm_.get() : nullptr;
         ops_.pass(mask ? OP_Q_GRADMASK : OP_Q_GRAD, p);
         const int blocks = pass_blocks(mask ? OP_Q_GRADMASK : OP_Q_GRAD, mixed_, n_, m_);
-        k_sum_totals<<<1, 256, 0, st_>>>(ops_.buf().totpart.get(), blocks, scal_.get());
-        const int g = cdiv(n_, 32) + cdiv(m_, 32);
+        const int g = cdiv(n_, 32) + cdiv(m_, 32) + 1;
         if (mixed_)
             k_q_grad<float><<<g, dim3(32, 8), 0, st_>>>(
                 (const float*)ops_.buf().rowpart.get(), sh.nslabs,
                 (const float*)ops_.buf().colpart.get(), sh.nrb, n_, m_, mask ? 1 : 0, gamma,
-                P_->a, P_->b, reg_, grad, h_.get(), h_.get() + n_, parts_.get(), state_.get());
+                P_->a, P_->b, reg_, grad, h_.get(), h_.get() + n_, parts_.get(), state_.get(),
+                ops_.buf().totpart.get(), blocks, scal_.get(), xrow_.get());
         else
             k_q_grad<double><<<g, dim3(32, 8), 0, st_>>>(
                 (const double*)ops_.buf().rowpart.get(), sh.nslabs,
                 (const double*)ops_.buf().colpart.get(), sh.nrb, n_, m_, mask ? 1 : 0, gamma,
-                P_->a, P_->b, reg_, grad, h_.get(), h_.get() + n_, parts_.get(), state_.get());
-        count_launch(2);
+                P_->a, P_->b, reg_, grad, h_.get(), h_.get() + n_, parts_.get(), state_.get(),
+                ops_.buf().totpart.get(), blocks, scal_.get(), xrow_.get());
+        count_launch();
         REGOT_CHECK_LAUNCH();
         double sq = 0.0;
         QState hs;
@@ -1632,6 +1667,10 @@ public:
         return obj;
     }
     double tau_grad() const { return tau_grad_; }
+    // From here on eval() keeps the primal value's row scalings of its point.
+    void keep_row_scalings() { xrow_.alloc(n_, st_); }
+    // Primal value at the point of the last eval(), from the scalings it kept.
+    double primal_there(const double* gamma) { return primal(gamma, xrow_.get()); }
 
     // Line-search trial at x = xp + step d: writes grad f(x) (without the tau
     // term) to grad() and returns f(x) - f(xp) without the tau and linear
@@ -1654,21 +1693,20 @@ public:
         p.grid = &state_.get()->maxabs;
         ops_.pass(OP_Q_GRADLS, p);
         const int blocks = pass_blocks(OP_Q_GRADLS, mixed_, n_, m_);
-        k_sum_totals<<<1, 256, 0, st_>>>(ops_.buf().totpart.get(), blocks, scal_.get());
-        k_sum_totals<<<1, 256, 0, st_>>>(ops_.buf().totpart.get() + blocks, blocks,
-                                          scal_.get() + 1);
-        const int g = cdiv(n_, 32) + cdiv(m_, 32);
+        const int g = cdiv(n_, 32) + cdiv(m_, 32) + 2;
         if (mixed_)
             k_q_grad<float><<<g, dim3(32, 8), 0, st_>>>(
                 (const float*)ops_.buf().rowpart.get(), sh.nslabs,
                 (const float*)ops_.buf().colpart.get(), sh.nrb, n_, m_, 0, gamma_.get(), P_->a,
-                P_->b, reg_, grad_.get(), h_.get(), h_.get() + n_, parts_.get(), state_.get());
+                P_->b, reg_, grad_.get(), h_.get(), h_.get() + n_, parts_.get(), state_.get(),
+                ops_.buf().totpart.get(), blocks, scal_.get(), nullptr);
         else
             k_q_grad<double><<<g, dim3(32, 8), 0, st_>>>(
                 (const double*)ops_.buf().rowpart.get(), sh.nslabs,
                 (const double*)ops_.buf().colpart.get(), sh.nrb, n_, m_, 0, gamma_.get(), P_->a,
-                P_->b, reg_, grad_.get(), h_.get(), h_.get() + n_, parts_.get(), state_.get());
-        count_launch(3);
+                P_->b, reg_, grad_.get(), h_.get(), h_.get() + n_, parts_.get(), state_.get(),
+                ops_.buf().totpart.get(), blocks, scal_.get(), nullptr);
+        count_launch();
         REGOT_CHECK_LAUNCH();
         double tot[2];
         d2h(tot, scal_.get(), 2 * sizeof(double), st_);
@@ -1684,8 +1722,11 @@ public:
     // stream gets there. The three passes share one split of gamma (grid:
     // max |gamma|, from `grid` when the caller has it); the merge kernels
     // write the next passes' row and column operands into the split arrays
-    // in place.
-    void primal_launch(const double* gamma, const double* grid, PrimRaw* raw) {
+    // in place. A caller that kept the row scalings x_i = min(a_i /
+    // (rowsum(D)_i / reg), 1) of the gradient at gamma gives them in `x`: two
+    // passes then (the first would form the same row sums again).
+    void primal_launch(const double* gamma, const double* grid, PrimRaw* raw,
+                       const double* x = nullptr) {
         const PassShape sh = ops_.buf().shape;
         double* xr = vec_.get();
         double* yc = xr + std::max(n_, m_);
@@ -1698,52 +1739,61 @@ public:
         p.ra = gamma;
         p.cb = gamma + n_;
         p.grid = grid;
-        const int gn = cdiv(n_, kVT), gm = cdiv(m_, kVT);
+        const int gn = cdiv(n_, 32), gm = cdiv(m_, 32);
+        const dim3 blk(32, 8);
         float4* rs = mixed_ ? ops_.rsplit_mut() : nullptr;
         float4* cs = mixed_ ? ops_.csplit_mut() : nullptr;
-        ops_.pass(OP_Q_P1, p);
+        if (x) {
+            p.rx = x;
+            ops_.pass(OP_Q_P2, p);
+        } else {
+            ops_.pass(OP_Q_P1, p);
+            const int g1 = cdiv(n_, kVT);
+            if (mixed_)
+                k_prim1<float><<<g1, kVT, 0, st_>>>((const float*)ops_.buf().rowpart.get(),
+                                                     sh.nslabs, n_, P_->a, reg_, xr, rs);
+            else
+                k_prim1<double><<<g1, kVT, 0, st_>>>((const double*)ops_.buf().rowpart.get(),
+                                                      sh.nslabs, n_, P_->a, reg_, xr, nullptr);
+            count_launch();
+            ++passes_;
+            p.rx = x = xr;
+            ops_.pass_presplit(OP_Q_P2, p);
+        }
         if (mixed_)
-            k_prim1<float><<<gn, kVT, 0, st_>>>((const float*)ops_.buf().rowpart.get(), sh.nslabs,
-                                                 n_, P_->a, reg_, xr, rs);
-        else
-            k_prim1<double><<<gn, kVT, 0, st_>>>((const double*)ops_.buf().rowpart.get(),
-                                                  sh.nslabs, n_, P_->a, reg_, xr, nullptr);
-        p.rx = xr;
-        ops_.pass_presplit(OP_Q_P2, p);
-        if (mixed_)
-            k_prim2<float><<<gm, kVT, 0, st_>>>((const float*)ops_.buf().colpart.get(), sh.nrb,
+            k_prim2<float><<<gm, blk, 0, st_>>>((const float*)ops_.buf().colpart.get(), sh.nrb,
                                                  m_, P_->b, reg_, yc, fc, parts_.get(),
                                                  state_.get(), cs);
         else
-            k_prim2<double><<<gm, kVT, 0, st_>>>((const double*)ops_.buf().colpart.get(), sh.nrb,
+            k_prim2<double><<<gm, blk, 0, st_>>>((const double*)ops_.buf().colpart.get(), sh.nrb,
                                                   m_, P_->b, reg_, yc, fc, parts_.get(),
                                                   state_.get(), nullptr);
         p.cx = yc;
         p.cx2 = fc;
         ops_.pass_presplit(OP_Q_P3, p);
         const int blocks = pass_blocks(OP_Q_P3, mixed_, n_, m_);
-        k_sum_totals<<<1, 256, 0, st_>>>(ops_.buf().totpart.get(), blocks, scal_.get());
-        k_sum_totals<<<1, 256, 0, st_>>>(ops_.buf().totpart.get() + blocks, blocks,
-                                          scal_.get() + 1);
+        double* tot = state_.get()->prim + 5;
         if (mixed_)
-            k_prim3<float><<<gn, kVT, 0, st_>>>((const float*)ops_.buf().rowpart.get(), sh.nslabs,
-                                                 n_, P_->a, xr, reg_, parts_.get(), state_.get());
+            k_prim3<float><<<gn + 2, blk, 0, st_>>>((const float*)ops_.buf().rowpart.get(),
+                                                     sh.nslabs, n_, P_->a, x, reg_, parts_.get(),
+                                                     state_.get(), ops_.buf().totpart.get(),
+                                                     blocks, tot);
         else
-            k_prim3<double><<<gn, kVT, 0, st_>>>((const double*)ops_.buf().rowpart.get(),
-                                                  sh.nslabs, n_, P_->a, xr, reg_, parts_.get(),
-                                                  state_.get());
-        count_launch(5);
+            k_prim3<double><<<gn + 2, blk, 0, st_>>>((const double*)ops_.buf().rowpart.get(),
+                                                      sh.nslabs, n_, P_->a, x, reg_, parts_.get(),
+                                                      state_.get(), ops_.buf().totpart.get(),
+                                                      blocks, tot);
+        count_launch(2);
         REGOT_CHECK_LAUNCH();
-        passes_ += 3;
+        passes_ += 2;
         // the scalars the value is formed from, copied to *raw (page-locked:
-        // the copies are asynchronous)
-        d2h(raw->tot, scal_.get(), 2 * sizeof(double), st_);
-        d2h(raw->prim, state_.get()->prim, 5 * sizeof(double), st_);
+        // the copy is asynchronous)
+        d2h(raw->prim, state_.get()->prim, sizeof(raw->prim), st_);
     }
     // The primal value from the scalars of primal_launch (once they landed).
     double primal_value(const PrimRaw& r) const {
-        const double RM = r.tot[0] / reg_;            // <R, M>, R_ij = P_ij x_i y_j
-        const double RR = r.tot[1] / (reg_ * reg_);  // ||R||^2
+        const double RM = r.prim[5] / reg_;            // <R, M>, R_ij = P_ij x_i y_j
+        const double RR = r.prim[6] / (reg_ * reg_);  // ||R||^2
         const double f2 = r.prim[0], S = r.prim[1], eCc = r.prim[2], xeB = r.prim[3],
                      e2 = r.prim[4];
         // res = R + e f' / S (approx_proj.h:22-24)
@@ -1751,9 +1801,9 @@ public:
         const double sqn = RR + 2.0 * xeB / S + e2 * f2 / (S * S);
         return val_M + 0.5 * reg_ * sqn;
     }
-    double primal(const double* gamma, const double* grid = nullptr) {
+    double primal(const double* gamma, const double* x = nullptr) {
         PrimRaw raw;
-        primal_launch(gamma, grid, &raw);
+        primal_launch(gamma, nullptr, &raw, x);
         sync(st_);
         return primal_value(raw);
     }
@@ -1850,7 +1900,7 @@ private:
     int n_, m_;
     double reg_, tau_;
     bool mixed_;
-    DBuf<double> gamma_, grad_, h_, vec_, parts_, scal_;
+    DBuf<double> gamma_, grad_, h_, vec_, parts_, scal_, xrow_;
     DBuf<QState> state_;
     DBuf<uint32_t> bm_;
     size_t bm_words_ = 0;
@@ -2139,114 +2189,243 @@ __global__ void k_lb_axpy(const double* __restrict__ xp, const double* __restric
     if (t < N) x[t] = xp[t] + step * d[t];
 }
 
+// Sums of the merge's products, over blocks of kLbItems items, then over the
+// blocks congruent modulo kLbGroups in order, then over those groups in a tree:
+// the order (and so the bits: L-BFGS doubles a rounding difference every
+// iteration) of a single block that takes block b in lane b mod 32. Each group's
+// last block adds the group's, the last group's last block adds the groups'.
+constexpr int kLbSums = 4 + kLbPairSums;
+constexpr int kLbItems = 64, kLbGroups = 32;
+
+// Whether this block is the last of `count` to arrive at *counter; what the
+// blocks' threads wrote before is then visible to all its threads.
+__device__ __forceinline__ bool lb_last(unsigned* counter, unsigned count) {
+    __shared__ int s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(counter, 1u) == count - 1;
+        if (s_last) *counter = 0u;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
+// merge_strided's sum, of partials that come through shared memory, p[k * 65],
+// in pieces (every piece but the last a multiple of eight).
+template <typename Acc> struct StagedSum;
+template <> struct StagedSum<float> {
+    float s0 = 0.f, c0 = 0.f, s1 = 0.f, c1 = 0.f;
+    __device__ void add(const float* p, int count) {
+        int k = 0;
+        for (; k + 8 <= count; k += 8) {
+#pragma unroll
+            for (int q = 0; q < 8; q += 2) {
+                float t, e;
+                two_sum_f(s0, p[(k + q) * 65], t, e);
+                s0 = t;
+                c0 += e;
+                two_sum_f(s1, p[(k + q + 1) * 65], t, e);
+                s1 = t;
+                c1 += e;
+            }
+        }
+        for (; k < count; ++k) {
+            float t, e;
+            two_sum_f(s0, p[k * 65], t, e);
+            s0 = t;
+            c0 += e;
+        }
+    }
+    __device__ double total() const { return ((double)s0 + (double)s1) + ((double)c0 + (double)c1); }
+};
+template <> struct StagedSum<double> {
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    __device__ void add(const double* p, int count) {
+        int k = 0;
+        for (; k + 8 <= count; k += 8) {
+            s0 += p[k * 65] + p[(k + 4) * 65];
+            s1 += p[(k + 1) * 65] + p[(k + 5) * 65];
+            s2 += p[(k + 2) * 65] + p[(k + 6) * 65];
+            s3 += p[(k + 3) * 65] + p[(k + 7) * 65];
+        }
+        for (; k < count; ++k) s0 += p[k * 65];
+    }
+    __device__ double total() const { return (s0 + s1) + (s2 + s3); }
+};
+
 // Gradient of the last dense pass at the trial point x (rows, then
 // columns: D1 - reg a, D'1 - reg b), the trial's correction pair s = x - xp,
 // y = g - gp into the staging buffer of x's buffer, the record's dot
 // products (with the pair products), the pass totals (sum D^2 and, with
-// nt == 2, the remainder sum) and max |x| beside x's buffer. Without gp
-// (the first evaluation) no pair is formed.
+// nt == 2, the remainder sum), max |x| beside x's buffer and, with xr given,
+// the row scalings min(a_i / (rowsum_i / reg), 1) of the primal value. Without
+// gp (the first evaluation) no pair is formed.
+//
+// A block of 16 warps takes 64 items. All of them load the items' partials
+// (up to kLbStage of each together) into shared memory, two add them in
+// merge_strided's order, and each then forms a few of the 38 products of 32
+// items, as FP64 issue bounds them (a warp instruction holds its SM quarter for
+// some 64 clocks): pair k in warps k and k + 8, the others in warps 6, 7, 14 and
+// 15. A block more sums the pass's totals beside them. With two warps a
+// block, whose threads each read a chain of partials and formed all 38
+// products, and one last block for all sums it took 26 us at n = m = 4096.
+constexpr int kLbStage = 64;
 template <typename Acc>
-__global__ void __launch_bounds__(kLbBlock) k_lb_merge(
+__global__ void __launch_bounds__(512) k_lb_merge(
     const Acc* __restrict__ rp, int nslabs, const Acc* __restrict__ cp, int nrb, int n, int m,
     const double* __restrict__ totpart, int nblocks, int nt, const double* __restrict__ x,
     const double* __restrict__ drt, const double* __restrict__ a, const double* __restrict__ b,
     double reg, double* __restrict__ grad, const double* __restrict__ xp,
     const double* __restrict__ gp, double* __restrict__ pairs, const LbCoef* __restrict__ cf,
-    int xbuf, double* parts, unsigned* counter, LbScal* out,
-    unsigned long long* __restrict__ mxparts, double* __restrict__ xmax) {
-    constexpr int K = 4 + kLbPairSums;
-    const int N = n + m;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[K];
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = 0.0;
-    unsigned long long xbits = 0ULL;
-    if (t < N) {
-        double g, w;
-        if (t < n) {
-            g = merge_strided(rp + t, nslabs, (size_t)n) - reg * a[t];
-            w = a[t];
-        } else {
-            const int j = t - n;
-            g = merge_strided(cp + j, nrb, (size_t)m) - reg * b[j];
-            w = b[j];
-        }
-        grad[t] = g;
-        const double xt = x[t];
-        xbits = abs_bits(xt);
-        v[0] = xt * w;
-        v[1] = g * drt[t];
-        v[2] = g * g;
-        v[3] = xt * xt;
-        if (gp) {
-        const double sn = xt - xp[t], yn = g - gp[t];
-        const int stg = cf->stage[xbuf];
-        pairs[(size_t)(2 * stg) * N + t] = sn;
-        pairs[(size_t)(2 * stg + 1) * N + t] = yn;
-        int ph[kLbM];
-#pragma unroll
-        for (int k = 0; k < kLbM; ++k) ph[k] = cf->phys[k];
-#pragma unroll
-        for (int k = 0; k < kLbM; ++k) {
-            const double sk = pairs[(size_t)(2 * ph[k]) * N + t];
-            const double yk = pairs[(size_t)(2 * ph[k] + 1) * N + t];
-            v[4 + 5 * k + 0] = sn * yk;
-            v[4 + 5 * k + 1] = sk * yn;
-            v[4 + 5 * k + 2] = yn * yk;
-            v[4 + 5 * k + 3] = sk * g;
-            v[4 + 5 * k + 4] = yk * g;
-        }
-        v[4 + 5 * kLbM + 0] = sn * yn;
-        v[4 + 5 * kLbM + 1] = yn * yn;
-        v[4 + 5 * kLbM + 2] = sn * g;
-        v[4 + 5 * kLbM + 3] = yn * g;
-        }
-    }
-    // max |x| of this block (bit patterns of non-negative doubles order like
-    // the values), for the split grid of a line search from x
-    {
-        __shared__ unsigned long long s_wmax[kLbBlock / 32];
-        const unsigned long long wm = warp_max_u64(xbits);
-        if ((threadIdx.x & 31) == 0) s_wmax[threadIdx.x >> 5] = wm;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long bm = 0ULL;
-            for (int w = 0; w < kLbBlock / 32; ++w) bm = s_wmax[w] > bm ? s_wmax[w] : bm;
-            mxparts[blockIdx.x] = bm;
-        }
-    }
-    __shared__ double s_sum[K];
-    if (!lb_reduce<K>(v, parts, counter, s_sum)) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp == 0) {
-        unsigned long long bm = 0ULL;
-        for (unsigned b = lane; b < gridDim.x; b += 32) {
-            const unsigned long long q = __ldcg(&mxparts[b]);
-            bm = q > bm ? q : bm;
-        }
-        bm = warp_max_u64(bm);
-        if (lane == 0) *xmax = __longlong_as_double((long long)bm);
-    }
-    __shared__ double s_tot[2];
-    if (warp < 2) {
-        double s = 0.0;
+    int xbuf, double* parts, unsigned long long* mxparts, unsigned* counters, LbScal* out,
+    double* __restrict__ xmax, double* __restrict__ xr) {
+    static_assert(kLbM == 6, "warps 0 .. 5 (8 .. 13) take a pair each");
+    const int N = n + m, nb = (N + kLbItems - 1) / kLbItems;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = warp >> 3, task = warp & 7;
+    if ((int)blockIdx.x == nb) {
         if (warp < nt) {
+            double s = 0.0;
 #pragma unroll 4
             for (int k = lane; k < nblocks; k += 32) s += totpart[(size_t)warp * nblocks + k];
+            s = warp_sum_d(s);
+            if (lane == 0) *(warp == 0 ? &out->sq : &out->rem) = s;
         }
-        s = warp_sum_d(s);
-        if (lane == 0) s_tot[warp] = s;
+        return;
+    }
+    __shared__ Acc s_part[kLbStage * 65];
+    __shared__ double s_g[kLbItems], s_red[2][kLbSums];
+    __shared__ unsigned long long s_mx[2];
+    double* gparts = parts + (size_t)nb * kLbSums;
+    unsigned long long* gmx = mxparts + nb;
+    const int i0 = (int)blockIdx.x * kLbItems;
+    const int t = i0 + half * 32 + lane;  // this warp's items
+    const bool valid = t < N;
+    // the operands of this warp's products, under way during the merge
+    double xt = 0.0, xpt = 0.0, gpt = 0.0, u0 = 0.0, u1 = 0.0;
+    if (valid) {
+        xt = x[t];
+        if (gp) {
+            xpt = xp[t];
+            gpt = gp[t];
+            if (task < kLbM) {
+                const int ph = cf->phys[task];
+                u0 = pairs[(size_t)(2 * ph) * N + t];
+                u1 = pairs[(size_t)(2 * ph + 1) * N + t];
+            }
+        }
+        if (task == 6) {
+            u0 = t < n ? a[t] : b[t - n];
+            u1 = drt[t];
+        }
+    }
+    // ---- partials of item i0 + c: thread column c, eight partials apart ----
+    const int most = nslabs > nrb ? nslabs : nrb;
+    const int c = tid & 63, at = i0 + c;
+    const Acc* src = at < n ? rp + at : cp + (at - n);
+    const int count = at >= N ? 0 : at < n ? nslabs : nrb;
+    const size_t stride = at < n ? (size_t)n : (size_t)m;
+    StagedSum<Acc> acc;
+    for (int k0 = 0; k0 < most; k0 += kLbStage) {
+        if (k0 > 0) __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kLbStage / 8; ++q) {
+            const int k = (tid >> 6) + 8 * q;
+            if (k0 + k < count) s_part[k * 65 + c] = __ldcg(src + (size_t)(k0 + k) * stride);
+        }
+        __syncthreads();
+        if (task == 0 && valid) {
+            const int left = (t < n ? nslabs : nrb) - k0;
+            if (left > 0) acc.add(s_part + half * 32 + lane, left < kLbStage ? left : kLbStage);
+        }
+    }
+    const double sum = acc.total();  // warps 0 and 8
+    if (task == 0) {
+        double gv = 0.0;
+        if (valid) {
+            const double w = t < n ? a[t] : b[t - n];
+            gv = sum - reg * w;
+            grad[t] = gv;
+        }
+        s_g[half * 32 + lane] = gv;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        out->sq = s_tot[0];
-        out->rem = nt > 1 ? s_tot[1] : 0.0;
-        out->dab = s_sum[0];
-        out->dg = s_sum[1];
-        out->gg = s_sum[2];
-        out->xx = s_sum[3];
+    const double g = s_g[half * 32 + lane];
+    const double sn = gp ? xt - xpt : 0.0, yn = gp ? g - gpt : 0.0;
+    double* red = s_red[half];
+    if (task < kLbM) {
+        const double v[5] = {sn * u1, u0 * yn, yn * u1, u0 * g, u1 * g};
+        warp_sums_multi<5>(v, lane, [&](int q, double s) { red[4 + 5 * task + q] = s; });
+    } else if (task == 6) {
+        const double v[4] = {xt * u0, g * u1, g * g, xt * xt};
+        warp_sums_multi<4>(v, lane, [&](int q, double s) { red[q] = s; });
+    } else {
+        if (gp && valid) {
+            const int stg = cf->stage[xbuf];
+            pairs[(size_t)(2 * stg) * N + t] = sn;
+            pairs[(size_t)(2 * stg + 1) * N + t] = yn;
+        }
+        __syncwarp();
+        const double v[4] = {sn * yn, yn * yn, sn * g, yn * g};
+        warp_sums_multi<4>(v, lane, [&](int q, double s) { red[4 + 5 * kLbM + q] = s; });
+        // max |x| of the items (bit patterns of non-negative doubles order
+        // like the values), for the split grid of a line search from x
+        const unsigned long long wm = warp_max_u64(abs_bits(xt));
+        if (lane == 0) s_mx[half] = wm;
     }
-    if (threadIdx.x < kLbPairSums) out->prod[threadIdx.x] = s_sum[4 + threadIdx.x];
+    __syncthreads();
+    if (tid < kLbSums) parts[(size_t)blockIdx.x * kLbSums + tid] = s_red[0][tid] + s_red[1][tid];
+    if (tid == 64) mxparts[blockIdx.x] = s_mx[0] > s_mx[1] ? s_mx[0] : s_mx[1];
+    // two divisions, beside the arrival: nothing waits for them
+    if (xr && task == 0 && t < n) xr[t] = fmin(a[t] / (sum / reg), 1.0);
+    const int group = (int)blockIdx.x % kLbGroups, ngroups = nb < kLbGroups ? nb : kLbGroups;
+    const int gcount = (nb - group + kLbGroups - 1) / kLbGroups;
+    if (!lb_last(counters + 1 + group, (unsigned)gcount)) return;
+    if (tid < kLbSums) {
+        double acc = 0.0;
+        for (int k0 = 0; k0 < gcount; k0 += 4) {
+            double v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                v[q] = k0 + q < gcount
+                           ? __ldcg(parts + (size_t)(group + (k0 + q) * kLbGroups) * kLbSums + tid)
+                           : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (k0 + q < gcount) acc += v[q];
+        }
+        gparts[(size_t)group * kLbSums + tid] = acc;
+    } else if (warp == 2) {
+        unsigned long long v = 0ULL;
+        for (int k = lane; k < gcount; k += 32) {
+            const unsigned long long q = __ldcg(mxparts + group + k * kLbGroups);
+            v = q > v ? q : v;
+        }
+        v = warp_max_u64(v);
+        if (lane == 0) gmx[group] = v;
+    }
+    if (!lb_last(counters, (unsigned)ngroups)) return;
+    if (warp < 8) {  // values warp, warp + 8, ...
+        constexpr int PER = (kLbSums + 7) / 8;
+        double v[PER];
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int k = warp + 8 * q;
+            v[q] = lane < ngroups && k < kLbSums ? __ldcg(gparts + (size_t)lane * kLbSums + k) : 0.0;
+        }
+        warp_sums_multi<PER>(v, lane, [&](int q, double s) {
+            const int k = warp + 8 * q;
+            if (k == 0) out->dab = s;
+            else if (k == 1) out->dg = s;
+            else if (k == 2) out->gg = s;
+            else if (k == 3) out->xx = s;
+            else if (k < kLbSums) out->prod[k - 4] = s;
+        });
+    } else if (warp == 8) {
+        const unsigned long long v = warp_max_u64(lane < ngroups ? __ldcg(gmx + lane) : 0ULL);
+        if (lane == 0) *xmax = __longlong_as_double((long long)v);
+    }
 }
 
 // drt = cv g + sum_k cy[k] y_k + cs[k] s_k over the stored pairs, and g'drt.
@@ -2417,15 +2596,20 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
     DBuf<double> X(kLbBufs * (size_t)N, st), G(kLbBufs * (size_t)N, st), drt(N, st);
     // pair buffers: the ring's M plus one staging pair per iterate buffer
     DBuf<double> pairs((size_t)(M + kLbBufs) * 2 * N, st);
-    DBuf<double> parts((size_t)gN * (4 + kLbPairSums), st);
-    DBuf<unsigned> counter(1, st);
+    // block and group sums of the merge; of the direction (a value a block)
+    const int nbm = cdiv(N, kLbItems);
+    DBuf<double> parts(std::max((size_t)(nbm + kLbGroups) * kLbSums, (size_t)gN), st);
+    DBuf<unsigned> counter(1 + kLbGroups, st);
     DBuf<LbCoef> dcoef(1, st);
     DBuf<LbScal> dscal(1, st);
     DBuf<double> grid(1, st);
     // max |x| of each iterate buffer, written by the merge of the pass at x
     // (the split grid of a line search from x)
     DBuf<double> xmax(kLbBufs, st);
-    DBuf<unsigned long long> mxparts(gN, st);
+    DBuf<unsigned long long> mxparts((size_t)(nbm + kLbGroups), st);
+    // row scalings of the primal value at each gradient buffer's point
+    DBuf<double> xrow(o.prim_vals ? kLbBufs * (size_t)n : 0, st);
+    auto xrbuf = [&](int i) { return o.prim_vals ? xrow.get() + (size_t)i * n : nullptr; };
     pairs.zero();
     counter.zero();
     LbHost ring;
@@ -2468,19 +2652,19 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
         const double* xp = xpi >= 0 ? xbuf(xpi) : xbuf(xi);
         const double* gp = gpi >= 0 ? gbuf(gpi) : nullptr;
         if (mixed)
-            k_lb_merge<float><<<gN, kLbBlock, 0, st>>>(
+            k_lb_merge<float><<<nbm + 1, 512, 0, st>>>(
                 (const float*)ops.buf().rowpart.get(), sh.nslabs,
                 (const float*)ops.buf().colpart.get(), sh.nrb, n, m, ops.buf().totpart.get(),
                 blocks, nt, xbuf(xi), drt.get(), P->a, P->b, reg, gbuf(gi), xp, gp, pairs.get(),
-                dcoef.get(), xi, parts.get(), counter.get(), dscal.get(), mxparts.get(),
-                xmax.get() + xi);
+                dcoef.get(), xi, parts.get(), mxparts.get(), counter.get(), dscal.get(),
+                xmax.get() + xi, xrbuf(gi));
         else
-            k_lb_merge<double><<<gN, kLbBlock, 0, st>>>(
+            k_lb_merge<double><<<nbm + 1, 512, 0, st>>>(
                 (const double*)ops.buf().rowpart.get(), sh.nslabs,
                 (const double*)ops.buf().colpart.get(), sh.nrb, n, m, ops.buf().totpart.get(),
                 blocks, nt, xbuf(xi), drt.get(), P->a, P->b, reg, gbuf(gi), xp, gp, pairs.get(),
-                dcoef.get(), xi, parts.get(), counter.get(), dscal.get(), mxparts.get(),
-                xmax.get() + xi);
+                dcoef.get(), xi, parts.get(), mxparts.get(), counter.get(), dscal.get(),
+                xmax.get() + xi, xrbuf(gi));
         count_launch();
         REGOT_CHECK_LAUNCH();
         d2h(hs, dscal.get(), sizeof(LbScal), st);
@@ -2595,11 +2779,11 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
             prim_pending = -1;
         }
     };
-    auto iterate = [&](int xi, double gnorm) {
+    auto iterate = [&](int xi, int gi, double gnorm) {
         stamp();
         prim_finish();  // the previous iteration's trials synchronised after it
         if (o.prim_vals) {
-            E.primal_launch(xbuf(xi), xmax.get() + xi, &pslots.p->s[it & 1]);
+            E.primal_launch(xbuf(xi), xmax.get() + xi, &pslots.p->s[it & 1], xrbuf(gi));
             prim_pending = it;
         }
         hobj.push_back(last_obj);
@@ -2617,7 +2801,7 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
     param.max_iterations = max_iter;
     int niter = 0;
     double gnorm = std::sqrt(gg);
-    iterate(ix, gnorm);
+    iterate(ix, ig, gnorm);
     if (gnorm <= param.epsilon || gnorm <= param.epsilon_rel * std::sqrt(xx)) {
         niter = 1;
     } else {
@@ -2781,7 +2965,7 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
             gg = ggt;
             xx = xxt;
             gnorm = std::sqrt(gg);
-            iterate(ix, gnorm);
+            iterate(ix, ig, gnorm);
             if (gnorm <= param.epsilon || gnorm <= param.epsilon_rel * std::sqrt(xx)) break;
             if (param.max_iterations != 0 && k >= param.max_iterations) break;
             // correction pair and direction coefficients (host), then the
@@ -3445,11 +3629,9 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
         sync(st);
         return f;
     };
-    auto primal = [&](const std::vector<double>& x) {
-        if (!o.prim_vals) return 0.0;
-        h2d(E.gamma(), x.data(), N * sizeof(double), st);
-        return E.primal(E.gamma());
-    };
+    // at the point of the last grad_at
+    if (o.prim_vals) E.keep_row_scalings();
+    auto primal = [&]() { return o.prim_vals ? E.primal_there(E.gamma()) : 0.0; };
     std::vector<double> hobj, hmar, htime, hprim;
     double t0 = clock.now_ms();
     double f = grad_at(gamma, g, true);
@@ -3458,7 +3640,7 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
     hobj.push_back(f);
     hmar.push_back(gnorm / reg);
     htime.push_back(dur);
-    hprim.push_back(primal(gamma));
+    hprim.push_back(primal());
     int i;
     for (i = 0; i < max_iter; i++) {
         if (o.verbose >= 1)
@@ -3471,11 +3653,15 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
         for (int q = 0; q < N; ++q) rhs[q] = -g[q];
         solve(rhs, mu, direc);
         for (int q = 0; q < N; ++q) u[q] = gamma[q] + direc[q];
-        grad_at(u, gu, false);
+        // masked: an accepted u is the next iterate, evaluated already
+        const double fu = grad_at(u, gu, true);
         const double gunorm = lbfgs::norm(gu);
-        if (gunorm <= nu * xi) {
+        const bool accepted = gunorm <= nu * xi;
+        if (accepted) {
             gamma.swap(u);
             xi = gunorm;
+            f = fu;
+            g.swap(gu);
         } else {
             const double numer = -lbfgs::dot(gu, direc);
             const double denom = lbfgs::dot(direc, direc);
@@ -3496,13 +3682,13 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
                 lam *= gamma2;
             }
         }
-        f = grad_at(gamma, g, true);
+        if (!accepted) f = grad_at(gamma, g, true);
         gnorm = lbfgs::norm(g);
         dur = clock.now_ms() - t0;
         hobj.push_back(f);
         hmar.push_back(gnorm / reg);
         htime.push_back(htime.back() + dur);
-        hprim.push_back(primal(gamma));
+        hprim.push_back(primal());
     }
     h2d(E.gamma(), gamma.data(), N * sizeof(double), st);
     finish_qrot(E, E.gamma(), hobj, hmar, htime, hprim, i, o, res);
@@ -3539,7 +3725,9 @@ void qrot_grssn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, i
         sync(st);
         return f;
     };
-    auto primal = [&]() { return o.prim_vals ? E.primal(E.gamma()) : 0.0; };
+    // at the point of the last grad_hess
+    if (o.prim_vals) E.keep_row_scalings();
+    auto primal = [&]() { return o.prim_vals ? E.primal_there(E.gamma()) : 0.0; };
 
     std::vector<double> hobj, hmar, htime, hprim;
     double t0 = clock.now_ms();
