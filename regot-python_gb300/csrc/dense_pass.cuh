@@ -23,9 +23,10 @@
 //                  T = 2^(arg * log2(e)/reg) by ex2.approx.
 //
 // Launch configurations (PassCfg): the row-copy ring depth and the number
-// of CTAs per SM, which sets the register budget of a thread. Both keep the
-// tile shape (kRB x CW) and so the partial layouts, which the solvers'
-// finalize kernels read.
+// of CTAs per SM, which sets the register budget of a thread. The tuned two keep
+// the tile shape (kRB x CW) and so the partial layouts, which the solvers'
+// finalize kernels read; a third has the small FP64 problems' tiles
+// (tile_rows).
 #pragma once
 
 #include <atomic>
@@ -346,7 +347,8 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
     constexpr int NRa = NR > 0 ? NR : 1, NCa = NC > 0 ? NC : 1, NTa = NT > 0 ? NT : 1;
     constexpr bool ISMAX = op_is_max(OP);
     constexpr bool EROT = op_is_erot(OP);
-    constexpr int RPW = kRB / kWarps;  // rows per warp per tile (4)
+    constexpr int RB = PassCfg<CFG>::kRows;
+    constexpr int RPW = RB / kWarps;  // rows per warp per tile
     constexpr int LOGR = RPW >= 8 ? 3 : RPW >= 4 ? 2 : RPW >= 2 ? 1 : 0;
     constexpr int NS = PassCfg<CFG>::kStages;
 
@@ -354,7 +356,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
     const int n = p.n, m = p.m;
     const long long ldm = p.ldm;
     const int nslabs = (m + CW - 1) / CW;
-    const int nrb = (n + kRB - 1) / kRB;
+    const int nrb = (n + RB - 1) / RB;
     const int ntiles = nslabs * nrb;
     const int my_tiles =
         (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -369,8 +371,8 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
     constexpr size_t kCredBytes = (size_t)NCa * (kWarps / 2) * CW * sizeof(Acc);
     float4* s_colp = reinterpret_cast<float4*>(dyn_smem + (size_t)kWarps * NS * CW * sizeof(TM) +
                                                (NC > 0 ? kCredBytes : 0));  // [2][CW]
-    float4* s_rowp = s_colp + 2 * CW;                                      // [2][kRB]
-    float* s_cdp = reinterpret_cast<float*>(s_rowp + 2 * kRB);             // [2][CW] (LS only)
+    float4* s_rowp = s_colp + 2 * CW;                                      // [2][RB]
+    float* s_cdp = reinterpret_cast<float*>(s_rowp + 2 * RB);             // [2][CW] (LS only)
     __shared__ __align__(8) uint64_t s_pbar[2];
     constexpr bool STAGE_PARAMS = MIXED && !ROOT;
 
@@ -383,9 +385,9 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
     auto issue_params = [&](int kk) {
         const int t = (int)blockIdx.x + kk * (int)gridDim.x;
         const int slab = t % nslabs, rb = t / nslabs;
-        const int c0 = slab * CW, r0 = rb * kRB;
+        const int c0 = slab * CW, r0 = rb * RB;
         const int ncol = (m - c0) < CW ? (m - c0) : CW;
-        const int nrow = (n - r0) < kRB ? (n - r0) : kRB;
+        const int nrow = (n - r0) < RB ? (n - r0) : RB;
         uint64_t* bar = &s_pbar[kk & 1];
         const bool want_cd = op_uses_cd(OP) && p.cdsplit != nullptr;
         // 16-byte multiples: float4 entries always; cd floats in groups of 4
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
                                (p.rsplit ? (uint32_t)nrow * 16u : 0u) + (uint32_t)ncd * 4u;
         mbar_arrive_expect_tx(bar, bytes);
         if (p.csplit) bulk_g2s(s_colp + (kk & 1) * CW, p.csplit + c0, (uint32_t)ncol * 16u, bar);
-        if (p.rsplit) bulk_g2s(s_rowp + (kk & 1) * kRB, p.rsplit + r0, (uint32_t)nrow * 16u, bar);
+        if (p.rsplit) bulk_g2s(s_rowp + (kk & 1) * RB, p.rsplit + r0, (uint32_t)nrow * 16u, bar);
         if (ncd) bulk_g2s(s_cdp + (kk & 1) * CW, p.cdsplit + c0, (uint32_t)ncd * 4u, bar);
     };
     if (STAGE_PARAMS && threadIdx.x == 0) {
@@ -412,7 +414,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
         const int t = (int)blockIdx.x + pk * (int)gridDim.x;
         const int slab = t % nslabs, rb = t / nslabs;
         const long long c0 = (long long)slab * CW;
-        prow = (long long)rb * kRB + rw0;
+        prow = (long long)rb * RB + rw0;
         psrc = Mb + prow * ldm + c0;
         pseg = (uint32_t)((ldm - c0) < CW ? (ldm - c0) : CW) * (uint32_t)sizeof(TM);
     };
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
     for (int k = 0; k < my_tiles; ++k) {
         const int t = (int)blockIdx.x + k * (int)gridDim.x;
         const int slab = t % nslabs, rb = t / nslabs;
-        const int c0 = slab * CW, r0 = rb * kRB;
+        const int c0 = slab * CW, r0 = rb * RB;
         const int seg = (int)((ldm - c0) < CW ? (ldm - c0) : CW);
 
         if constexpr (STAGE_PARAMS) {
@@ -559,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, PassCfg<CFG>::kMinBlocks) dense_pass
                     if constexpr (ROOT) {
                         prad[r2] = p.ra ? p.ra[i] : 0.0;
                     } else if constexpr (MIXED) {
-                        const float4 r = p.rsplit ? s_rowp[(k & 1) * kRB + (i - r0)]
+                        const float4 r = p.rsplit ? s_rowp[(k & 1) * RB + (i - r0)]
                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
                         prh[r2] = r.x;
                         prlk[r2] = EROT ? __fmul_rn(r.y, kexp) : r.y;
@@ -991,7 +993,7 @@ constexpr size_t pass_smem_bytes() {
     constexpr int NS = PassCfg<CFG>::kStages;
     return (size_t)kWarps * NS * CW * sizeof(TM) +
            (size_t)(op_nc(OP) > 0 ? op_nc(OP) : 0) * (kWarps / 2) * CW * sizeof(Acc) +
-           2 * ((size_t)CW * 16 + (size_t)kRB * 16 + (op_uses_cd(OP) ? (size_t)CW * 4 : 0));
+           2 * ((size_t)CW * 16 + (size_t)PassCfg<CFG>::kRows * 16 + (op_uses_cd(OP) ? (size_t)CW * 4 : 0));
 }
 
 // Opt in to the pass's dynamic shared memory, once per device (host threads

@@ -294,7 +294,9 @@ void ErotOps::optimal_beta(const double* alpha, double* beta, double* mx) {
     p.grid = mx;
     p.cb = anchor_.get();
     const int nrb = cdiv(n_, kRB);
+    int sums = buf_.shape.nrb;  // partials a column
     if (!mixed_ && nrb <= 65535) {
+        sums = nrb;  // at most the shape's
         k_colsum64<<<dim3(cdiv(m_, 32), nrb), 256, 0, st_>>>(
             static_cast<const double*>(P_->M), P_->ldm, n_, m_, alpha, anchor_.get(), exp64_for(reg_),
             reinterpret_cast<double*>(buf_.colpart.get()));
@@ -303,8 +305,8 @@ void ErotOps::optimal_beta(const double* alpha, double* beta, double* mx) {
     } else {
         pass(OP_E_COL, p);
     }
-    REGOT_LAUNCH_ACC(k_col_lse, m_, buf_.colpart.get(), buf_.shape.nrb, m_, anchor_.get(),
-                     P_->logb, reg_, beta);
+    REGOT_LAUNCH_ACC(k_col_lse, m_, buf_.colpart.get(), sums, m_, anchor_.get(), P_->logb, reg_,
+                     beta);
 }
 
 // sinkhorn_problem_bcd.cpp:177-201, the row analogue of optimal_beta.

@@ -50,6 +50,7 @@ void* dev_alloc(size_t bytes, cudaStream_t st);
 constexpr int kThreads = 256;            // 8 warps per CTA
 constexpr int kWarps = kThreads / 32;
 constexpr int kRB = 64;                  // rows per tile (8 per warp)
+constexpr int kSmallRB = 16;             // ... of small FP64 problems (tile_rows)
 
 template <typename TM> struct Geo;
 template <> struct Geo<float> {
@@ -154,8 +155,13 @@ struct PassShape {
 // depth of each warp's ring of row buffers. The autotuner (passes.cu)
 // chooses one per (device, precision, pass, size class of n m).
 template <int CFG> struct PassCfg;
-template <> struct PassCfg<0> { static constexpr int kMinBlocks = 2, kStages = 4; };
-template <> struct PassCfg<1> { static constexpr int kMinBlocks = 1, kStages = 8; };
+template <> struct PassCfg<0> { static constexpr int kMinBlocks = 2, kStages = 4, kRows = kRB; };
+template <> struct PassCfg<1> { static constexpr int kMinBlocks = 1, kStages = 8, kRows = kRB; };
+// tiles of kSmallRB rows, for the problems of tile_rows() == kSmallRB (not tuned)
+constexpr int kSmallCfg = 2;
+template <> struct PassCfg<kSmallCfg> {
+    static constexpr int kMinBlocks = 2, kStages = 4, kRows = kSmallRB;
+};
 constexpr int kPassConfigs = 2;
 template <typename TM, int CFG>
 void launch_pass_cfg(int op, const PassParams& p, cudaStream_t st, int blocks);
@@ -183,11 +189,23 @@ int device_sm_count();
 // number of tiles); per-CTA totals of that pass have this many entries.
 int pass_blocks(int op, bool mixed, int n, int m);
 
+// Rows of the tiles of an n x m problem. FP64 issue bounds the FP64 passes, so
+// that a pass takes as long as the SM with the most rows: 64-row tiles give a
+// 1023 x 769 problem 64 blocks on 152 SMs, 16-row tiles 256. Up to 2^24 entries
+// (1024 tiles of 64 rows on 304 resident blocks) the finer tiles even out the
+// last round; beyond, their four times as many column partials (1/16 of M's
+// memory a sum) buy nothing. FP32 passes of small problems are bound by
+// latencies instead.
+template <typename TM>
+inline int tile_rows(int n, int m) {
+    return sizeof(TM) == 8 && (long long)n * m <= (1LL << 24) ? kSmallRB : kRB;
+}
+
 template <typename TM>
 inline PassShape pass_shape(int n, int m) {
     PassShape s;
     s.nslabs = cdiv(m, Geo<TM>::CW);
-    s.nrb = cdiv(n, kRB);
+    s.nrb = cdiv(n, tile_rows<TM>(n, m));
     s.ntiles = s.nslabs * s.nrb;
     const int cap = device_sm_count() * kMaxPassCtasPerSm;
     s.nblocks = s.ntiles < cap ? s.ntiles : cap;

@@ -278,15 +278,22 @@ namespace {
 int occupancy(int op, bool mixed, int cfg) {
     int dev = 0;
     REGOT_CUDA(cudaGetDevice(&dev));
-    static std::atomic<int> cache[64][2][kPassConfigs][OP_COUNT] = {};
+    static std::atomic<int> cache[64][2][kPassConfigs + 1][OP_COUNT] = {};
     const bool ok = dev < 64 && op >= 0 && op < OP_COUNT;
     int occ = ok ? cache[dev][mixed][cfg][op].load(std::memory_order_relaxed) : 0;
     if (!occ) {
-        if (cfg == 0) occ = mixed ? occupancy_cfg<float, 0>(op) : occupancy_cfg<double, 0>(op);
+        if (cfg == kSmallCfg) occ = occupancy_cfg<double, kSmallCfg>(op);
+        else if (cfg == 0) occ = mixed ? occupancy_cfg<float, 0>(op) : occupancy_cfg<double, 0>(op);
         else occ = mixed ? occupancy_cfg<float, 1>(op) : occupancy_cfg<double, 1>(op);
         if (ok) cache[dev][mixed][cfg][op].store(occ, std::memory_order_relaxed);
     }
     return occ;
+}
+
+// The configuration a pass runs in: the tuned one, or that of the small FP64 tiles.
+int run_config(int op, bool mixed, int n, int m) {
+    if (!mixed && tile_rows<double>(n, m) == kSmallRB) return kSmallCfg;
+    return pass_config(op, mixed, n, m);
 }
 
 int blocks_for(int op, bool mixed, int n, int m, int cfg) {
@@ -307,14 +314,20 @@ void launch_pass(int op, const PassParams& p, cudaStream_t st) {
     q.inv_reg_d = 1.0 / p.reg;
     q.wait_limit = wait_limit();
     constexpr bool mixed = std::is_same<TM, float>::value;
-    const int cfg = pass_config(op, mixed, p.n, p.m);
+    const int cfg = run_config(op, mixed, p.n, p.m);
     const int blocks = blocks_for(op, mixed, p.n, p.m, cfg);
+    if constexpr (!mixed) {
+        if (cfg == kSmallCfg) {
+            launch_pass_cfg<double, kSmallCfg>(op, q, st, blocks);
+            return;
+        }
+    }
     if (cfg == 0) launch_pass_cfg<TM, 0>(op, q, st, blocks);
     else launch_pass_cfg<TM, 1>(op, q, st, blocks);
 }
 
 int pass_blocks(int op, bool mixed, int n, int m) {
-    return blocks_for(op, mixed, n, m, pass_config(op, mixed, n, m));
+    return blocks_for(op, mixed, n, m, run_config(op, mixed, n, m));
 }
 
 void launch_split(const PassParams& p, float4* rs, float4* cs, float* cds, cudaStream_t st) {
