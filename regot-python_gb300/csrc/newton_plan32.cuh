@@ -12,7 +12,10 @@
 // row buffers filled by cp.async four rows ahead - across tiles and across
 // steps, as T does not change, so the first rows of a step are in flight
 // during the barriers before it. Odd steps walk the tiles backwards: what the
-// end of a step left in L2 is read first by the next.
+// end of a step left in L2 is read first by the next. Tiles of one slab that
+// follow each other in a group share the column entries of the direction.
+// (Rows straight into registers, two or four ahead, took longer than the ring:
+// a pair of tiles about 30 instead of 20 thousand clocks.)
 //
 // A step has three barriers (the captured step had four kernel boundaries):
 // the next direction's entries are formed where they are used, from the
@@ -129,17 +132,23 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
     // nothing may be in flight when the block ends
     auto drain = []() { asm volatile("cp.async.wait_all;" ::: "memory"); };
 
+    // Sums over the warp of v0 (in the lower lanes) and v1 (in the upper), each in
+    // warp_sum_d's order: half the additions of two such sums.
+    auto pair_sum = [&](double v0, double v1) {
+        const bool upper = (lane & 16) != 0;
+        const double send = upper ? v0 : v1;
+        double s = (upper ? v1 : v0) + __shfl_xor_sync(0xffffffffu, send, 16);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
     // Two sums over all items, one value each a thread and round of 512 items
     // (v0, v1 by item), as grid_reduce<2> forms them over blocks of 64 threads:
     // publish the groups' sums; after a barrier, final_sums leaves the totals
     // in lane 0 of warp 0.
     auto publish2 = [&](int t, double v0, double v1) {
-        v0 = warp_sum_d(v0);
-        v1 = warp_sum_d(v1);
-        if (lane == 0) {
-            s_w[0][warp] = v0;
-            s_w[1][warp] = v1;
-        }
+        const double v = pair_sum(v0, v1);
+        if ((lane & 15) == 0) s_w[lane >> 4][warp] = v;
         __syncthreads();
         if ((tid & 63) < 2 && t - (tid & 63) < items) {
             const int q = tid & 63, w = warp & ~1;
@@ -156,12 +165,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
                 a1 += q.y;
             }
             __syncwarp();
-            a0 = warp_sum_d(a0);
-            a1 = warp_sum_d(a1);
-            if (lane == 0) {
-                s_w[0][warp] = a0;
-                s_w[1][warp] = a1;
-            }
+            const double a = pair_sum(a0, a1);
+            if ((lane & 15) == 0) s_w[lane >> 4][warp] = a;
         }
         __syncthreads();
         o0 = tid == 0 ? s_w[0][0] + s_w[0][1] : 0.0;
@@ -218,14 +223,18 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
             const double z = __ldcg(p.z + at);
             return it == 0 ? z : fma(beta, __ldcg(p_old + at), z);
         };
+        int cx_slab = -1;  // whose entries s_cx holds
 #pragma unroll 1
         for (int k = 0; k < my_tiles; ++k) {
             const int t = tile_at(it, k);
             const int slab = t % nslabs, rb = t / nslabs;
             const int c0 = slab * CW, r0 = rb * kRB;
             const int seg = (int)((p.ldt - c0) < CW ? (p.ldt - c0) : CW);
-            for (int c = gt; c < CW; c += GT)
-                s_cx[c] = c0 + c < m ? (float)direction(n + c0 + c) : 0.f;
+            if (slab != cx_slab) {
+                cx_slab = slab;
+                for (int c = gt; c < CW; c += GT)
+                    s_cx[c] = c0 + c < m ? (float)direction(n + c0 + c) : 0.f;
+            }
             if (gt < kRB) s_rx[gt] = r0 + gt < n ? (float)direction(r0 + gt) : 0.f;
             group_sync();
             float cx[16], cacc[16], rowv[RPW];
@@ -330,6 +339,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
             const bool row = g < nar;
             const int item = (row ? g : g - nar) * 32 + lane;
             const bool ok = g < ae && (row ? item < n : item < m - 1);
+            const int at = row ? item : n + item;
+            const bool have = g < ae && (row ? item < n : item < m);
+            // under way while the partials are added
+            double pv = 0.0, hd = 0.0;
+            if (wg == 0 && have) {
+                pv = __ldcg(p_new + at);
+                hd = __ldg(p.hdiag + at);
+            }
             float sum = 0.f, err = 0.f;
             if (ok) {
                 const float* src = row ? p.rowpart + item : p.colpart + item;
@@ -365,10 +382,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
                 }
                 const double tp = (double)ss + (double)cc;
                 double py = 0.0;
-                const int at = row ? item : n + item;
-                if (g < ae && (row ? item < n : item < m)) {
-                    const double pv = __ldcg(p_new + at);
-                    const double y = ok ? fma(__ldg(p.hdiag + at), pv, tp / p.reg) : 0.0;
+                if (have) {
+                    const double y = ok ? fma(hd, pv, tp / p.reg) : 0.0;
                     __stcg(p.y + at, y);
                     py = pv * y;
                 }
@@ -383,6 +398,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
             drain();
             return;
         }
+        // the first round's y, under way while alpha is formed
+        double y0 = 0.0;
+        if (tid < items && i0 + tid < N) y0 = __ldcg(p.y + i0 + tid);
         if (warp == 0) {
             double s = 0.0;
             for (int g = lane; g < nab; g += 32 * 8) {
@@ -407,7 +425,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
                 double v0 = 0.0, v1 = 0.0;
                 if (t < items && i0 + t < N) {
                     s_x[t] = fma(alpha, s_p[t], s_x[t]);
-                    const double ri = fma(-alpha, __ldcg(p.y + i0 + t), s_r[t]);
+                    const double yv = t0 == 0 ? y0 : __ldcg(p.y + i0 + t);
+                    const double ri = fma(-alpha, yv, s_r[t]);
                     s_r[t] = ri;
                     const double zi = ri / s_h[t];
                     s_z[t] = zi;
