@@ -1950,7 +1950,8 @@ private:
                 k_root_update<<<cdiv(m_, 32), dim3(32, 8), 0, st_>>>(
                     (const double*)ops_.buf().colpart.get(), sh.nrb, m_, P_->b, reg_, x,
                     vec_.get(), state_.get());
-            k_root_loop<<<1, 1, 0, st_>>>(state_.get(), len + 2, h);
+            // each round drops entries of some row's (column's) active set
+            k_root_loop<<<1, 1, 0, st_>>>(state_.get(), std::max(n_, m_) + 2, h);
             count_launch(2);
         } catch (...) {
             cudaGraph_t tmp = nullptr;
