@@ -958,6 +958,13 @@ struct DsmCgArgs {
     int* err;
 };
 
+// A CTA's index-list slices go to shared memory when they fit.
+struct DwCgArgs {
+    DsmCgArgs d;
+    int idx_cap;  // ints of dynamic shared memory after the vectors for the
+                  // CTA's index-list slices (each slice fits when >= nnz)
+};
+
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
@@ -1012,63 +1019,51 @@ struct DsSlices {
     }
 };
 
-// sum_{k in [ptr[i], ptr[i+1])} v[idx[k]] with v in this CTA's shared memory
-template <bool MIXED>
-__device__ __forceinline__ double list_sum_s(const int* ptr, const int* idx, int i,
-                                             const void* vs) {
-    const int b = __ldg(ptr + i), e = __ldg(ptr + i + 1);
+// FP64 sum of v[idx[k]], k in [b, e): v in this CTA's shared memory, idx there
+// or in global memory.
+__device__ __forceinline__ double gather_sum_d(const int* idx, int b, int e, const double* v) {
+    double s0 = 0.0, s1 = 0.0;
     int k = b;
-    if (MIXED) {
-        const float2* v2 = static_cast<const float2*>(vs);
-        float s = 0.f, er = 0.f;
-        for (; k + 4 <= e; k += 4) {
-            float2 u[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) u[q] = v2[__ldg(idx + k + q)];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) cadd(s, er, u[q]);
-        }
-        for (; k < e; ++k) cadd(s, er, v2[__ldg(idx + k)]);
-        return (double)s + (double)er;
-    } else {
-        const double* v = static_cast<const double*>(vs);
-        double acc = 0.0;
-        for (; k + 4 <= e; k += 4) {
-            double u[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) u[q] = v[__ldg(idx + k + q)];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc += u[q];
-        }
-        for (; k < e; ++k) acc += v[__ldg(idx + k)];
-        return acc;
+    for (; k + 2 <= e; k += 2) {
+        const double u0 = v[idx[k]], u1 = v[idx[k + 1]];
+        s0 += u0;
+        s1 += u1;
     }
-}
-template <bool MIXED>
-__device__ __forceinline__ void put_slot(void* vs, int j, double v) {
-    if (MIXED) static_cast<float2*>(vs)[j] = split_f2(v);
-    else static_cast<double*>(vs)[j] = v;
+    if (k < e) s0 += v[idx[k]];
+    return s0 + s1;
 }
 
 struct DsShared {
-    double vals[kDsT];
+    double wsum[kDsT / 32];
     double red[2][16];  // CTA totals of p'q and r'r, by sending CTA
     double bc[2];       // the cluster total and the quotient formed from it
-    uint64_t bar[4];    // arrivals of t, p, the p'q totals, the r'r totals
+    uint64_t bar[4];    // arrivals of t and the p'q totals, r and the r'r totals, -, x
     int abort;
 };
 
-template <bool MIXED>
-__global__ void __launch_bounds__(kDsT, 1) k_schur_cg_dsm(DsmCgArgs da) {
+// K: rows and columns per thread (the CTA's slices hold at most K * kDsT). Each
+// thread keeps its rows' and columns' CG state in registers and the CTA's
+// slices of the index lists sit in shared memory: after a cluster-scope
+// acquire, global loads no longer hit L1, and the L2 round trips of re-reading
+// pointers, indices and state every step were most of it (19.5 thousand clocks
+// a step at 1023 x 769 with 1.4 entries a row, 8 to 9 now; what is left is two
+// exchanges and the chains of FP64 additions and divisions between them). The
+// CTAs send r, not p: a row keeps s = sigma p, updated like p, so r travels
+// with the r'r totals; and p' Delta p is formed from p and s, so its totals
+// travel with t. Its rounding error is of the order of eps sum (h2 + mu) p^2,
+// as that of sum p y is.
+template <int K>
+__global__ void __launch_bounds__(kDsT, 1) k_schur_cg_dsm(DwCgArgs wa) {
     extern __shared__ __align__(16) unsigned char ds_dyn[];
     __shared__ DsShared sh;
-    const ClusterCgArgs& a = da.c;
+    const ClusterCgArgs& a = wa.d.c;
     const unsigned nc = cluster_nctarank(), rk = cluster_ctarank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n, m = a.m;
     const double mu = a.mu;
-    void* Ts = ds_dyn;                                        // (n + 1) & ~1 slots
-    void* Ps = ds_dyn + (size_t)((n + 1) & ~1) * 8;           // (m + 1) & ~1 slots
+    double* Ts = reinterpret_cast<double*>(ds_dyn);
+    double* Ps = Ts + ((n + 1) & ~1);
+    int* sidx = reinterpret_cast<int*>(Ps + ((m + 1) & ~1));
     const DsSlices rs(n, nc), cs(m, nc);
     const int r0 = rs.begin(n, rk), r1 = rs.end(n, rk);
     const int c0 = cs.begin(m, rk), c1 = cs.end(m, rk);
@@ -1083,136 +1078,204 @@ __global__ void __launch_bounds__(kDsT, 1) k_schur_cg_dsm(DsmCgArgs da) {
         sm100::fence_mbar_init();
         sh.abort = 0;
     }
+    if (tid < kDsT / 32) sh.wsum[tid] = 0.0;  // of the warps without columns
+    // this CTA's slices of the index lists, in shared memory when they fit
+    const int rbase = __ldg(a.rowptr + r0), rcount = __ldg(a.rowptr + r1) - rbase;
+    const int cbase = __ldg(a.colptr + c0), ccount = __ldg(a.colptr + c1) - cbase;
+    const bool fit = rcount + ccount <= wa.idx_cap;
+    const int* ridx = fit ? sidx : a.colidx + rbase;
+    const int* cidx = fit ? sidx + rcount : a.rowidx + cbase;
+    if (fit) {
+        for (int k = tid; k < rcount; k += kDsT) sidx[k] = __ldg(a.colidx + rbase + k);
+        for (int k = tid; k < ccount; k += kDsT) sidx[rcount + k] = __ldg(a.rowidx + cbase + k);
+    }
+    // per-thread rows i = r0 + tid + u kDsT and columns j = c0 + tid + u kDsT
+    int rb[K], re[K], cb[K], ce[K];
+    double dinv[K], hm[K], x[K], r[K], p[K], y[K], sp[K];
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+        const int i = r0 + tid + u * kDsT, j = c0 + tid + u * kDsT;
+        rb[u] = re[u] = cb[u] = ce[u] = 0;
+        dinv[u] = hm[u] = x[u] = r[u] = p[u] = y[u] = sp[u] = 0.0;
+        if (i < r1) {
+            rb[u] = __ldg(a.rowptr + i) - rbase;
+            re[u] = __ldg(a.rowptr + i + 1) - rbase;
+            dinv[u] = 1.0 / (a.h1[i] + mu);
+            Ts[i] = a.w[i] * dinv[u];
+        }
+        if (j < c1) {
+            cb[u] = __ldg(a.colptr + j) - cbase;
+            ce[u] = __ldg(a.colptr + j + 1) - cbase;
+            hm[u] = a.h2[j] + mu;
+        }
+    }
     uint32_t ph = 0u;  // bit q: the parity barrier q waits for next
     // barriers initialised and every CTA running before any remote access
     cluster_barrier();
 
-    // Sends this CTA's slice [b, b + bytes) of vector buffer `vs` to every
-    // other CTA, then waits for theirs (barrier q).
-    auto exchange = [&](void* vs, int b, uint32_t bytes, uint32_t in_bytes, int q) -> bool {
+    // One round on barrier q: send() passes this CTA's slice [b, b + bytes) of vs
+    // to every other CTA and, with slot >= 0, the CTA total of v; wait() returns
+    // in a thread once all of theirs are here. The last warp, which seldom has
+    // rows, then forms the cluster total and a quotient (finish) while the others
+    // gather; settle() synchronises and says whether every wait ended.
+    constexpr int kSumWarp = kDsT / 32 - 1;
+    auto send = [&](int q, double* vs, int b, uint32_t bytes, uint32_t in_bytes, int slot, double v) {
+        if (slot >= 0 && (r0 + warp * 32 < r1 || c0 + warp * 32 < c1)) {
+            const double ws = warp_allsum_d(v);
+            if (lane == 0) sh.wsum[warp] = ws;
+        }
         sm100::fence_proxy_async_smem();
         __syncthreads();
+        const uint32_t bar = sm100::smem_u32(&sh.bar[q]);
+        const bool other = lane < (int)nc && lane != (int)rk;
         if (warp == 0) {
-            const uint32_t src = sm100::smem_u32(vs) + (uint32_t)b * 8u;
-            const uint32_t bar = sm100::smem_u32(&sh.bar[q]);
-            if (bytes > 0 && lane < (int)nc && lane != (int)rk)
-                bulk_s2cluster(mapa_u32(src, lane), src, bytes, mapa_u32(bar, lane));
-            if (lane == 0) {
-                sm100::mbar_arrive_expect_tx(&sh.bar[q], in_bytes);
-                if (!mbar_wait_cluster(&sh.bar[q], (ph >> q) & 1u, da.polls)) {
-                    sh.abort = 1;
-                    atomicExch(da.err, 1);
-                }
-            }
-        }
-        __syncthreads();
-        ph ^= 1u << q;
-        return sh.abort == 0;
-    };
-    // Cluster total of one value per thread; bc[1] = num / total (or, with
-    // inv, total / num), formed once.
-    auto all_sum = [&](double v, int slot, double num, bool inv) -> bool {
-        const int q = 2 + slot;
-        sh.vals[tid] = v;
-        __syncthreads();
-        if (warp == 0) {
-            double s = 0.0;
-#pragma unroll
-            for (int k = 0; k < kDsT / 32; ++k) s += sh.vals[k * 32 + lane];
-            s = warp_allsum_d(s);
-            const uint32_t bar = sm100::smem_u32(&sh.bar[q]);
-            if (lane == (int)rk) sh.red[slot][rk] = s;
-            else if (lane < (int)nc)
-                st_async_f64(mapa_u32(sm100::smem_u32(&sh.red[slot][rk]), lane), s,
-                             mapa_u32(bar, lane));
-            if (lane == 0) {
-                sm100::mbar_arrive_expect_tx(&sh.bar[q], (nc - 1) * 8u);
-                if (!mbar_wait_cluster(&sh.bar[q], (ph >> q) & 1u, da.polls)) {
-                    sh.abort = 1;
-                    atomicExch(da.err, 1);
-                }
-            }
+            if (lane == 0)
+                sm100::mbar_arrive_expect_tx(&sh.bar[q], in_bytes + (slot >= 0 ? (nc - 1) * 8u : 0u));
             __syncwarp();
+            const uint32_t src = sm100::smem_u32(vs) + (uint32_t)b * 8u;
+            if (bytes > 0 && other)
+                bulk_s2cluster(mapa_u32(src, lane), src, bytes, mapa_u32(bar, lane));
+        }
+        if (slot >= 0 && warp == kSumWarp) {
+            double t = lane < kDsT / 32 ? sh.wsum[lane] : 0.0;
+#pragma unroll
+            for (int o = kDsT / 64; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (lane == (int)rk) sh.red[slot][rk] = t;
+            else if (other)
+                st_async_f64(mapa_u32(sm100::smem_u32(&sh.red[slot][rk]), lane), t,
+                             mapa_u32(bar, lane));
+        }
+        __syncwarp();
+    };
+    auto wait = [&](int q) {
+        if (!mbar_wait_cluster(&sh.bar[q], (ph >> q) & 1u, wa.d.polls)) {
+            sh.abort = 1;
+            atomicExch(wa.d.err, 1);
+        }
+        __syncwarp();
+        ph ^= 1u << q;
+    };
+    // bc[0] = the cluster total of slot, bc[1] = num / total, or total / num with inv
+    auto finish = [&](int slot, double num, bool inv) {
+        if (warp == kSumWarp) {
             double c = lane < (int)nc ? sh.red[slot][lane] : 0.0;
-            c = warp_allsum_d(c);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
             if (lane == 0) {
                 sh.bc[0] = c;
                 sh.bc[1] = inv ? c / num : num / c;
             }
+            __syncwarp();
         }
+    };
+    auto settle = [&]() -> bool {
         __syncthreads();
-        ph ^= 1u << q;
         return sh.abort == 0;
     };
 
-    bool ok = true;
-    for (int i = r0 + tid; i < r1; i += kDsT) {
-        const double di = 1.0 / (a.h1[i] + mu);
-        a.dinv[i] = di;
-        put_slot<MIXED>(Ts, i, a.w[i] * di);
-    }
-    ok = exchange(Ts, r0, rs.bytes(n, rk), t_in, 0);
-    double part = 0.0;
+    // v = w / (h1 + mu), zy = z - sigma' v
+    send(0, Ts, r0, rs.bytes(n, rk), t_in, -1, 0.0);
+    wait(0);
+    bool ok = settle();
+    double rr = 0.0, beta = 0.0, part = 0.0;
     if (ok) {
-        for (int j = c0 + tid; j < c1; j += kDsT) {
-            const double zy = a.z[j] - list_sum_s<MIXED>(a.colptr, a.rowidx, j, Ts);
-            a.x[j] = 0.0;
-            a.r[j] = zy;
-            a.p[j] = zy;
-            put_slot<MIXED>(Ps, j, zy);
-            part += zy * zy;
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const int j = c0 + tid + u * kDsT;
+            if (j < c1) {
+                r[u] = a.z[j] - gather_sum_d(cidx, cb[u], ce[u], Ts);
+                Ps[j] = r[u];
+                part += r[u] * r[u];
+            }
         }
-        ok = all_sum(part, 1, 1.0, false);
+        __syncwarp();
+        send(1, Ps, c0, cs.bytes(m, rk), p_in, 1, part);
+        wait(1);
+        finish(1, 1.0, true);
+        ok = settle();
+        rr = sh.bc[0];
     }
-    double rr = sh.bc[0];
-    if (ok) ok = exchange(Ps, c0, cs.bytes(m, rk), p_in, 1);
     const double thresh2 = fmax(a.tol * a.tol * rr, 2.2250738585072014e-308);
     bool done = rr == 0.0 || rr < thresh2;
     int it = 0;
+    double g[K];  // (sigma r)_i of the own rows
+#pragma unroll
+    for (int u = 0; u < K; ++u) g[u] = ok && !done ? gather_sum_d(ridx, rb[u], re[u], Ps) : 0.0;
     while (ok && !done) {
-        for (int i = r0 + tid; i < r1; i += kDsT)
-            put_slot<MIXED>(Ts, i, list_sum_s<MIXED>(a.rowptr, a.colidx, i, Ps) * a.dinv[i]);
-        if (!(ok = exchange(Ts, r0, rs.bytes(n, rk), t_in, 0))) break;
+        // p = r + beta p, s = sigma p = g + beta s, t = s / (h1 + mu), and
+        // p' Delta p = sum (h2 + mu) p^2 - sum s t: known before t is exchanged
         part = 0.0;
-        for (int j = c0 + tid; j < c1; j += kDsT) {
-            const double u = list_sum_s<MIXED>(a.colptr, a.rowidx, j, Ts);
-            const double pj = a.p[j];
-            const double yj = a.h2[j] * pj + mu * pj - u;
-            a.y[j] = yj;
-            part += pj * yj;
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const int i = r0 + tid + u * kDsT;
+            if (i < r1) {
+                sp[u] = fma(beta, sp[u], g[u]);
+                const double t = sp[u] * dinv[u];
+                Ts[i] = t;
+                part = fma(-sp[u], t, part);
+            }
+            p[u] = fma(beta, p[u], r[u]);
+            part = fma(hm[u] * p[u], p[u], part);
         }
-        if (!(ok = all_sum(part, 0, rr, false))) break;
+        __syncwarp();
+        send(0, Ts, r0, rs.bytes(n, rk), t_in, 0, part);
+        wait(0);
+        finish(0, rr, false);
+#pragma unroll
+        for (int u = 0; u < K; ++u)
+            y[u] = fma(hm[u], p[u], -gather_sum_d(cidx, cb[u], ce[u], Ts));
+        __syncwarp();
+        if (!(ok = settle())) break;
         const double alpha = sh.bc[1];
         part = 0.0;
-        for (int j = c0 + tid; j < c1; j += kDsT) {
-            a.x[j] += alpha * a.p[j];
-            const double rj = a.r[j] - alpha * a.y[j];
-            a.r[j] = rj;
-            part += rj * rj;
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const int j = c0 + tid + u * kDsT;
+            r[u] = fma(-alpha, y[u], r[u]);
+            if (j < c1) Ps[j] = r[u];
+            part = fma(r[u], r[u], part);
         }
-        if (!(ok = all_sum(part, 1, rr, true))) break;
+        __syncwarp();
+        send(1, Ps, c0, cs.bytes(m, rk), p_in, 1, part);
+#pragma unroll
+        for (int u = 0; u < K; ++u) x[u] = fma(alpha, p[u], x[u]);
+        wait(1);
+        finish(1, rr, true);
+#pragma unroll
+        for (int u = 0; u < K; ++u) g[u] = gather_sum_d(ridx, rb[u], re[u], Ps);
+        __syncwarp();
+        if (!(ok = settle())) break;
         const double rn = sh.bc[0];
         ++it;
         if (rn < thresh2 || it >= a.cg_max || !(rn == rn)) {
             done = true;
         } else {
-            const double beta = sh.bc[1];  // rn / rr
+            beta = sh.bc[1];  // rn / rr
             rr = rn;
-            for (int j = c0 + tid; j < c1; j += kDsT) {
-                const double pj = a.r[j] + beta * a.p[j];
-                a.p[j] = pj;
-                put_slot<MIXED>(Ps, j, pj);
-            }
-            ok = exchange(Ps, c0, cs.bytes(m, rk), p_in, 1);
         }
     }
+    // x takes r's place: every CTA has its r slices before any x is sent
+    cluster_barrier();
     if (ok) {
         // r1 = (w - sigma x) / (h1 + mu)
-        for (int j = c0 + tid; j < c1; j += kDsT) put_slot<MIXED>(Ps, j, a.x[j]);
-        ok = exchange(Ps, c0, cs.bytes(m, rk), p_in, 1);
-        if (ok)
-            for (int i = r0 + tid; i < r1; i += kDsT)
-                a.r1[i] = (a.w[i] - list_sum_s<MIXED>(a.rowptr, a.colidx, i, Ps)) * a.dinv[i];
+#pragma unroll
+        for (int u = 0; u < K; ++u) {
+            const int j = c0 + tid + u * kDsT;
+            if (j < c1) a.x[j] = Ps[j] = x[u];
+        }
+        __syncwarp();
+        send(3, Ps, c0, cs.bytes(m, rk), p_in, -1, 0.0);
+        wait(3);
+        ok = settle();
+        if (ok) {
+#pragma unroll
+            for (int u = 0; u < K; ++u) {
+                const int i = r0 + tid + u * kDsT;
+                if (i < r1)
+                    a.r1[i] = (a.w[i] - gather_sum_d(ridx, rb[u], re[u], Ps)) * dinv[u];
+            }
+        }
     }
     if (rk == 0 && tid == 0) *a.it_out = it;
     // no CTA leaves while another may still write to or read its shared memory
@@ -1230,12 +1293,6 @@ __global__ void __launch_bounds__(kDsT, 1) k_schur_cg_dsm(DsmCgArgs da) {
 // (exact, so the iterates are the same numbers scaled), which keeps every
 // quantity far inside FP32's exponent range. Same exchange scheme as
 // k_schur_cg_dsm.
-struct DwCgArgs {
-    DsmCgArgs d;
-    int idx_cap;  // ints of dynamic shared memory after the vectors for the
-                  // CTA's index-list slices (each slice fits when >= nnz)
-};
-
 struct DwShared {
     float2 vals[kDsT];
     float2 red[2][16];
@@ -3315,9 +3372,9 @@ private:
         // both vectors' copies in every CTA's shared memory when they fit
         const size_t ds_bytes = (size_t)(((n + 1) & ~1) + ((m + 1) & ~1)) * 8;
         int Cd = ds_bytes <= (size_t)kDsMaxBytes && mode != 3 ? dsm_ctas(E_.mixed()) : 0;
-        // mixed engine: rows and columns per thread of the double-word kernel
+        // rows and columns per thread
         int K = 0;
-        if (Cd && E_.mixed()) {
+        if (Cd) {
             const int per = std::max(((n + 2 * Cd - 1) / (2 * Cd)) * 2,
                                      ((m + 2 * Cd - 1) / (2 * Cd)) * 2);
             K = cdiv(per, kDsT);
@@ -3345,16 +3402,19 @@ private:
             da.c = a;
             da.polls = wait_limit();
             da.err = it_d_.get() + 1;
+            DwCgArgs wa;
+            wa.d = da;
+            wa.idx_cap = idx_cap;
             if (E_.mixed()) {
-                DwCgArgs wa;
-                wa.d = da;
-                wa.idx_cap = idx_cap;
                 if (K == 1) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dw<1>, wa));
                 else if (K == 2) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dw<2>, wa));
                 else if (K == 4) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dw<4>, wa));
                 else REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dw<8>, wa));
             } else {
-                REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dsm<false>, da));
+                if (K == 1) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dsm<1>, wa));
+                else if (K == 2) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dsm<2>, wa));
+                else if (K == 4) REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dsm<4>, wa));
+                else REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_dsm<8>, wa));
             }
         } else if (E_.mixed()) {
             REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_schur_cg_cluster<true>, a));
@@ -3412,11 +3472,18 @@ private:
     // CTAs per cluster of the shared-memory-exchange CG (the largest
     // dynamic shared memory it may use set once), as cluster_ctas.
     static int dsm_ctas(bool mixed) {
-        static const int sizes[2] = {probe_dsm(k_schur_cg_dsm<false>), probe_dw()};
+        static const int sizes[2] = {probe_ds(), probe_dw()};
         return sizes[mixed ? 1 : 0];
     }
-    // every instance of the double-word kernel takes the same cluster and
-    // shared-memory attributes; the cluster size is probed on the first
+    // every instance of a kernel takes the same cluster and shared-memory
+    // attributes; the cluster size is probed on the first
+    static int probe_ds() {
+        const int c = probe_dsm(k_schur_cg_dsm<1>);
+        if (c && (set_dsm_attrs(k_schur_cg_dsm<2>) && set_dsm_attrs(k_schur_cg_dsm<4>) &&
+                  set_dsm_attrs(k_schur_cg_dsm<8>)))
+            return c;
+        return 0;
+    }
     static int probe_dw() {
         const int c = probe_dsm(k_schur_cg_dw<1>);
         if (c && (set_dsm_attrs(k_schur_cg_dw<2>) && set_dsm_attrs(k_schur_cg_dw<4>) &&
