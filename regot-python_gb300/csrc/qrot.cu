@@ -1727,8 +1727,7 @@ public:
     double tau_grad() const { return tau_grad_; }
     // From here on eval() keeps the primal value's row scalings of its point.
     void keep_row_scalings() { xrow_.alloc(n_, st_); }
-    // Primal value at the point of the last eval(), from the scalings it kept.
-    double primal_there(const double* gamma) { return primal(gamma, xrow_.get()); }
+    const double* row_scalings() const { return xrow_.get(); }
 
     // Line-search trial at x = xp + step d: writes grad f(x) (without the tau
     // term) to grad() and returns f(x) - f(xp) without the tau and linear
@@ -3199,6 +3198,63 @@ void qrot_lbfgs_dual_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
 
 namespace {
 
+// Primal values on a stream and an engine of their own, beside the next Newton
+// system (whose CG runs on 16 SMs): at each launch the point of the last eval()
+// and its row scalings are copied, then the passes run at their own pace.
+class SidePrimal {
+public:
+    SidePrimal(regot_dproblem* P, double reg, cudaStream_t main) : main_(main) {
+        side_.create();
+        REGOT_CUDA(cudaEventCreateWithFlags(&copied_.e, cudaEventDisableTiming));
+        REGOT_CUDA(cudaEventRecord(copied_.e, main_));
+        REGOT_CUDA(cudaStreamWaitEvent(side_.s, copied_.e, 0));
+        x_.alloc(P->n, side_.s);
+        E_.reset(new QrotEngine(P, reg, 0.0, side_.s));
+    }
+    // Appends the value at the point of E's last eval() to out, where it arrives
+    // by finish() at the latest. The caller has synchronised the main stream.
+    void launch(QrotEngine& E, std::vector<double>& out) {
+        const int q = (int)out.size();
+        if (q >= 2) {
+            REGOT_CUDA(cudaEventSynchronize(side_.done[q & 1]));
+            out[q - 2] = E_->primal_value(slots_.p->s[q & 1]);
+        }
+        out.push_back(0.0);
+        const size_t n = E.n(), N = n + E.m();
+        d2d(E_->gamma(), E.gamma(), N * sizeof(double), side_.s);
+        d2d(x_.get(), E.row_scalings(), n * sizeof(double), side_.s);
+        REGOT_CUDA(cudaEventRecord(copied_.e, side_.s));
+        REGOT_CUDA(cudaStreamWaitEvent(main_, copied_.e, 0));
+        E_->primal_launch(E_->gamma(), nullptr, &slots_.p->s[q & 1], x_.get());
+        REGOT_CUDA(cudaEventRecord(side_.done[q & 1], side_.s));
+    }
+    void finish(QrotEngine& E, std::vector<double>& out) {
+        sync(side_.s);
+        const int L = (int)out.size();
+        for (int q = L > 1 ? L - 2 : 0; q < L; ++q) out[q] = E_->primal_value(slots_.p->s[q & 1]);
+        E_->ops().check_err();
+        E.add_passes(E_->passes());
+    }
+
+private:
+    struct Slots {
+        PrimRaw s[2];
+    };
+    struct Event {
+        cudaEvent_t e = nullptr;
+        ~Event() {
+            if (e) cudaEventDestroy(e);
+        }
+    };
+    // in this order: the side stream is waited for before the slots go
+    cudaStream_t main_;
+    Pinned<Slots> slots_;
+    Event copied_;
+    SideStream side_;
+    DBuf<double> x_;
+    std::unique_ptr<QrotEngine> E_;
+};
+
 // (H + mu I)^{-1} rhs for the generalized Hessian H of the last masked
 // evaluation (sigma bitmask, h1, h2): hess_cg (qrot_cg.cpp:9-50) with the
 // Schur complement on the column block, identity preconditioner, relative
@@ -3737,10 +3793,16 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
         sync(st);
         return f;
     };
-    // at the point of the last grad_at
-    if (o.prim_vals) E.keep_row_scalings();
-    auto primal = [&]() { return o.prim_vals ? E.primal_there(E.gamma()) : 0.0; };
     std::vector<double> hobj, hmar, htime, hprim;
+    std::unique_ptr<SidePrimal> side;
+    if (o.prim_vals) {
+        E.keep_row_scalings();
+        side.reset(new SidePrimal(P, reg, st));
+    }
+    auto primal = [&]() {  // at the point of the last grad_at
+        if (side) side->launch(E, hprim);
+        else hprim.push_back(0.0);
+    };
     double t0 = clock.now_ms();
     double f = grad_at(gamma, g, true);
     double gnorm = lbfgs::norm(g);
@@ -3748,7 +3810,7 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
     hobj.push_back(f);
     hmar.push_back(gnorm / reg);
     htime.push_back(dur);
-    hprim.push_back(primal());
+    primal();
     int i;
     for (i = 0; i < max_iter; i++) {
         if (o.verbose >= 1)
@@ -3796,8 +3858,9 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
         hobj.push_back(f);
         hmar.push_back(gnorm / reg);
         htime.push_back(htime.back() + dur);
-        hprim.push_back(primal());
+        primal();
     }
+    if (side) side->finish(E, hprim);
     h2d(E.gamma(), gamma.data(), N * sizeof(double), st);
     finish_qrot(E, E.gamma(), hobj, hmar, htime, hprim, i, o, res);
 }
@@ -3833,18 +3896,24 @@ void qrot_grssn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, i
         sync(st);
         return f;
     };
-    // at the point of the last grad_hess
-    if (o.prim_vals) E.keep_row_scalings();
-    auto primal = [&]() { return o.prim_vals ? E.primal_there(E.gamma()) : 0.0; };
 
     std::vector<double> hobj, hmar, htime, hprim;
+    std::unique_ptr<SidePrimal> side;
+    if (o.prim_vals) {
+        E.keep_row_scalings();
+        side.reset(new SidePrimal(P, reg, st));
+    }
+    auto primal = [&]() {  // at the point of the last grad_hess
+        if (side) side->launch(E, hprim);
+        else hprim.push_back(0.0);
+    };
     double t0 = clock.now_ms();
     double f = grad_hess();
     double gnorm = lbfgs::norm(g);
     hobj.push_back(f);
     hmar.push_back(gnorm / reg);
     htime.push_back(clock.now_ms() - t0);
-    hprim.push_back(primal());
+    primal();
     int i;
     for (i = 0; i < max_iter; i++) {
         if (o.verbose >= 1) std::printf("iter = %d, objval = %g, ||grad|| = %g\n", i, f, gnorm);
@@ -3882,8 +3951,9 @@ void qrot_grssn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, i
         hobj.push_back(f);
         hmar.push_back(gnorm / reg);
         htime.push_back(htime.back() + dur);
-        hprim.push_back(primal());
+        primal();
     }
+    if (side) side->finish(E, hprim);
     finish_qrot(E, E.gamma(), hobj, hmar, htime, hprim, i, o, res);
 }
 
