@@ -1610,6 +1610,9 @@ __global__ void __launch_bounds__(kDsT, 1) k_schur_cg_dw(DwCgArgs wa) {
             rr = rn;
         }
     }
+    // x takes r's place and its round this barrier's: every CTA must have its r
+    // slices before any x is sent
+    cluster_barrier();
     if (ok) {
         // x (unscaled, FP64) and r1 = (w - sigma x) / (h1 + mu)
         const double inv_scale = ldexp(1.0, ex);
