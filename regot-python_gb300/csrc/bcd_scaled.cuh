@@ -308,17 +308,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_bcd_scaled(const ScaledParam
         p.beta[j0 + j] = fma(p.reg, log(colbad ? s_vp[j] : s_v[j0 + j]), p.beta[j0 + j]);
 }
 
-// The largest x >= 0 with sqrt(x) < tol, so that the kernel's test on squares
-// decides as the one on roots (tol = infinity: everything but NaN).
-inline double largest_square_below(double tol) {
-    if (!(tol > 0.0)) return -1.0;
-    if (std::isinf(tol)) return std::numeric_limits<double>::max();
-    double x = tol * tol;
-    while (std::sqrt(x) >= tol && x > 0.0) x = std::nextafter(x, -1.0);
-    while (std::sqrt(std::nextafter(x, INFINITY)) < tol) x = std::nextafter(x, INFINITY);
-    return std::sqrt(x) < tol ? x : -1.0;
-}
-
 // Launch shape of the sweeps: one cluster for problems whose products are
 // short against a barrier of the whole grid, else a block an SM.
 struct ScaledPlan {

@@ -373,6 +373,17 @@ __device__ __forceinline__ double max_2d(const Acc* p, int count, size_t stride,
     return (double)r;
 }
 
+// The largest x >= 0 with sqrt(x) < tol, so that the kernel's test on squares
+// decides as the one on roots (tol = infinity: everything but NaN).
+inline double largest_square_below(double tol) {
+    if (!(tol > 0.0)) return -1.0;
+    if (std::isinf(tol)) return std::numeric_limits<double>::max();
+    double x = tol * tol;
+    while (std::sqrt(x) >= tol && x > 0.0) x = std::nextafter(x, -1.0);
+    while (std::sqrt(std::nextafter(x, INFINITY)) < tol) x = std::nextafter(x, INFINITY);
+    return std::sqrt(x) < tol ? x : -1.0;
+}
+
 // Grid-wide sum of K values when one full warp of each of the grid's first
 // `blocks` blocks (0: all) holds them (the other warps take no part). Returns true in every lane of that
 // warp of the last block to finish, with the totals in out[]. The last warp

@@ -26,8 +26,9 @@
 // body is two sweeps and a loop kernel): it continues while a problem is
 // running, no dual has left the split grid, and fewer than max_iter / 2 + 3
 // bodies have run. Once few problems are left, the rest of their sweeps run
-// in one launch of the tail kernel (k_btail: a thread-block cluster per
-// problem, cluster barriers in place of kernel boundaries).
+// in one launch of a tail kernel (k_btail: a thread-block cluster per problem,
+// cluster barriers in place of kernel boundaries; k_bteam: teams of CTAs of a
+// cooperative launch, where clusters are too small or too many).
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -35,10 +36,12 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <queue>
 #include <string>
 #include <vector>
 
 #include "device_util.cuh"
+#include "grid_sync.cuh"
 #include "sm100_util.cuh"
 #include "solvers.h"
 
@@ -121,9 +124,9 @@ __device__ __forceinline__ void lse_merge(float& mx, float& s, float m2, float s
     mx = m;
 }
 
-// Costs of two pairs at once, u = x and v = -y per dimension (the row
-// kernel pairs two rows with one column, the column kernel one row with two
-// columns). The packed FP32x2 instructions round each half exactly as the
+// Costs of two pairs at once, u = -x and v = y or u = x and v = -y per dimension
+// (the row kernel pairs two rows with one column, the column kernel one row with
+// two columns; the squares are the same). The packed FP32x2 instructions round each half exactly as the
 // scalar fadd / ffma / fmul would, so both kernels produce the same M_ij.
 // Four partial sums over the dimensions (k mod 4) keep the FMA chains short:
 // with one running sum the kernels were bound by its latency.
@@ -174,128 +177,205 @@ __device__ __forceinline__ T bld(const T* p) {
     else return *p;
 }
 
+// The other side's points and duals of a half-sweep's items, a tile of kBTile at
+// a time through two buffers in shared memory: the next tile is on its way
+// (cp.async; the duals, which another CTA may have written, through a register)
+// while this one is used, across items; up to two tiles stay for all items.
+// Loaded and stored before use, a tile cost some four thousand clocks of L2
+// latency, more than its arithmetic. Points lie as floats, DP + 1 apart (no bank
+// conflicts), zero from dimension d on (pad()).
+template <int DP, bool COH>
+struct PointTiles {
+    float* pts;    // [2][kBTile][DP + 1]
+    float2* duals; // [2][kBTile]
+    const float* P;
+    const float2* D;
+    int len, d, nt, total;
+    unsigned magic;  // e / d = umulhi(e, magic) for e < 2^12
+    float2 next;
+
+    __device__ PointTiles(float* pts_, float2* duals_, const float* P_, const float2* D_, int len_,
+                          int d_, int items)
+        : pts(pts_), duals(duals_), P(P_), D(D_), len(len_), d(d_),
+          nt((len_ + kBTile - 1) / kBTile), total(nt > 2 ? nt * items : nt),
+          magic(0xffffffffu / d_ + 1u) {
+        if (items > 0) fetch(0);
+    }
+    // The padding dimensions of both buffers, once before the first item.
+    __device__ static void pad(float* pts, int d) {
+        for (int k = d; k < DP; ++k) {
+            pts[threadIdx.x * (DP + 1) + k] = 0.f;
+            pts[(kBTile + threadIdx.x) * (DP + 1) + k] = 0.f;
+        }
+    }
+    __device__ void fetch(int g) {  // tile g of the stream, into buffer g mod 2
+        const int j0 = (g % nt) * kBTile, cnt = min(kBTile, len - j0);
+        const float* src = P + (long long)j0 * d;
+        const unsigned dst =
+            (unsigned)__cvta_generic_to_shared(pts + (g & 1) * kBTile * (DP + 1));
+        for (int e = threadIdx.x; e < cnt * d; e += kBWarps * 32) {
+            const int jj = d == 1 ? e : (int)__umulhi((unsigned)e, magic);
+            const int at = jj * (DP + 1) + (e - jj * d);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 4u * at), "l"(src + e)
+                         : "memory");
+        }
+        next = (int)threadIdx.x < cnt ? bld<COH>(D + j0 + threadIdx.x) : make_float2(0.f, 0.f);
+    }
+    // Tile g of the stream for the whole block, whose buffer is returned; the next
+    // one sets out.
+    __device__ int ready(int g) {
+        if (g >= total) return g % nt;  // one of at most two that stayed
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        duals[(g & 1) * kBTile + threadIdx.x] = next;
+        __syncthreads();
+        if (g + 1 < total) fetch(g + 1);
+        return g & 1;
+    }
+    __device__ const float* point(int buf, int jj) const {
+        return pts + (buf * kBTile + jj) * (DP + 1);
+    }
+    __device__ float2 dual(int buf, int jj) const { return duals[buf * kBTile + jj]; }
+};
+static_assert(kBTile == kBWarps * 32, "PointTiles: a thread a point");
+
+// Half-sweep of the row (COLS: column) blocks first, first + step, ... < end of
+// problem p: the log-sum-exp S of each row against all columns, the new dual
+// own + reg (log a - log S) and, for rows, each block's sum of (S - a)^2 in part.
+// own / oth: splits of the duals of both sides. Every warp takes four rows of a
+// block against all columns; what it leaves of them, (mx, sm), waits in shared
+// memory until kBLater blocks are done, and is then finished in FP64, a block a
+// warp: an FP64 instruction holds its SM quarter for some 64 clocks however few
+// lanes are active, and with four rows a warp and block these took longer than
+// the entries of a small problem. out_split = null: no split (first half-sweep,
+// before the grid exists).
+constexpr int kBLater = 16;
+// spar: the duals of two tiles, then (mx, sm) of kBLater blocks; spts: two tiles'
+// points, kBTile (DP + 1) pairs of floats.
+constexpr int kBParam = 2 * kBTile + kBLater * kBItems;
+
+template <int DP, bool COH, bool COLS>
+__device__ __forceinline__ void half_sweep(const BatchDev& B, int p, int first, int step, int end,
+                                           const float2* own_split, const float2* oth_split,
+                                           const double* own, double* out, float2* out_split,
+                                           double* part, BatchState* st, int* rgf, float k2,
+                                           double reg, float2* spts, float2* spar) {
+    float2 (*s_lse)[kBItems] = reinterpret_cast<float2 (*)[kBItems]>(spar + 2 * kBTile);
+    const int n = COLS ? B.m[p] : B.n[p], m = COLS ? B.n[p] : B.m[p], d = B.d[p];
+    const float sc = B.scale[p];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float* X = COLS ? B.Y + B.yo[p] : B.X + B.xo[p];
+    const float* Y = COLS ? B.X + B.xo[p] : B.Y + B.yo[p];
+    const int ro = COLS ? B.co[p] : B.ro[p], co = COLS ? B.ro[p] : B.co[p];
+    const double* mass = COLS ? nullptr : B.a;
+    const double* logmass = COLS ? B.logb : B.loga;
+    const float2 sc2 = make_float2(sc, sc), k22 = make_float2(k2, k2);
+
+    PointTiles<DP, COH> tiles(reinterpret_cast<float*>(spts), spar, Y, oth_split + co, m, d,
+                              first < end ? (end - first + step - 1) / step : 0);
+    int g = 0, later = 0;
+    for (int blk = first; blk < end; blk += step) {
+        const int i0 = blk * kBItems + warp * kBPer;
+        // rows in pairs, negated: xp[h][k] = (-x_{2h}[k], -x_{2h+1}[k])
+        float2 xp[kBPer / 2][DP], ah[kBPer / 2], al[kBPer / 2];
+        float mx[kBPer], sm[kBPer];
+#pragma unroll
+        for (int r = 0; r < kBPer; ++r) {
+            const int i = i0 + r;
+            const bool ok = i < n;
+#pragma unroll
+            for (int k = 0; k < DP; ++k) {
+                const float v = (ok && k < d) ? -X[(long long)i * d + k] : 0.f;
+                if (r & 1) xp[r >> 1][k].y = v;
+                else xp[r >> 1][k].x = v;
+            }
+            const float2 s = ok ? bld<COH>(own_split + ro + i) : make_float2(0.f, 0.f);
+            const float lk = __fmul_rn(s.y, k2);
+            if (r & 1) {
+                ah[r >> 1].y = s.x;
+                al[r >> 1].y = lk;
+            } else {
+                ah[r >> 1].x = s.x;
+                al[r >> 1].x = lk;
+            }
+            mx[r] = -INFINITY;
+            sm[r] = 0.f;
+        }
+        for (int j0 = 0; j0 < m; j0 += kBTile, ++g) {
+            const int cnt = min(kBTile, m - j0);
+            const int buf = tiles.ready(g);
+            for (int jj = lane; jj < cnt; jj += 32) {
+                float2 ny[DP];
+                const float* pt = tiles.point(buf, jj);
+#pragma unroll
+                for (int k = 0; k < DP; ++k) ny[k] = make_float2(pt[k], pt[k]);
+                const float2 bj = tiles.dual(buf, jj);
+                const float blo = __fmul_rn(bj.y, k2);
+                float z[kBPer];
+#pragma unroll
+                for (int h = 0; h < kBPer / 2; ++h) {
+                    const float2 Mv = bcost2<DP>(xp[h], ny, sc2);
+                    const float2 zz = bexpo2(ah[h], make_float2(bj.x, bj.x), al[h],
+                                             make_float2(blo, blo), Mv, k22);
+                    z[2 * h] = zz.x;
+                    z[2 * h + 1] = zz.y;
+                }
+                lse_add4(mx, sm, z);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kBPer; ++r)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const float m2 = __shfl_xor_sync(0xffffffffu, mx[r], o);
+                const float s2 = __shfl_xor_sync(0xffffffffu, sm[r], o);
+                lse_merge(mx[r], sm[r], m2, s2);
+            }
+        float2 v = make_float2(mx[0], sm[0]);
+#pragma unroll
+        for (int r = 1; r < kBPer; ++r)
+            if (lane == r) v = make_float2(mx[r], sm[r]);
+        if (lane < kBPer) s_lse[later][warp * kBPer + lane] = v;
+        ++later;
+        if (later < kBLater && blk + step < end) continue;
+        __syncthreads();
+        for (int q = warp; q < later; q += kBWarps) {
+            const int b = blk - (later - 1 - q) * step, i = b * kBItems + lane;
+            const float2 lse = s_lse[q][lane];
+            double g2 = 0.0;
+            if (i < n) {
+                const double lg2 = (double)lse.x + (double)log2f(lse.y);  // log2 S_i
+                const double an = bld<COH>(own + ro + i) +
+                                  reg * (logmass[ro + i] - 0.69314718055994531 * lg2);
+                out[ro + i] = an;
+                if (out_split) out_split[ro + i] = bsplit(an, st, rgf);
+                if (!COLS) {
+                    const double gi = row_sum(lse.x, lse.y) - mass[ro + i];
+                    g2 = gi * gi;
+                }
+            }
+            if (!COLS) {
+                // block partial of sum (S_i - a_i)^2 in a fixed order: fours, then those
+                __syncwarp();
+                g2 += __shfl_xor_sync(0xffffffffu, g2, 1);
+                g2 += __shfl_xor_sync(0xffffffffu, g2, 2);
+                double t = 0.0;
+#pragma unroll
+                for (int w = 0; w < kBWarps; ++w) t += __shfl_sync(0xffffffffu, g2, 4 * w);
+                if (lane == 0) part[B.rbo[p] + b] = t;
+            }
+        }
+        later = 0;
+        if (blk + step < end) __syncthreads();  // s_lse is written again
+    }
+}
+static_assert(kBItems == 32, "half_sweep: a row of a block a lane");
+
 // Row half-sweep of iterate k for the row blocks `items` (problem, block):
 // S_i = sum_j exp((alpha_i + beta_j - M_ij)/reg) at (alpha_k, beta_k), the
 // new alpha_i = alpha_i + reg (log a_i - log S_i) (sinkhorn_problem_bcd.cpp:
 // 177-201 with the current alpha as shift) with its split, and the block's
 // sum of (S_i - a_i)^2 for the marginal error. A dual leaving the split
-// grid sets *rgf. The column tile is staged in the caller's shared memory:
-// spts holds kBTile x (DP + 1) pairs, spar kBTile pairs.
-template <int DP, bool COH = false>
-__device__ __forceinline__ void row_item(const BatchDev& B, int2 it, const float2* __restrict__ as_cur,
-                                         const float2* __restrict__ bs,
-                                         const double* __restrict__ alpha_cur, double* alpha_next,
-                                         float2* as_next, double* part, BatchState* st, int* rgf,
-                                         float k2, double reg, float2* spts, float2* spar) {
-    const int p = it.x;
-    const int n = B.n[p], m = B.m[p], d = B.d[p];
-    const float sc = B.scale[p];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = it.y * kBItems + warp * kBPer;
-    const float* X = B.X + B.xo[p];
-    const float* Y = B.Y + B.yo[p];
-    const int ro = B.ro[p], co = B.co[p];
-
-    // rows in pairs: xp[h][k] = (x_{2h}[k], x_{2h+1}[k])
-    float2 xp[kBPer / 2][DP], ah[kBPer / 2], al[kBPer / 2];
-    float mx[kBPer], sm[kBPer];
-#pragma unroll
-    for (int r = 0; r < kBPer; ++r) {
-        const int i = i0 + r;
-        const bool ok = i < n;
-#pragma unroll
-        for (int k = 0; k < DP; ++k) {
-            const float v = (ok && k < d) ? X[(long long)i * d + k] : 0.f;
-            if (r & 1) xp[r >> 1][k].y = v;
-            else xp[r >> 1][k].x = v;
-        }
-        const float2 s = ok ? bld<COH>(as_cur + ro + i) : make_float2(0.f, 0.f);
-        const float lk = __fmul_rn(s.y, k2);
-        if (r & 1) {
-            ah[r >> 1].y = s.x;
-            al[r >> 1].y = lk;
-        } else {
-            ah[r >> 1].x = s.x;
-            al[r >> 1].x = lk;
-        }
-        mx[r] = -INFINITY;
-        sm[r] = 0.f;
-    }
-    const float2 sc2 = make_float2(sc, sc), k22 = make_float2(k2, k2);
-    // columns staged negated and duplicated, (-y, -y), ready for the packed
-    // instructions (rows padded by one entry against bank conflicts)
-    float2 (*sy)[DP + 1] = reinterpret_cast<float2 (*)[DP + 1]>(spts);
-    float2* sb = spar;
-    for (int j0 = 0; j0 < m; j0 += kBTile) {
-        const int cnt = min(kBTile, m - j0);
-        for (int e = threadIdx.x; e < kBTile * DP; e += kBWarps * 32) {
-            const int jj = e / DP, k = e % DP;
-            const float v = (jj < cnt && k < d) ? -Y[(long long)(j0 + jj) * d + k] : 0.f;
-            sy[jj][k] = make_float2(v, v);
-        }
-        for (int jj = threadIdx.x; jj < kBTile; jj += kBWarps * 32)
-            sb[jj] = jj < cnt ? bld<COH>(bs + co + j0 + jj) : make_float2(0.f, 0.f);
-        __syncthreads();
-        for (int jj = lane; jj < cnt; jj += 32) {
-            float2 ny[DP];
-#pragma unroll
-            for (int k = 0; k < DP; ++k) ny[k] = sy[jj][k];
-            const float2 bj = sb[jj];
-            const float blk = __fmul_rn(bj.y, k2);
-            float z[kBPer];
-#pragma unroll
-            for (int h = 0; h < kBPer / 2; ++h) {
-                const float2 Mv = bcost2<DP>(xp[h], ny, sc2);
-                const float2 zz = bexpo2(ah[h], make_float2(bj.x, bj.x), al[h],
-                                         make_float2(blk, blk), Mv, k22);
-                z[2 * h] = zz.x;
-                z[2 * h + 1] = zz.y;
-            }
-            lse_add4(mx, sm, z);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < kBPer; ++r)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float m2 = __shfl_xor_sync(0xffffffffu, mx[r], o);
-            const float s2 = __shfl_xor_sync(0xffffffffu, sm[r], o);
-            lse_merge(mx[r], sm[r], m2, s2);
-        }
-    // lane r < kBPer finishes row i0 + r in FP64
-    double g2 = 0.0;
-    float mxr = mx[0], smr = sm[0];
-#pragma unroll
-    for (int r = 1; r < kBPer; ++r)
-        if (lane == r) {
-            mxr = mx[r];
-            smr = sm[r];
-        }
-    const int i = i0 + lane;
-    if (lane < kBPer && i < n) {
-        const double lg2 = (double)mxr + (double)log2f(smr);  // log2 S_i
-        const double S = row_sum(mxr, smr);
-        const double gi = S - B.a[ro + i];
-        g2 = gi * gi;
-        const double an =
-            bld<COH>(alpha_cur + ro + i) + reg * (B.loga[ro + i] - 0.69314718055994531 * lg2);
-        alpha_next[ro + i] = an;
-        as_next[ro + i] = bsplit(an, st, rgf);
-    }
-    // block partial of sum (S_i - a_i)^2 in a fixed order
-    __shared__ double s_g2[kBWarps];
-    g2 += __shfl_xor_sync(0xffffffffu, g2, 1);
-    g2 += __shfl_xor_sync(0xffffffffu, g2, 2);
-    if (lane == 0) s_g2[warp] = g2;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-#pragma unroll
-        for (int w = 0; w < kBWarps; ++w) t += s_g2[w];
-        part[B.rbo[p] + it.y] = t;
-    }
-}
+// grid sets the state's regrid flag.
 
 // One CTA per work item; the CTAs of finished problems return at once.
 // (Persistent CTAs fetching items from a counter measured 1.8x slower on the
@@ -310,9 +390,10 @@ __global__ void __launch_bounds__(kBWarps * 32) k_brow(
     const int2 it = items[blockIdx.x];
     if (done[it.x]) return;
     __shared__ float2 sy[kBTile][DP + 1];
-    __shared__ float2 sb[kBTile];
-    row_item<DP>(B, it, as_cur, bs, alpha_cur, alpha_next, as_next, part, st, &st->regrid, k2, reg,
-                 &sy[0][0], sb);
+    __shared__ float2 sb[kBParam];
+    PointTiles<DP, false>::pad(reinterpret_cast<float*>(&sy[0][0]), B.d[it.x]);
+    half_sweep<DP, false, false>(B, it.x, it.y, 1, it.y + 1, as_cur, bs, alpha_cur, alpha_next,
+                                 as_next, part, st, &st->regrid, k2, reg, &sy[0][0], sb);
 }
 
 
@@ -321,103 +402,6 @@ __global__ void __launch_bounds__(kBWarps * 32) k_brow(
 // log S_j) in place (sinkhorn_problem_bcd.cpp:149-174, current beta as
 // shift). write_split = 0 skips the split (first half-sweep, before the grid
 // is known).
-template <int DP, bool COH = false>
-__device__ __forceinline__ void col_item(const BatchDev& B, int2 it, const float2* __restrict__ as,
-                                         float2* bs, double* beta, BatchState* st, int* rgf,
-                                         float k2, double reg, int write_split, float2* spts,
-                                         float2* spar) {
-    const int p = it.x;
-    const int n = B.n[p], m = B.m[p], d = B.d[p];
-    const float sc = B.scale[p];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int j0c = it.y * kBItems + warp * kBPer;
-    const float* X = B.X + B.xo[p];
-    const float* Y = B.Y + B.yo[p];
-    const int ro = B.ro[p], co = B.co[p];
-
-    // columns in pairs, negated: ny[h][k] = (-y_{2h}[k], -y_{2h+1}[k])
-    float2 ny[kBPer / 2][DP], bh[kBPer / 2], bl[kBPer / 2];
-    float mx[kBPer], sm[kBPer];
-#pragma unroll
-    for (int r = 0; r < kBPer; ++r) {
-        const int j = j0c + r;
-        const bool ok = j < m;
-#pragma unroll
-        for (int k = 0; k < DP; ++k) {
-            const float v = (ok && k < d) ? -Y[(long long)j * d + k] : 0.f;
-            if (r & 1) ny[r >> 1][k].y = v;
-            else ny[r >> 1][k].x = v;
-        }
-        const float2 s = ok ? bld<COH>(bs + co + j) : make_float2(0.f, 0.f);
-        const float lk = __fmul_rn(s.y, k2);
-        if (r & 1) {
-            bh[r >> 1].y = s.x;
-            bl[r >> 1].y = lk;
-        } else {
-            bh[r >> 1].x = s.x;
-            bl[r >> 1].x = lk;
-        }
-        mx[r] = -INFINITY;
-        sm[r] = 0.f;
-    }
-    const float2 sc2 = make_float2(sc, sc), k22 = make_float2(k2, k2);
-    // rows staged duplicated, (x, x), for the packed instructions
-    float2 (*sx)[DP + 1] = reinterpret_cast<float2 (*)[DP + 1]>(spts);
-    float2* sa = spar;
-    for (int i0 = 0; i0 < n; i0 += kBTile) {
-        const int cnt = min(kBTile, n - i0);
-        for (int e = threadIdx.x; e < kBTile * DP; e += kBWarps * 32) {
-            const int ii = e / DP, k = e % DP;
-            const float v = (ii < cnt && k < d) ? X[(long long)(i0 + ii) * d + k] : 0.f;
-            sx[ii][k] = make_float2(v, v);
-        }
-        for (int ii = threadIdx.x; ii < kBTile; ii += kBWarps * 32)
-            sa[ii] = ii < cnt ? bld<COH>(as + ro + i0 + ii) : make_float2(0.f, 0.f);
-        __syncthreads();
-        for (int ii = lane; ii < cnt; ii += 32) {
-            float2 xv[DP];
-#pragma unroll
-            for (int k = 0; k < DP; ++k) xv[k] = sx[ii][k];
-            const float2 ai = sa[ii];
-            const float alk = __fmul_rn(ai.y, k2);
-            float z[kBPer];
-#pragma unroll
-            for (int h = 0; h < kBPer / 2; ++h) {
-                // the same operations, in the same order, as the row kernel
-                const float2 Mv = bcost2<DP>(xv, ny[h], sc2);
-                const float2 zz = bexpo2(make_float2(ai.x, ai.x), bh[h], make_float2(alk, alk),
-                                         bl[h], Mv, k22);
-                z[2 * h] = zz.x;
-                z[2 * h + 1] = zz.y;
-            }
-            lse_add4(mx, sm, z);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < kBPer; ++r)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float m2 = __shfl_xor_sync(0xffffffffu, mx[r], o);
-            const float s2 = __shfl_xor_sync(0xffffffffu, sm[r], o);
-            lse_merge(mx[r], sm[r], m2, s2);
-        }
-    float mxr = mx[0], smr = sm[0];
-#pragma unroll
-    for (int r = 1; r < kBPer; ++r)
-        if (lane == r) {
-            mxr = mx[r];
-            smr = sm[r];
-        }
-    const int j = j0c + lane;
-    if (lane < kBPer && j < m) {
-        const double lg2 = (double)mxr + (double)log2f(smr);
-        const double bn =
-            bld<COH>(beta + co + j) + reg * (B.logb[co + j] - 0.69314718055994531 * lg2);
-        beta[co + j] = bn;
-        if (write_split) bs[co + j] = bsplit(bn, st, rgf);
-    }
-}
 
 template <int DP>
 __global__ void __launch_bounds__(kBWarps * 32) k_bcol(
@@ -427,8 +411,11 @@ __global__ void __launch_bounds__(kBWarps * 32) k_bcol(
     const int2 it = items[blockIdx.x];
     if (done[it.x]) return;
     __shared__ float2 sx[kBTile][DP + 1];
-    __shared__ float2 sa[kBTile];
-    col_item<DP>(B, it, as, bs, beta, st, &st->regrid, k2, reg, write_split, &sx[0][0], sa);
+    __shared__ float2 sa[kBParam];
+    PointTiles<DP, false>::pad(reinterpret_cast<float*>(&sx[0][0]), B.d[it.x]);
+    half_sweep<DP, false, true>(B, it.x, it.y, 1, it.y + 1, bs, as, beta, beta,
+                                write_split ? bs : nullptr, nullptr, st, &st->regrid, k2, reg,
+                                &sx[0][0], sa);
 }
 
 // ---- tensor-core variant of the half-sweeps ----
@@ -486,9 +473,9 @@ __device__ __forceinline__ void tc_put_point(unsigned char* hi, unsigned char* l
 }
 
 // Half-sweep with the cost tile on the tensor cores. COLS = false: the row
-// half-sweep of row_item (items are blocks of 128 rows; each warp of the
+// half-sweep of half_sweep (items are blocks of 128 rows; each warp of the
 // first four writes the marginal-error partial of its 32 rows, the layout
-// k_bfin reads); COLS = true: the column half-sweep of col_item.
+// k_bfin reads); COLS = true: the column half-sweep.
 template <bool COLS>
 __global__ void __launch_bounds__(256, 1) k_bsweep_tc(
     const BatchDev B, const int2* __restrict__ items, const float2* __restrict__ own_split,
@@ -709,8 +696,7 @@ __global__ void k_bloop(BatchState* st, cudaGraphConditionalHandle h) {
 // gives each running problem one cluster of C CTAs (16, or 8 where a device
 // cannot hold clusters of 16), which runs that problem's sweeps to its stop in
 // one launch: CTA r takes the row blocks and the column blocks r, r + C, ...
-// of the problem (the same row_item /
-// col_item arithmetic as the sweep kernels), and a cluster barrier stands
+// of the problem (half_sweep, as in the sweep kernels), and a cluster barrier stands
 // where a kernel boundary stood. The problems' clusters are independent and
 // nothing waits across them.
 //
@@ -722,11 +708,13 @@ __global__ void k_bloop(BatchState* st, cudaGraphConditionalHandle h) {
 // done flag and final parity.
 constexpr int kTailCta = 16;  // CTAs per cluster where the device holds such clusters, else 8
 constexpr size_t kTailSmem = (size_t)kBTile * (kBClassDim[kBClasses - 1] + 1) * sizeof(float2) +
-                             (size_t)kBTile * sizeof(float2);
+                             (size_t)kBParam * sizeof(float2);
 
 struct TailArgs {
     BatchDev B;
-    const int* plist;  // the running problems, one per cluster
+    const int* plist;  // the running problems, one per cluster (k_btail)
+    const int4* team;  // problem, rank and CTAs of each CTA's team (k_bteam)
+    unsigned* count;   // barrier of each problem's team, zero at the launch
     const int* pcls;   // dimension class of each problem
     float2* as[2];
     double* a[2];
@@ -742,7 +730,7 @@ struct TailArgs {
     int max_iter;
     int body_cap;
     int loops0;        // loop bodies run before this launch (for the sweep count)
-    double tol;
+    double stop2;      // the largest s with sqrt(s) < tol (negative: none)
     float k2;
     double reg;
 };
@@ -754,34 +742,75 @@ __device__ __forceinline__ void tail_barrier() {
         "barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
 
-template <int DP>
-__device__ void tail_solve(const TailArgs& a, int p, int rank, int ncta, float2* spts,
+// Barrier of a problem's cluster.
+struct ClusterTeam {
+    __device__ bool sync() {
+        tail_barrier();
+        return true;
+    }
+};
+
+// Barrier of a problem's team of CTAs of one cooperative launch: a counter in
+// global memory that only grows. A wait that gives up (after some seconds) sets
+// st->err, at which the waits of all teams end.
+struct GridTeam {
+    unsigned* count;
+    BatchState* st;
+    int size;
+    unsigned target;
+    __device__ bool sync() {
+        __shared__ int s_ok;
+        __syncthreads();
+        target += (unsigned)size;
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+            int ok = 0;
+            for (unsigned s = 0; s < kGridSpins; ++s) {
+                unsigned c;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+                if ((int)(c - target) >= 0) {
+                    ok = 1;
+                    break;
+                }
+                if ((s & 1023u) == 1023u && *(volatile int*)&st->err) break;
+            }
+            if (!ok) atomicOr(&st->err, 2);
+            s_ok = ok;
+        }
+        __syncthreads();
+        return s_ok != 0;
+    }
+};
+
+template <int DP, typename Team>
+__device__ void tail_solve(const TailArgs& a, int p, int rank, int ncta, Team team, float2* spts,
                            float2* spar) {
     const BatchDev& B = a.B;
     const int nb = (B.n[p] + kBItems - 1) / kBItems, mb = (B.m[p] + kBItems - 1) / kBItems;
     int* rgf = a.pflag + p;
-    __shared__ double s_g;
+    __shared__ double s_s;
+    const double stop2 = a.stop2;
+    PointTiles<DP, true>::pad(reinterpret_cast<float*>(spts), B.d[p]);
     int k = __ldcg(a.iter + p);  // written by rank 0 only, after this read
     for (int body = 0; body < a.body_cap; ++body) {
         // alpha of the current iterate in buffers 0 at the start of a body,
         // as in the graph loop
         for (int q = 0; q < 2; ++q) {
-            for (int rb = rank; rb < nb; rb += ncta)
-                row_item<DP, true>(B, make_int2(p, rb), a.as[q], a.bs, a.a[q], a.a[1 - q],
-                                   a.as[1 - q], a.part, a.st, rgf, a.k2, a.reg, spts, spar);
-            tail_barrier();
+            half_sweep<DP, true, false>(B, p, rank, ncta, nb, a.as[q], a.bs, a.a[q], a.a[1 - q],
+                                        a.as[1 - q], a.part, a.st, rgf, a.k2, a.reg, spts, spar);
+            if (!team.sync()) return;
             // marginal error and stopping test of the iterate (k_bfin)
             if (threadIdx.x < 32) {
                 double s = 0.0;
                 for (int j = threadIdx.x; j < nb; j += 32) s += __ldcg(a.part + B.rbo[p] + j);
                 s = warp_sum_d(s);
-                if (threadIdx.x == 0) s_g = sqrt(s);
+                if (threadIdx.x == 0) s_s = s;
             }
             __syncthreads();
-            const double g = s_g;
-            const bool stop = g < a.tol || k >= a.max_iter;
+            const double s = s_s;
+            const bool stop = s <= stop2 || k >= a.max_iter;  // sqrt(s) < tol
             if (rank == 0 && threadIdx.x == 0) {
-                a.mar[p] = g;
+                if (stop || body + 1 == a.body_cap) a.mar[p] = sqrt(s);
                 if (stop) {
                     a.done[p] = 1;
                     a.fpar[p] = q;
@@ -793,10 +822,9 @@ __device__ void tail_solve(const TailArgs& a, int p, int rank, int ncta, float2*
             }
             if (stop) return;
             ++k;
-            for (int cb = rank; cb < mb; cb += ncta)
-                col_item<DP, true>(B, make_int2(p, cb), a.as[1 - q], a.bs, a.beta, a.st, rgf,
-                                   a.k2, a.reg, 1, spts, spar);
-            tail_barrier();
+            half_sweep<DP, true, true>(B, p, rank, ncta, mb, a.bs, a.as[1 - q], a.beta, a.beta,
+                                       a.bs, nullptr, a.st, rgf, a.k2, a.reg, spts, spar);
+            if (!team.sync()) return;
         }
         // a dual of this problem left the split grid: stop at the body's end
         // (alpha in buffers 0) for the host to re-split on a new grid. Every
@@ -804,7 +832,7 @@ __device__ void tail_solve(const TailArgs& a, int p, int rank, int ncta, float2*
         // (in the next row half-sweep) before all have passed the barrier,
         // so all CTAs see the same value.
         const int rg = __ldcg(rgf);
-        tail_barrier();
+        if (!team.sync()) return;
         if (rg) {
             if (rank == 0 && threadIdx.x == 0) {
                 atomicOr(&a.st->regrid, 1);
@@ -826,9 +854,29 @@ __global__ void __launch_bounds__(kBWarps * 32) k_btail(const TailArgs a) {
     float2* spts = tail_smem;
     float2* spar = tail_smem + kBTile * (kBClassDim[kBClasses - 1] + 1);
     switch (a.pcls[p]) {
-        case 0: tail_solve<4>(a, p, (int)rank, (int)ncta, spts, spar); break;
-        case 1: tail_solve<8>(a, p, (int)rank, (int)ncta, spts, spar); break;
-        default: tail_solve<16>(a, p, (int)rank, (int)ncta, spts, spar); break;
+        case 0: tail_solve<4>(a, p, (int)rank, (int)ncta, ClusterTeam(), spts, spar); break;
+        case 1: tail_solve<8>(a, p, (int)rank, (int)ncta, ClusterTeam(), spts, spar); break;
+        default: tail_solve<16>(a, p, (int)rank, (int)ncta, ClusterTeam(), spts, spar); break;
+    }
+}
+
+// The same with teams of any number of CTAs, all resident (a cooperative
+// launch): problems of more row or column blocks than a cluster has CTAs, or
+// more problems than clusters fit (sixteen CTAs for each of 64 problems of 64 to
+// 2048 points run in four rounds, most of their CTAs idle, and the largest
+// problem takes four blocks a CTA and half-sweep: 29 ms for the call, 21 with
+// teams and the half-sweeps' tiles and endings as they are now).
+__global__ void __launch_bounds__(kBWarps * 32, 2) k_bteam(const TailArgs a) {
+    extern __shared__ __align__(16) float2 tail_smem[];
+    const int4 t = a.team[blockIdx.x];
+    const int p = t.x;
+    float2* spts = tail_smem;
+    float2* spar = tail_smem + kBTile * (kBClassDim[kBClasses - 1] + 1);
+    const GridTeam team{a.count + p, a.st, t.z, 0u};
+    switch (a.pcls[p]) {
+        case 0: tail_solve<4>(a, p, t.y, t.z, team, spts, spar); break;
+        case 1: tail_solve<8>(a, p, t.y, t.z, team, spts, spar); break;
+        default: tail_solve<16>(a, p, t.y, t.z, team, spts, spar); break;
     }
 }
 
@@ -1078,6 +1126,56 @@ int tail_cluster_size() {
     cudaGetLastError();  // a refused query leaves no error behind
     if (dev < 64) cached[dev].store(size);
     return size;
+}
+
+// Bodies (pairs of sweeps) of a k_bteam launch of several problems: some
+// milliseconds, against some 40 us for the launch and the reads around it.
+constexpr int kTeamBodies = 16;
+// Problems up to which the tail runs in clusters, where these have the CTAs.
+constexpr int kTailClusters = 4;
+
+// CTAs of k_bteam that the device holds at once, 0 without cooperative launches.
+int team_slots() {
+    int dev = 0, coop = 0, per_sm = 0;
+    REGOT_CUDA(cudaGetDevice(&dev));
+    REGOT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return 0;
+    REGOT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bteam, kBWarps * 32, kTailSmem));
+    return per_sm * device_sm_count();
+}
+
+// The teams of the running problems (at most `slots`), CTA by CTA. A sweep in C
+// CTAs takes about a fixed time (barriers, reductions: kFixed points a half) and
+// ceil(row blocks / C) m + ceil(column blocks / C) n points a CTA; the CTAs are
+// dealt out to the problem that is slowest by that, as long as one more block
+// less a CTA makes it faster.
+std::vector<int4> make_teams(const std::vector<int>& running, const std::vector<int>& hn,
+                             const std::vector<int>& hm, int slots) {
+    constexpr double kFixed = 375.0;
+    auto cost = [&](int p, int c) {
+        const int nb = cdiv(hn[p], kBItems), mb = cdiv(hm[p], kBItems);
+        return 2 * kFixed + (double)cdiv(nb, c) * hm[p] + (double)cdiv(mb, c) * hn[p];
+    };
+    std::vector<int> width(running.size(), 1);
+    std::priority_queue<std::pair<double, int>> slowest;
+    for (size_t k = 0; k < running.size(); ++k) slowest.push({cost(running[k], 1), (int)k});
+    int left = slots - (int)running.size();
+    while (!slowest.empty() && left > 0) {
+        const int k = slowest.top().second, p = running[k];
+        const double now = slowest.top().first;
+        slowest.pop();
+        const int most = std::min(std::max(cdiv(hn[p], kBItems), cdiv(hm[p], kBItems)), width[k] + left);
+        int c = width[k] + 1;
+        while (c <= most && cost(p, c) >= now) ++c;
+        if (c > most) continue;
+        left -= c - width[k];
+        width[k] = c;
+        slowest.push({cost(p, c), k});
+    }
+    std::vector<int4> teams;
+    for (size_t k = 0; k < running.size(); ++k)
+        for (int r = 0; r < width[k]; ++r) teams.push_back(make_int4(running[k], r, width[k], 0));
+    return teams;
 }
 
 }  // namespace
@@ -1495,8 +1593,10 @@ void erot_solve_batched_gpu(regot_ctx* ctx, const regot_batch_desc* D, double re
     // continue, after a re-split, in the next launch.
     if (hs.active > 0) {
         DBuf<int> dcls, plist(P, st), pflag(P, st);
+        DBuf<unsigned> tcount(P, st);
+        DBuf<int4> dteam;
         upload_vec(dcls, cls, st);
-        const int tail_cta = tail_cluster_size();
+        const int tail_cta = tail_cluster_size(), slots = team_slots();
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = tail_cta;
@@ -1508,11 +1608,27 @@ void erot_solve_batched_gpu(regot_ctx* ctx, const regot_batch_desc* D, double re
             for (int p = 0; p < P; ++p)
                 if (!hdone[p]) running.push_back(p);
             if (running.empty()) break;
-            h2d(plist.get(), running.data(), running.size() * sizeof(int), st);
+            int blocks = 0;  // row or column blocks of the largest problem
+            for (int p : running)
+                blocks = std::max(blocks, std::max(cdiv(hn[p], kBItems), cdiv(hm[p], kBItems)));
+            // a cluster's barrier takes a third of a team's, but the device holds few
+            // clusters of tail_cta CTAs, and one of more blocks is slow in them
+            const bool teams = (int)running.size() <= slots &&
+                               (blocks > tail_cta || (int)running.size() > kTailClusters);
+            std::vector<int4> hteam;
+            if (teams) {
+                hteam = make_teams(running, hn, hm, slots);
+                upload_vec(dteam, hteam, st);
+                tcount.zero();
+            } else {
+                h2d(plist.get(), running.data(), running.size() * sizeof(int), st);
+            }
             pflag.zero();
             TailArgs ta{};
             ta.B = B;
             ta.plist = plist.get();
+            ta.team = dteam.get();
+            ta.count = tcount.get();
             ta.pcls = dcls.get();
             for (int q = 0; q < 2; ++q) {
                 ta.as[q] = AS[q].get();
@@ -1529,8 +1645,10 @@ void erot_solve_batched_gpu(regot_ctx* ctx, const regot_batch_desc* D, double re
             ta.st = S;
             ta.max_iter = max_iter;
             ta.body_cap = std::max(1, hs.loop_cap - hs.loops);
+            // problems end one after another: the teams are dealt out anew
+            if (teams && running.size() > 1) ta.body_cap = std::min(ta.body_cap, kTeamBodies);
             ta.loops0 = hs.loops;
-            ta.tol = tol;
+            ta.stop2 = largest_square_below(tol);
             ta.k2 = k2;
             ta.reg = reg;
             cudaLaunchConfig_t cfg = {};
@@ -1540,13 +1658,24 @@ void erot_solve_batched_gpu(regot_ctx* ctx, const regot_batch_desc* D, double re
             cfg.stream = st;
             cfg.attrs = at;
             cfg.numAttrs = 1;
-            REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_btail, ta));
+            if (teams) {
+                cudaLaunchAttribute co[1];
+                co[0].id = cudaLaunchAttributeCooperative;
+                co[0].val.cooperative = 1;
+                cfg.gridDim = dim3((unsigned)hteam.size());
+                cfg.attrs = co;
+                REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_bteam, ta));
+            } else {
+                REGOT_CUDA(cudaLaunchKernelEx(&cfg, k_btail, ta));
+            }
             count_launch();
             read_small(ctx, &hs, S, sizeof(hs), st);
+            if (hs.err)
+                throw Error(REGOT_ERR_TIMEOUT, "a team of the batched tail gave up waiting for its CTAs");
             if (hs.active == 0) break;
-            if (!hs.regrid || hs.loops >= hs.loop_cap)
+            if ((!hs.regrid && !teams) || hs.loops >= hs.loop_cap)
                 throw Error(REGOT_ERR_NUMERIC, "batched BCD did not terminate");
-            regrid(0);
+            if (hs.regrid) regrid(0);
         }
     }
 
