@@ -1978,7 +1978,6 @@ private:
     RootGraph& root_graph(bool rows, const double* other, double* x) {
         RootGraph& g = root_graphs_[std::make_tuple(rows, other, x)];
         if (g.exec) return g;
-        const int len = rows ? n_ : m_;
         REGOT_CUDA(cudaGraphCreate(&g.graph, 0));
         cudaGraphConditionalHandle h;
         REGOT_CUDA(cudaGraphConditionalHandleCreate(&h, g.graph, 1, cudaGraphCondAssignDefault));
