@@ -411,10 +411,25 @@ __device__ bool warp_grid_reduce(const double (&vals)[K], double* block_parts, u
     double part[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) part[k] = 0.0;
-    for (unsigned b = lane; b < blocks; b += 32) {
+    // up to 24 loads a lane under way together: one after another, the sums of
+    // 256 blocks took eight L2 latencies
+    constexpr unsigned U = K <= 3 ? 8 : 4;
+    for (unsigned b = lane; b < blocks; b += 32 * U) {
+        double v[U][K];
 #pragma unroll
-        for (int k = 0; k < K; ++k) part[k] += __ldcg(&block_parts[(size_t)b * K + k]);
+        for (unsigned u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                v[u][k] = b + 32 * u < blocks ? __ldcg(&block_parts[(size_t)(b + 32 * u) * K + k]) : 0.0;
+#pragma unroll
+        for (unsigned u = 0; u < U; ++u) {
+            if (b + 32 * u < blocks) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) part[k] += v[u][k];
+            }
+        }
     }
+    __syncwarp();
 #pragma unroll
     for (int k = 0; k < K; ++k) out[k] = warp_sum_d(part[k]);
     if (lane == 0) *counter = 0u;

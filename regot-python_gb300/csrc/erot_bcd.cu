@@ -37,7 +37,8 @@ namespace {
 // continues: the dual update, the split, the max-abs (integer) and the grid
 // sums (warp_grid_reduce) need one thread per row or column, and keeping
 // FP64 instructions to that one warp matters on a part whose FP64 rate is a
-// small fraction of its FP32 rate.
+// small fraction of its FP32 rate. (In the row finalize warp 1 forms the sums
+// while warp 0 takes the logarithms.)
 constexpr int kFinItems = 32;
 const dim3 kFinBlock(32, 8);
 
@@ -143,32 +144,50 @@ __global__ void k_bcd_row(const Acc* rp, int nslabs, int n, const double* anchor
                           double* hmar, double* htime, double* parts, BcdState* st,
                           int robust, SplitOut so) {
     if (st->done) return;
+    __shared__ double s_S[kFinItems];
     const int i = blockIdx.x * kFinItems + threadIdx.x;
-    const double S = merge_2d(rp + i, nslabs, (size_t)n, i < n);
-    if (threadIdx.y != 0) return;  // the rest runs in warp 0 only
+    // operands under way during the merge
+    double al = 0.0, an = 0.0, ai = 0.0, la = 0.0;
+    if (threadIdx.y < 2 && i < n) {
+        al = alpha[i];
+        an = anchor[i];
+        ai = a[i];
+        if (threadIdx.y == 0) la = loga[i];
+    }
+    const double S0 = merge_2d(rp + i, nslabs, (size_t)n, i < n);
+    if (threadIdx.y == 0) s_S[threadIdx.x] = S0;
+    __syncthreads();
+    if (threadIdx.y > 1) return;
+    const double S = s_S[threadIdx.x];
+    if (threadIdx.y == 0) {  // the new duals, beside warp 1's sums
+        double vmax = 0.0;
+        if (i < n) {
+            const double an_next = an + reg * (la - log(S));
+            alpha_next[i] = an_next;
+            vmax = an_next;
+            if (so.out) {
+                if (!(fabs(an_next) < st->sbound)) atomicOr(&st->bad, 4);
+                so.out[i] = split_fixed(an_next, st);
+            }
+        }
+        __syncwarp();
+        warp_atomic_max_abs(&st->maxabs, vmax);
+        return;
+    }
     double v[3] = {0.0, 0.0, 0.0};
-    double vmax = 0.0;
     if (i < n) {
-        const double al = alpha[i];
-        const double an = anchor[i];
         if (!robust && !sum_ok<MIXED>(S)) atomicOr(&st->bad, 1);
         const double r = robust ? exp(log(S) + (al - an) / reg) : S;
-        const double g = r - a[i];
+        const double g = r - ai;
         v[0] = g * g;
         v[1] = r;
-        v[2] = a[i] * al;
-        const double an_next = an + reg * (loga[i] - log(S));
-        alpha_next[i] = an_next;
-        vmax = an_next;
-        if (so.out) {
-            if (!(fabs(an_next) < st->sbound)) atomicOr(&st->bad, 4);
-            so.out[i] = split_fixed(an_next, st);
-        }
+        v[2] = ai * al;
     }
-    warp_atomic_max_abs(&st->maxabs, vmax);
     __threadfence();
     double out[3];
     if (warp_grid_reduce<3>(v, parts, &st->counter, out) && threadIdx.x == 0) {
+        // (a dual off the split grid may show only in the column finalize, which
+        // stops the sweeps before it advances)
         if (atomicAdd(&st->bad, 0)) {
             st->done = 1;
             return;
@@ -197,15 +216,22 @@ __global__ void k_bcd_col(const Acc* cp, int nrb, int m, const double* anchor,
                           double* parts, BcdState* st, int robust, SplitOut so, int advance) {
     if (st->done) return;
     const int j = blockIdx.x * kFinItems + threadIdx.x;
+    // operands under way during the merge
+    double an = 0.0, lb = 0.0, bj = 0.0;
+    if (threadIdx.y == 0 && j < m) {
+        an = anchor[j];
+        lb = logb[j];
+        bj = b[j];
+    }
     const double S = merge_2d(cp + j, nrb, (size_t)m, j < m);
     if (threadIdx.y != 0) return;  // the rest runs in warp 0 only
     double v[1] = {0.0};
     double vmax = 0.0;
     if (j < m) {
         if (!robust && !sum_ok<MIXED>(S)) atomicOr(&st->bad, 2);
-        const double bn = anchor[j] + reg * (logb[j] - log(S));
+        const double bn = an + reg * (lb - log(S));
         beta_next[j] = bn;
-        if (j < m - 1) v[0] = b[j] * bn;
+        if (j < m - 1) v[0] = bj * bn;
         vmax = bn;
         if (so.out) {
             if (!(fabs(bn) < st->sbound)) atomicOr(&st->bad, 8);
