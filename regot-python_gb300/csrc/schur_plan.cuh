@@ -117,16 +117,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_schur_cg(const SchurCgParams
             if (lane == 0) s_s[r] = s;
         }
     };
-    auto columns = [&]() {  // s_c = S' s_u (without 1 / reg)
-        for (int c = warp; c < C; c += kResWarps) {
+    auto columns = [&](int w, int warps) {  // s_c = S' s_u (without 1 / reg)
+        for (int c = w; c < C; c += warps) {
             const int j = j0 + c;
             const double s = stored_dot(static_cast<const double*>(S.cvals) + (size_t)j * S.ldc,
                                         S.crows + (size_t)j * S.ldc, __ldg(S.ccount + j), s_u);
             if (lane == 0) s_c[c] = s;
         }
-    };
-    auto stage_u = [&]() {
-        for (int i = tid; i < n; i += kResThreads) s_u[i] = __ldcg(p.ubuf + i);
     };
 
     // ---- right-hand side of the Schur system, its diagonal, first residual ----
@@ -139,9 +136,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_schur_cg(const SchurCgParams
     }
     bar.arrive();
     if (!bar.wait()) return;
-    stage_u();
+    for (int i = tid; i < n; i += kResThreads) s_u[i] = __ldcg(p.ubuf + i);
     __syncthreads();
-    columns();
+    columns(warp, kResWarps);
     for (int c = warp; c < C; c += kResWarps) {
         const int j = j0 + c;
         const double dj = p.h[n + j] + shift;
@@ -223,14 +220,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_schur_cg(const SchurCgParams
         }
         bar.arrive();
         if (!bar.wait()) return;
+        // the step length in warp 0 (some three thousand clocks of additions and a
+        // division), u and the columns' products in the others
         if (warp == 0) {
             const double pq = total(1).x;
             if (lane == 0) s_sc = rz / pq;
             __syncwarp();
+        } else {
+            for (int i = tid - 32; i < n; i += kResThreads - 32) s_u[i] = __ldcg(p.ubuf + i);
+            asm volatile("bar.sync 1, %0;" ::"n"(kResThreads - 32) : "memory");
+            columns(warp - 1, kResWarps - 1);
         }
-        stage_u();
-        __syncthreads();
-        columns();
         __syncthreads();
         {
             const double alpha = s_sc;
