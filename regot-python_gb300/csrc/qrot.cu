@@ -31,6 +31,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cfloat>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -615,14 +616,19 @@ __global__ void k_cs_col_counts(const uint32_t* bm, int n, int m, int nslabs, in
 
 // Per column: the chunk counts become exclusive offsets within the column,
 // ccol_j = the column's total.
-__global__ void k_cs_col_offsets(int m, int chunks, int* ccnt, int* ccol) {
+__global__ void k_cs_col_offsets(int m, int* ccnt, int* ccol) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= m) return;
+    // all counts under way together: read, summed and written one by one they
+    // took 12 us at any size
+    int v[kColChunks];
+#pragma unroll
+    for (int c = 0; c < kColChunks; ++c) v[c] = ccnt[(size_t)c * m + j];
     int run = 0;
-    for (int c = 0; c < chunks; ++c) {
-        const int v = ccnt[(size_t)c * m + j];
+#pragma unroll
+    for (int c = 0; c < kColChunks; ++c) {
         ccnt[(size_t)c * m + j] = run;
-        run += v;
+        run += v[c];
     }
     ccol[j] = run;
 }
@@ -1640,10 +1646,6 @@ __global__ void __launch_bounds__(kDsT, 1) k_schur_cg_dw(DwCgArgs wa) {
     cluster_barrier();
 }
 
-__global__ void k_time(unsigned long long t0, unsigned long long* out) {
-    *out = globaltimer_ns() - t0;
-}
-
 }  // namespace
 
 // --------------------------------------------------------------- engine --
@@ -1684,12 +1686,13 @@ public:
     double* grad() { return grad_.get(); }
     QState* state() { return state_.get(); }
 
-    // obj and grad at the device vector gamma (n + m). With `mask`, also the
-    // sigma bitmask and h = (h1, h2) of compute_D_hess.
-    double eval(const double* gamma, double* grad, bool mask) {
+    // obj and grad at the device vector gamma (n + m), grad also into host_grad if
+    // given (behind the same synchronisation). With `mask`, also the sigma bitmask
+    // and h = (h1, h2) of compute_D_hess.
+    double eval(const double* gamma, double* grad, bool mask, double* host_grad = nullptr) {
         const PassShape sh = ops_.buf().shape;
         if (mask && !bm_.get()) bm_.alloc(bm_words_, st_);
-        ops_.maxabs(gamma, n_ + m_, nullptr, 0, &state_.get()->maxabs);
+        if (mixed_) ops_.maxabs(gamma, n_ + m_, nullptr, 0, &state_.get()->maxabs);
         PassParams p = ops_.base_params();
         p.ra = gamma;
         p.cb = gamma + n_;
@@ -1712,11 +1715,17 @@ public:
                 ops_.buf().totpart.get(), blocks, scal_.get(), xrow_.get());
         count_launch();
         REGOT_CHECK_LAUNCH();
-        double sq = 0.0;
-        QState hs;
-        d2h(&sq, scal_.get(), sizeof(double), st_);
-        d2h(&hs, state_.get(), sizeof(hs), st_);
+        const size_t N = (size_t)n_ + m_;
+        double* h = static_cast<double*>(
+            ctx_stage(P_->ctx, (1 + N) * sizeof(double) + sizeof(QState)));
+        d2h(h, scal_.get(), sizeof(double), st_);
+        if (host_grad) d2h(h + 1, grad, N * sizeof(double), st_);
+        d2h(h + 1 + N, state_.get(), sizeof(QState), st_);
         sync(st_);
+        const double sq = h[0];
+        QState hs;
+        std::memcpy(&hs, h + 1 + N, sizeof(hs));
+        if (host_grad) std::memcpy(host_grad, h + 1, N * sizeof(double));
         ++passes_;
         // qrot_problem.cpp:226-253 (tau terms: 342-351)
         double obj = 0.5 * sq - reg_ * hs.dot_ab;
@@ -1742,7 +1751,7 @@ public:
     // by the caller). Also returns sum D(x)^2 in *sq.
     double eval_step(const double* xp, const double* d, double step, double* sq) {
         const PassShape sh = ops_.buf().shape;
-        ops_.maxabs(xp, n_ + m_, nullptr, 0, &state_.get()->maxabs);
+        if (mixed_) ops_.maxabs(xp, n_ + m_, nullptr, 0, &state_.get()->maxabs);
         PassParams p = ops_.base_params();
         p.ra = xp;
         p.cb = xp + n_;
@@ -1791,7 +1800,7 @@ public:
         double* xr = vec_.get();
         double* yc = xr + std::max(n_, m_);
         double* fc = yc + std::max(n_, m_);
-        if (!grid) {
+        if (!grid && mixed_) {  // only a mixed pass splits gamma
             ops_.maxabs(gamma, n_ + m_, nullptr, 0, &state_.get()->maxabs);
             grid = &state_.get()->maxabs;
         }
@@ -2065,23 +2074,22 @@ void finish_qrot(QrotEngine& E, const double* d_gamma, const std::vector<double>
                      [&](double* dst) { E.plan(d_gamma, dst); });
 }
 
-// Wall clock in milliseconds on the device (globaltimer), like the
-// reference's std::chrono Timer (timer.h:9-54).
-class DevClock {
+// Wall clock in milliseconds once the stream is idle, like the reference's
+// std::chrono Timer (timer.h:9-54). (The callers have mostly synchronised it
+// already: a kernel for the device's clock, its copy and their wait cost 15 us
+// each time.)
+class StreamClock {
 public:
-    explicit DevClock(cudaStream_t st) : st_(st), buf_(1, st) {}
+    explicit StreamClock(cudaStream_t st) : st_(st) {}
     double now_ms() {
-        unsigned long long t = 0;
-        k_time<<<1, 1, 0, st_>>>(0ULL, buf_.get());
-        count_launch();
-        d2h(&t, buf_.get(), sizeof(t), st_);
         sync(st_);
-        return (double)t * 1e-6;
+        return std::chrono::duration<double, std::milli>(
+                   std::chrono::steady_clock::now().time_since_epoch())
+            .count();
     }
 
 private:
     cudaStream_t st_;
-    DBuf<unsigned long long> buf_;
 };
 
 void init_gamma(QrotEngine& E, const regot_opts& o, std::vector<double>& gamma) {
@@ -3108,7 +3116,7 @@ void qrot_lbfgs_dual_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
     const int n = P->n, m = P->m, N = n + m;
     QrotEngine E(P, reg, o.tau, st);
     const bool mixed = P->prec == REGOT_PREC_MIXED;
-    DevClock clock(st);
+    StreamClock clock(st);
     lbfgs::Param param;
     param.epsilon = tol;
     param.epsilon_rel = tol;
@@ -3376,13 +3384,13 @@ private:
             k_cs_col_counts<Geo<double>::CW, Geo<double>::VW, Geo<double>::LC>
                 <<<cgrid, 128, 0, st_>>>(bm, n, m, ns, ccnt_.get());
         }
-        k_cs_col_offsets<<<cdiv(m, 128), 128, 0, st_>>>(m, kColChunks, ccnt_.get(), ccol_.get());
+        k_cs_col_offsets<<<cdiv(m, 128), 128, 0, st_>>>(m, ccnt_.get(), ccol_.get());
         k_cs_scan<<<1, 1024, 0, st_>>>(rcnt_.get(), n, rowptr_.get(), ccol_.get(), m,
                                        colptr_.get(), nnz_d_.get());
         count_launch(5);
         long long nnz[2] = {0, 0};
-        d2h(nnz, nnz_d_.get(), sizeof(nnz), st_);
-        sync(st_);
+        regot_ctx* ctx = E_.ops().problem()->ctx;
+        read_small(ctx, nnz, nnz_d_.get(), sizeof(nnz), st_);
         if (nnz[0] != nnz[1])
             throw Error(REGOT_ERR_NUMERIC, "qrot Schur CG: row and column counts of sigma differ");
         if (nnz[0] > (long long)INT32_MAX / 2) return false;
@@ -3482,10 +3490,14 @@ private:
         count_launch(3);
         out.resize(n + m);
         int it[2] = {0, 0};
-        d2h(out.data(), r1_, n * sizeof(double), st_);
-        d2h(out.data() + n, xs_, m * sizeof(double), st_);
-        d2h(it, it_d_.get(), 2 * sizeof(int), st_);
+        const size_t N = (size_t)n + m;
+        double* h = static_cast<double*>(ctx_stage(ctx, N * sizeof(double) + sizeof(it)));
+        d2h(h, r1_, n * sizeof(double), st_);
+        d2h(h + n, xs_, m * sizeof(double), st_);
+        d2h(h + N, it_d_.get(), sizeof(it), st_);
         sync(st_);
+        std::memcpy(out.data(), h, N * sizeof(double));
+        std::memcpy(it, h + N, sizeof(it));
         if (it[1])
             throw Error(REGOT_ERR_TIMEOUT,
                         "qrot Schur CG: a cluster exchange did not complete within the wait limit");
@@ -3663,7 +3675,7 @@ void qrot_lbfgs_semi_dual_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, dou
     const int n = P->n, m = P->m, N = n + m;
     const bool mixed = P->prec == REGOT_PREC_MIXED;
     QrotEngine E(P, reg, 0.0, st);
-    DevClock clock(st);
+    StreamClock clock(st);
     lbfgs::Param param;
     param.epsilon = tol;
     param.epsilon_rel = tol;
@@ -3777,7 +3789,7 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
     cudaStream_t st = ctx->stream;
     const int n = P->n, m = P->m, N = n + m;
     QrotEngine E(P, reg, 0.0, st);
-    DevClock clock(st);
+    StreamClock clock(st);
     constexpr double nu = 0.99, eta1 = 0.25, eta2 = 0.75, gamma1 = 2.0, gamma2 = 4.0,
                      lam_min = 0.01, beta_ = 0.5, cg_tol = 1e-8;
     double xi = 0.0, lam = 1.0;
@@ -3790,10 +3802,7 @@ void qrot_assn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, in
     };
     auto grad_at = [&](const std::vector<double>& x, std::vector<double>& gr, bool mask) {
         h2d(E.gamma(), x.data(), N * sizeof(double), st);
-        const double f = E.eval(E.gamma(), E.grad(), mask);
-        d2h(gr.data(), E.grad(), N * sizeof(double), st);
-        sync(st);
-        return f;
+        return E.eval(E.gamma(), E.grad(), mask, gr.data());
     };
     std::vector<double> hobj, hmar, htime, hprim;
     std::unique_ptr<SidePrimal> side;
@@ -3885,7 +3894,7 @@ void qrot_grssn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, i
     constexpr int nlinesearch = 20;
     const double shift = o.shift;
     QrotEngine E(P, reg, 0.0, st);
-    DevClock clock(st);
+    StreamClock clock(st);
     std::vector<double> gamma, newgamma(N), g(N), direc(N), rhs(N);
     init_gamma(E, o, gamma);
     QrotSchurCG cg(E, cg_tol, o.verbose);
@@ -3893,10 +3902,7 @@ void qrot_grssn_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, i
     // f, g and the generalized Hessian (sigma bitmask, h1, h2) at gamma
     auto grad_hess = [&]() {
         h2d(E.gamma(), gamma.data(), N * sizeof(double), st);
-        const double f = E.eval(E.gamma(), E.grad(), true);
-        d2h(g.data(), E.grad(), N * sizeof(double), st);
-        sync(st);
-        return f;
+        return E.eval(E.gamma(), E.grad(), true, g.data());
     };
 
     std::vector<double> hobj, hmar, htime, hprim;
@@ -3988,7 +3994,7 @@ void qrot_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int
     cudaStream_t st = ctx->stream;
     const int n = P->n, m = P->m, N = n + m;
     QrotEngine E(P, reg, 0.0, st);
-    DevClock clock(st);
+    StreamClock clock(st);
     qrot_initial(E, o, n, m);
     std::vector<double> g(N), hobj, hmar, htime, hprim;
     auto grad = [&]() {
@@ -4035,7 +4041,7 @@ void qrot_gd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int 
     constexpr double theta = 0.5, kappa = 0.5;
     constexpr int nlinesearch = 20;
     QrotEngine E(P, reg, o.tau, st);
-    DevClock clock(st);
+    StreamClock clock(st);
     qrot_initial(E, o, n, m);
     std::vector<double> gamma(N), newgamma(N), g(N), d(N), hobj, hmar, htime, hprim;
     d2h(gamma.data(), E.gamma(), N * sizeof(double), st);
@@ -4214,7 +4220,7 @@ void qrot_apdagd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, 
     constexpr int max_inner = 20;
     QrotEngine E(P, reg, 0.0, st);
     QrotAvgPlan X(ctx, E, P);
-    DevClock clock(st);
+    StreamClock clock(st);
     qrot_initial(E, o, n, m);
     HVec gamma(N), g(N), dual(N), dual_new(N), dualp(N), dualp_new(N), dualt(N), d(N);
     d2h(gamma.data(), E.gamma(), N * sizeof(double), st);
@@ -4315,7 +4321,7 @@ void qrot_pdaam_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, i
     constexpr int max_inner = 20;
     QrotEngine E(P, reg, 0.0, st);
     QrotAvgPlan X(ctx, E, P);
-    DevClock clock(st);
+    StreamClock clock(st);
     qrot_initial(E, o, n, m);
     HVec gamma(N), gt(N), g(N), dual(N), dualp(N), dualt(N), d(N);
     d2h(gamma.data(), E.gamma(), N * sizeof(double), st);
