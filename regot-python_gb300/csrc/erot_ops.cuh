@@ -69,6 +69,7 @@ public:
     // z = rx / cx entries of a CG vector) between passes.
     float4* rsplit_mut() { return rsplit_.get(); }
     float4* csplit_mut() { return csplit_.get(); }
+    float* cdsplit_mut() { return cdsplit_.get(); }
     PassParams base_params() const;
 
     // Maximum of |x| over up to two device vectors, into *out (device).

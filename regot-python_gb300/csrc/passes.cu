@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "split.cuh"
 
 namespace regot {
 
@@ -38,38 +39,19 @@ int device_sm_count() {
 namespace {
 std::atomic<long long> g_wait_limit{kDefaultWaitSpins};
 
-__device__ __forceinline__ void split(double v, double g, double inv_g, float& hi, float& lo) {
-    if (!isfinite(v)) {
-        hi = (float)v;
-        lo = 0.f;
-        return;
-    }
-    const double h = rint(v * inv_g) * g;
-    hi = (float)h;
-    lo = (float)(v - h);
-}
-
 // FP32 copies of the per-row / per-column vectors of a mixed pass; the duals
 // are split on the common grid G = 2^(floor(log2 bound) - 21).
 __global__ void k_split(const PassParams p, float4* rs, float4* cs, float* cds) {
-    double g = 1.0, inv_g = 1.0;
-    if (p.grid) {
-        const double mx = *p.grid;
-        if (mx > 0.0 && isfinite(mx)) {
-            const int e = ilogb(mx) - 21;
-            g = ldexp(1.0, e);
-            inv_g = ldexp(1.0, -e);
-        }
-    }
+    const SplitGrid grid(p.grid);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < p.n) {
         float hi = 0.f, lo = 0.f;
-        if (p.ra) split(p.ra[t], g, inv_g, hi, lo);
+        if (p.ra) grid.split(p.ra[t], hi, lo);
         rs[t] = make_float4(hi, lo, p.rx ? (float)p.rx[t] : 0.f, p.rd ? (float)p.rd[t] : 0.f);
     } else if (t < p.n + p.m) {
         const int j = t - p.n;
         float hi = 0.f, lo = 0.f;
-        if (p.cb) split(p.cb[j], g, inv_g, hi, lo);
+        if (p.cb) grid.split(p.cb[j], hi, lo);
         cs[j] = make_float4(hi, lo, p.cx ? (float)p.cx[j] : 0.f, p.cx2 ? (float)p.cx2[j] : 0.f);
         if (cds) cds[j] = p.cd ? (float)p.cd[j] : 0.f;
     }

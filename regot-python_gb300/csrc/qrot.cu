@@ -44,6 +44,7 @@
 #include "erot_ops.cuh"
 #include "lbfgs.h"
 #include "solvers.h"
+#include "split.cuh"
 
 namespace regot {
 
@@ -2497,14 +2498,21 @@ __global__ void __launch_bounds__(512) k_lb_merge(
 }
 
 // drt = cv g + sum_k cy[k] y_k + cs[k] s_k over the stored pairs, and g'drt.
-// With xt given, also the first trial point xt = xp + step drt.
+// With xt given, also the first trial point xt = xp + step drt and (mixed) the
+// split of xp and drt that the trial pass reads: a launch of 4 us less a trial.
+struct LbSplit {
+    const double* grid = nullptr;  // max |xp|
+    float4 *rs = nullptr, *cs = nullptr;
+    float* cds = nullptr;
+    int n = 0;
+};
 __global__ void __launch_bounds__(kLbBlock) k_lb_dir(const double* __restrict__ g,
                                                      const double* __restrict__ pairs, int N,
                                                      double* __restrict__ drt, double* parts,
                                                      unsigned* counter,
                                                      const LbCoef* __restrict__ cf, LbScal* out,
                                                      const double* __restrict__ xp, double step,
-                                                     double* __restrict__ xt) {
+                                                     double* __restrict__ xt, LbSplit sp) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     double v[1] = {0.0};
     if (t < N) {
@@ -2527,7 +2535,20 @@ __global__ void __launch_bounds__(kLbBlock) k_lb_dir(const double* __restrict__ 
             }
         }
         drt[t] = d;
-        if (xt) xt[t] = xp[t] + step * d;
+        if (xt) {
+            const double x0 = xp[t];
+            xt[t] = x0 + step * d;
+            if (sp.rs) {
+                float hi, lo;
+                SplitGrid(sp.grid).split(x0, hi, lo);
+                if (t < sp.n) {
+                    sp.rs[t] = make_float4(hi, lo, 0.f, (float)d);
+                } else {
+                    sp.cs[t - sp.n] = make_float4(hi, lo, 0.f, 0.f);
+                    sp.cds[t - sp.n] = (float)d;
+                }
+            }
+        }
         v[0] = gt * d;
     }
     __shared__ double r[1];
@@ -2827,11 +2848,19 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
         try {
             REGOT_CUDA(cudaMemcpyAsync(dcoef.get(), coef, sizeof(LbCoef),
                                        cudaMemcpyHostToDevice, st));
+            LbSplit sp;
+            if (mixed) {
+                sp.grid = xmax.get() + xi;
+                sp.rs = ops.rsplit_mut();
+                sp.cs = ops.csplit_mut();
+                sp.cds = ops.cdsplit_mut();
+                sp.n = n;
+            }
             k_lb_dir<<<gN, kLbBlock, 0, st>>>(gbuf(gi), pairs.get(), N, drt.get(), parts.get(),
                                               counter.get(), dcoef.get(), dscal.get(), xbuf(xi),
-                                              1.0, xbuf((xi + 1) % kLbBufs));
+                                              1.0, xbuf((xi + 1) % kLbBufs), sp);
             count_launch();
-            trial_launch(xi, gi, (xi + 1) % kLbBufs, (gi + 1) % kLbBufs, 1.0, true, true);
+            trial_launch(xi, gi, (xi + 1) % kLbBufs, (gi + 1) % kLbBufs, 1.0, false, true);
         } catch (...) {
             cudaGraph_t g = nullptr;
             cudaStreamEndCapture(st, &g);
@@ -2910,7 +2939,7 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
         h2d(dcoef.get(), coef, sizeof(LbCoef), st);
         k_lb_dir<<<gN, kLbBlock, 0, st>>>(gbuf(ig), pairs.get(), N, drt.get(), parts.get(),
                                           counter.get(), dcoef.get(), dscal.get(), nullptr, 0.0,
-                                          nullptr);
+                                          nullptr, LbSplit());
         count_launch();
         REGOT_CHECK_LAUNCH();
         double step = 1.0 / gnorm;
