@@ -77,7 +77,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     const int items = R + C, iwarps = (items + 31) / 32 < kResWarps ? (items + 31) / 32 : kResWarps;
 
     // Pairs (v0, v1) summed over the block's item threads into red[slot][b]:
-    // called by all threads (the warps without items only synchronise).
+    // called by all threads (the warps without items only synchronise). A slot is
+    // written again only behind a barrier of all blocks that follows its last
+    // total(): slot 0 of a step is written in the phase after the residual's
+    // totals are read, so those (of the first residual too) are in slot 1.
     auto publish = [&](int slot, double v0, double v1) {
         if (warp < iwarps) {
             const bool upper = (lane & 16) != 0;
@@ -153,7 +156,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
         }
         __syncthreads();
         publish_z();
-        publish(0, v[0], v[1]);
+        publish(1, v[0], v[1]);
         __syncthreads();
         publish(2, v[2], v[3]);
     }
@@ -163,9 +166,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     double rz = 0.0, thresh2 = 0.0;
     const int cg_max = p.st->cg_max;
     if (warp == 0) {
-        const double2 q0 = total(0), q2 = total(2);
-        const double rr0 = q0.x, sr = q2.x, sg = q2.y;
-        rz = q0.y;
+        const double2 q1 = total(1), q2 = total(2);
+        const double rr0 = q1.x, sr = q2.x, sg = q2.y;
+        rz = q1.y;
         if (lane == 0) {
             thresh2 = fmax(p.cg_tol * p.cg_tol * rr0, 2.2250738585072014e-308);
             int stop = rr0 == 0.0 || rr0 < thresh2 ? 1 : 0;
