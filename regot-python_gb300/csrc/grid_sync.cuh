@@ -2,7 +2,10 @@
 // cooperative launch (one counter in global memory), or the blocks of one
 // thread-block cluster (the hardware's cluster barrier). Both order global
 // memory: what a block wrote before it arrived is seen, through L2 (__ldcg),
-// by every block after it waited.
+// by every block after it waited. arrive() is a barrier of the block in both
+// forms: a warp goes on behind it only when no other of the block's still reads
+// or writes shared memory before it. (The cluster's own arrive does not wait, so
+// a warp past it could write what another was about to read.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -57,7 +60,7 @@ template <>
 struct GridBarrier<true> {
     __device__ GridBarrier(unsigned*, int*, int*) {}
     __device__ void arrive() {
-        __syncwarp();
+        __syncthreads();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     }
     __device__ bool wait() {

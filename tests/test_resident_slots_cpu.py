@@ -69,3 +69,20 @@ def test_slots_are_rewritten_behind_a_barrier(file, kernel):
     assert {"publish", "total", "wait"} <= {c[0] for c in pre} and len(turn) >= 6
     for turns in (0, 1, 2, 3):
         assert _violations(pre + turns * turn + post) == []
+
+
+@pytest.mark.parametrize("form", ["false", "true"])
+def test_arriving_at_a_barrier_orders_the_block(form):
+    """GridBarrier::arrive() (csrc/grid_sync.cuh) stands between a block's
+    reading of its shared memory and its warps' next writing of it: in both
+    forms all of the block's threads pass a barrier of the block before one of
+    them goes on. The cluster's arrive instruction alone lets a warp go on
+    while another still reads."""
+    with open(os.path.join(CSRC, "grid_sync.cuh")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    start = text.index("struct GridBarrier<%s> {" % form)
+    body = text[start:_block(text, start)]
+    at = body.index("void arrive()")
+    arrive = body[at:_block(body, at)]
+    assert "__syncthreads();" in arrive
+    assert arrive.index("__syncthreads();") < arrive.index("asm volatile")
