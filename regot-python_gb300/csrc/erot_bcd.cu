@@ -171,6 +171,9 @@ __global__ void k_bcd_row(const Acc* rp, int nslabs, int n, const double* anchor
             }
         }
         __syncwarp();
+        // a dual off the split grid is flagged before warp 1 arrives at the grid's
+        // counter: the last block records the iterate only if no block flagged one
+        if (so.out) asm volatile("bar.arrive 1, 64;" ::: "memory");
         warp_atomic_max_abs(&st->maxabs, vmax);
         return;
     }
@@ -183,11 +186,11 @@ __global__ void k_bcd_row(const Acc* rp, int nslabs, int n, const double* anchor
         v[1] = r;
         v[2] = ai * al;
     }
+    __syncwarp();
+    if (so.out) asm volatile("bar.sync 1, 64;" ::: "memory");
     __threadfence();
     double out[3];
     if (warp_grid_reduce<3>(v, parts, &st->counter, out) && threadIdx.x == 0) {
-        // (a dual off the split grid may show only in the column finalize, which
-        // stops the sweeps before it advances)
         if (atomicAdd(&st->bad, 0)) {
             st->done = 1;
             return;

@@ -39,3 +39,32 @@ def test_newton_is_the_same_from_run_to_run(n, m):
         q = P.sinkhorn_newton(0.02, tol=1e-9, max_iter=50)
         assert np.array_equal(q.obj_vals, r.obj_vals) and np.array_equal(q.dual, r.dual)
     P.close()
+
+
+@pytest.mark.parametrize("n,m,reg", [(100, 80, 0.05), (33, 2000, 0.02), (3000, 400, 0.01),
+                                     (2049, 2049, 0.01)])
+def test_first_record_from_a_dual_off_the_split_grid(n, m, reg):
+    # Mixed precision from a dual far below its final size: the first row update
+    # leaves the grid of the FP32 splits, iterate 0 is handed to the general path
+    # unrecorded, and its marginal error keeps the column part, which only a user's
+    # dual has. The FP32 sums of the plan entries (FP32 exponentials at arguments
+    # up to 1 / reg: a few 1e-6 relative each) bound the difference.
+    M, a, b = erot_points(n, m, seed=5)
+    x0 = np.full(n + m - 1, 1e-4)
+    o = O.sinkhorn_bcd(M.astype(np.float64), a, b, reg, tol=1e-13, max_iter=2, x0=x0)
+    T = np.exp((2e-4 - M.astype(np.float64)) / reg)
+    T[:, -1] = np.exp((1e-4 - M[:, -1].astype(np.float64)) / reg)
+    rows, cols = T.sum(1) - a, (T.sum(0) - b)[:-1]
+    want = np.sqrt((rows ** 2).sum() + (cols ** 2).sum())
+    np.testing.assert_allclose(o.mar_errs[0], want, rtol=1e-9)
+    assert (cols ** 2).sum() > 0.01 * want ** 2  # the part that could go missing
+    P = regot.Problem(M, a, b, precision="mixed")
+    first = None
+    for _ in range(25):
+        r = P.sinkhorn_bcd(reg, tol=1e-13, max_iter=2, x0=x0)
+        np.testing.assert_allclose(r.mar_errs[0], want, rtol=1e-4)
+        first = r if first is None else first
+        assert np.array_equal(r.mar_errs, first.mar_errs)
+        assert np.array_equal(r.obj_vals, first.obj_vals)
+        assert np.array_equal(r.dual, first.dual)
+    P.close()
