@@ -283,11 +283,15 @@ constexpr long long kClusterEntries = 64 * 1024;
 // solvers keep to the dense passes.
 constexpr double kPlanMaxBytes = 32.0 * (1ULL << 30);
 
-inline size_t max_block_smem() {
+// The most dynamic shared memory a block of `kernel` may have: what its static
+// arrays leave (k_plan_cg32 has 4.6 KB of them).
+inline size_t max_block_smem(const void* kernel) {
     int dev = 0, optin = 0;
+    cudaFuncAttributes at;
     REGOT_CUDA(cudaGetDevice(&dev));
     REGOT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    return (size_t)optin - 1024;  // static shared memory of the kernels
+    REGOT_CUDA(cudaFuncGetAttributes(&at, kernel));
+    return (size_t)optin - at.sharedSizeBytes;
 }
 
 inline cudaLaunchConfig_t resident_config(cudaLaunchAttribute* at, bool cluster, int blocks,
@@ -313,7 +317,9 @@ inline cudaLaunchConfig_t resident_config(cudaLaunchAttribute* at, bool cluster,
 // Whether `kernel` runs n m = entries entries in one cluster of 16 blocks.
 template <typename P>
 bool resident_cluster(void (*kernel)(P), long long entries, size_t smem) {
-    if (entries > kClusterEntries || smem > max_block_smem()) return false;
+    if (entries > kClusterEntries ||
+        smem > max_block_smem(reinterpret_cast<const void*>(kernel)))
+        return false;
     cudaLaunchAttribute at[1];
     const cudaLaunchConfig_t cfg = resident_config(at, true, 16, smem, nullptr);
     int clusters = 0;
@@ -333,7 +339,7 @@ bool resident_grid(void (*kernel)(P), size_t smem) {
     int dev = 0, coop = 0, occ = 0;
     REGOT_CUDA(cudaGetDevice(&dev));
     REGOT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop || smem > max_block_smem()) return false;
+    if (!coop || smem > max_block_smem(reinterpret_cast<const void*>(kernel))) return false;
     REGOT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     REGOT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kResThreads, smem));
     return occ >= 1;
