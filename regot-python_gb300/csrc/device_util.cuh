@@ -5,7 +5,11 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
+#include <limits>
+#include <map>
+#include <mutex>
 #include <utility>
 
 #include "internal.h"
@@ -371,6 +375,32 @@ __device__ __forceinline__ double max_2d(const Acc* p, int count, size_t stride,
         for (int q = 0; q < 8; ++q) r = fmax(r, s_mx[q][threadIdx.x]);
     }
     return (double)r;
+}
+
+// The most dynamic shared memory a block of `kernel` may have: what its static
+// arrays leave. The kernel is opted in to all of
+// it, and to clusters of 16, once a device: these attributes belong to the
+// function, for every thread and context of the process, so a problem's own size
+// must not be written there (a smaller solve beside it would take back what
+// another is about to launch with).
+inline size_t max_block_smem(const void* kernel) {
+    static std::mutex mutex;
+    static std::map<std::pair<const void*, int>, size_t> limits;
+    int dev = 0, optin = 0;
+    REGOT_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mutex);
+    auto it = limits.find({kernel, dev});
+    if (it != limits.end()) return it->second;
+    cudaFuncAttributes at;
+    REGOT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    REGOT_CUDA(cudaFuncGetAttributes(&at, kernel));
+    const size_t most = (size_t)optin - at.sharedSizeBytes;
+    REGOT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+    // refused where a device has no such clusters: the grid form runs there
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        cudaGetLastError();
+    limits[{kernel, dev}] = most;
+    return most;
 }
 
 // The largest x >= 0 with sqrt(x) < tol, so that the kernel's test on squares

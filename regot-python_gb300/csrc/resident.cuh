@@ -283,17 +283,6 @@ constexpr long long kClusterEntries = 64 * 1024;
 // solvers keep to the dense passes.
 constexpr double kPlanMaxBytes = 32.0 * (1ULL << 30);
 
-// The most dynamic shared memory a block of `kernel` may have: what its static
-// arrays leave (k_plan_cg32 has 4.6 KB of them).
-inline size_t max_block_smem(const void* kernel) {
-    int dev = 0, optin = 0;
-    cudaFuncAttributes at;
-    REGOT_CUDA(cudaGetDevice(&dev));
-    REGOT_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    REGOT_CUDA(cudaFuncGetAttributes(&at, kernel));
-    return (size_t)optin - at.sharedSizeBytes;
-}
-
 inline cudaLaunchConfig_t resident_config(cudaLaunchAttribute* at, bool cluster, int blocks,
                                           size_t smem, cudaStream_t st) {
     if (cluster) {
@@ -324,10 +313,6 @@ bool resident_cluster(void (*kernel)(P), long long entries, size_t smem) {
     const cudaLaunchConfig_t cfg = resident_config(at, true, 16, smem, nullptr);
     int clusters = 0;
     const bool ok =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-            cudaSuccess &&
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-            cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
     if (!ok) cudaGetLastError();
     return ok;
@@ -340,7 +325,6 @@ bool resident_grid(void (*kernel)(P), size_t smem) {
     REGOT_CUDA(cudaGetDevice(&dev));
     REGOT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop || smem > max_block_smem(reinterpret_cast<const void*>(kernel))) return false;
-    REGOT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     REGOT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kResThreads, smem));
     return occ >= 1;
 }
