@@ -1076,9 +1076,7 @@ void r_dispatch(int vpt, F&& f) {
 template <typename Kern>
 int r_grid(Kern kern, int count, size_t smem) {
     // the row buffer may exceed the default 48 KB of dynamic shared memory
-    // (idempotent; host threads may race here)
-    REGOT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+    max_block_smem(reinterpret_cast<const void*>(kern));
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kRT, smem) != cudaSuccess ||
         occ < 1)
@@ -1671,19 +1669,13 @@ public:
         const int sms = device_sm_count();
         col_cache_ = (size_t)ldt_ * sizeof(TM) <= kMaxCacheBytes;
         const size_t col_smem = col_cache_ ? (size_t)ldt_ * sizeof(TM) : 0;
-        REGOT_CUDA(cudaFuncSetAttribute(k_col_select<TM>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)col_smem));
-        REGOT_CUDA(cudaFuncSetAttribute(k_csc_fill<TM>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)col_smem));
+        max_block_smem(reinterpret_cast<const void*>(k_col_select<TM>));
+        max_block_smem(reinterpret_cast<const void*>(k_csc_fill<TM>));
         col_smem_ = col_smem;
         const long long rowpad = ((long long)m1_ + 3) & ~3LL;
         row_cache_ = 2 * (size_t)rowpad * sizeof(TM) <= kMaxCacheBytes;
         row_smem_ = row_cache_ ? 2 * (size_t)rowpad * sizeof(TM) : 0;
-        REGOT_CUDA(cudaFuncSetAttribute(k_row_stage<TM>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)row_smem_));
+        max_block_smem(reinterpret_cast<const void*>(k_row_stage<TM>));
         col_grid_ = std::max(1, std::min(m1_, sms * 4));
         row_grid_ = std::max(1, std::min(n_, sms * 4));
         if (!row_cache_) row_scratch_.alloc((size_t)row_grid_ * 2 * rowpad, st_);

@@ -56,6 +56,8 @@ def _solves(solver, precision, sizes, reg, count, errors, results, **kw):
     ("sinkhorn_newton", "mixed", dict(tol=1e-5, max_iter=20)),
     ("sinkhorn_newton", "fp64", dict(tol=1e-8, max_iter=20)),
     ("sinkhorn_bcd", "fp64", dict(tol=1e-8, max_iter=60)),
+    ("sinkhorn_ssns", "fp64", dict(tol=1e-8, max_iter=200)),
+    ("sinkhorn_ssns", "mixed", dict(tol=1e-5, max_iter=200)),
 ])
 def test_two_threads_solve_two_sizes_at_once(solver, precision, kw, monkeypatch):
     monkeypatch.setattr(_lib, "context", lambda device=0: _thread.ctx)
