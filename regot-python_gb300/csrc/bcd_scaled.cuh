@@ -9,8 +9,9 @@
 // algorithms for entropy regularized transport problems", SIAM J. Sci.
 // Comput. 41, 2019) in place of two exponentials an entry. All arithmetic is
 // FP64. The base duals move ("absorption": K is rebuilt at the current
-// duals) when a scaling leaves 2^-kScaleLim .. 2^kScaleLim, so that what K
-// loses to underflow stays far below the rounding of any sum.
+// duals) when a scaling leaves 2^-kScaleLim .. 2^kScaleLim, and no sum beyond
+// 2^-kSumLim .. 2^kSumLim is used, so that what K loses to underflow stays far
+// below the rounding of any sum.
 //
 // One cooperative launch runs the sweeps to the stop, one block an SM (or one
 // cluster of 16 blocks for small problems, whose barrier is cheaper): blocks
@@ -24,8 +25,15 @@
 namespace regot {
 namespace {
 
-constexpr int kScaleLim = 100;   // scalings stay within 2^-100 .. 2^100
-constexpr int kSumLim = 896;     // sums within 2^-896 .. 2^896 are exact enough
+constexpr int kScaleLim = 100;   // scalings beyond 2^-100 .. 2^100 end a launch
+// Sums beyond 2^-kSumLim .. 2^kSumLim go to the max-anchored updates. A launch ends
+// one sweep after a scaling left its range, so that scaling, up to a / s, meets K
+// once more: an entry of K is off by up to 2^-1075 (what underflow loses), n of
+// them times a scaling of 2^480 by n 2^-595, which a sum of at least 2^-480 has
+// 115 - log2 n bits below its leading one. (Sums down to 2^-896 were taken before:
+// a row at 2^-866 got the scaling 2^865, and a column whose largest entry it was
+// came out of what was left, wrong by hundreds of reg in its dual.)
+constexpr int kSumLim = 480;
 constexpr double kMinMarginal = 1e-150;
 
 struct ScaledParams {
