@@ -444,11 +444,15 @@ int regot_time_pass(regot_ctx* ctx, regot_dproblem* prob, int kind, double reg, 
  * writes); -1 for an invalid argument. */
 long long regot_pass_bytes(regot_dproblem* prob, int kind);
 /* Limit (polls of about 200 us) of the dense passes' bounded waits on their
- * parameter copies; returns the previous limit, and a negative value
+ * parameter copies, and (256 polls of about a microsecond for each) of the
+ * barriers between the blocks of the kernels that run many sweeps or CG steps
+ * in one launch; returns the previous limit, and a negative value
  * restores the default (16384). A pass whose wait gives up drains the copy
- * under the default limit, marks its result invalid and the call returns
- * REGOT_ERR_TIMEOUT; 0 makes every such wait give up at once. Process-wide;
- * for exercising the timeout path. No counterpart in the reference. */
+ * under the default limit, a block whose barrier gives up leaves, and the call
+ * returns REGOT_ERR_TIMEOUT; 0 makes every such wait give up at once. (The
+ * barriers of one thread-block cluster are the hardware's and have no limit.)
+ * Process-wide; for exercising the timeout path. No counterpart in the
+ * reference. */
 long long regot_set_wait_limit(long long spins);
 
 /* ---- Autotuner of the dense passes (no counterpart in the reference,

@@ -52,7 +52,8 @@ struct ScaledParams {
     double* blast;    // beta_{m-1}
     double* fin;      // [G + 1]: the last iterate's sums of b beta~, beta_{m-1}
     unsigned* count;  // grid barrier
-    int* err;
+    int* err;        // set when a barrier gives up
+    unsigned polls;  // before it does
     BcdState* st;
     double *hobj, *hmar, *htime;
     int first_col;  // start with v = b / K'1 (beta0 is an anchor, alpha0 = 0)
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_bcd_scaled(const ScaledParam
     double* s_c = s_vp + Cm;                     // [Cm] own columns' sums
     double* s_wa = s_c + Cm;                     // [kResWarps] sums of a alpha
     double* s_wb = s_wa + kResWarps;             // [kResWarps] sums of b beta~
-    GridBarrier<CLUSTER> bar(p.count, p.err, &s_ok);
+    GridBarrier<CLUSTER> bar(p.count, p.err, p.polls, &s_ok);
 
     for (int j = tid; j < ldk; j += kResThreads) s_v[j] = j < m ? 1.0 : 0.0;
     for (int r = tid; r < R; r += kResThreads) s_u[r] = s_un[r] = 1.0;

@@ -79,7 +79,7 @@ struct BatchState {
     int loops;
     int loop_cap;
     int stop_below;  // leave the device loop when this few problems still run
-    int err;         // a bounded wait of a tensor-core sweep gave up
+    int err;         // a bounded wait gave up: 1 of a tensor-core sweep, 2 of a team
     double maxabs;  // max |dual| for the grid
     double g, inv_g, bound;
 };
@@ -715,6 +715,7 @@ struct TailArgs {
     const int* plist;  // the running problems, one per cluster (k_btail)
     const int4* team;  // problem, rank and CTAs of each CTA's team (k_bteam)
     unsigned* count;   // barrier of each problem's team, zero at the launch
+    unsigned polls;    // before such a barrier gives up
     const int* pcls;   // dimension class of each problem
     float2* as[2];
     double* a[2];
@@ -752,12 +753,12 @@ struct ClusterTeam {
 
 // Barrier of a problem's team of CTAs of one cooperative launch: a counter in
 // global memory that only grows. A wait that gives up (after some seconds) sets
-// st->err, at which the waits of all teams end.
+// st->err, at which the waits of all teams end within 1024 polls.
 struct GridTeam {
     unsigned* count;
     BatchState* st;
     int size;
-    unsigned target;
+    unsigned target, polls;
     __device__ bool sync() {
         __shared__ int s_ok;
         __syncthreads();
@@ -765,7 +766,7 @@ struct GridTeam {
         if (threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
             int ok = 0;
-            for (unsigned s = 0; s < kGridSpins; ++s) {
+            for (unsigned s = 0; s < polls; ++s) {
                 unsigned c;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
                 if ((int)(c - target) >= 0) {
@@ -872,7 +873,7 @@ __global__ void __launch_bounds__(kBWarps * 32, 2) k_bteam(const TailArgs a) {
     const int p = t.x;
     float2* spts = tail_smem;
     float2* spar = tail_smem + kBTile * (kBClassDim[kBClasses - 1] + 1);
-    const GridTeam team{a.count + p, a.st, t.z, 0u};
+    const GridTeam team{a.count + p, a.st, t.z, 0u, a.polls};
     switch (a.pcls[p]) {
         case 0: tail_solve<4>(a, p, t.y, t.z, team, spts, spar); break;
         case 1: tail_solve<8>(a, p, t.y, t.z, team, spts, spar); break;
@@ -1629,6 +1630,7 @@ void erot_solve_batched_gpu(regot_ctx* ctx, const regot_batch_desc* D, double re
             ta.plist = plist.get();
             ta.team = dteam.get();
             ta.count = tcount.get();
+            ta.polls = grid_polls();
             ta.pcls = dcls.get();
             for (int q = 0; q < 2; ++q) {
                 ta.as[q] = AS[q].get();

@@ -52,7 +52,7 @@ struct BcdState {
     unsigned counter;
     int loops;     // bodies of the device-side sweep loop run so far
     int loop_cap;  // hard bound on loops (the loop kernel stops there)
-    int pad;
+    int err;       // a barrier of the sweeps on the stored plan gave up
     double tol;
     double sum_bb;     // sum_{j<m-1} b_j beta_j of the current beta
     double beta_last;  // beta_{m-1}
@@ -510,7 +510,8 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
         q.fin = q.blast + 1;
         q.redf = reinterpret_cast<int*>(q.fin + sp.blocks + 1);
         q.count = reinterpret_cast<unsigned*>(q.redf + sp.blocks);
-        q.err = ops.err_flag();
+        q.err = &S->err;
+        q.polls = grid_polls();
         q.st = S;
         q.hobj = hobj;
         q.hmar = hmar;
@@ -526,8 +527,8 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
             launch_scaled(sp, q, st);
             REGOT_CHECK_LAUNCH();
             read_state();
+            check_barriers(hs.err);
             if (hs.done) break;
-            ops.check_err();
             q.first_col = 0;
             if (hs.bad) robust(hs.bad);
         }

@@ -279,7 +279,7 @@ void newton_on_plan(regot_ctx* ctx, regot_dproblem* P, ErotOps& ops, PlanCgLaunc
         double tots[4];
         d2h(tots, lsout.get(), sizeof(double), st);
         read_small(ctx, &hs, S, sizeof(hs), st);
-        if (!hs.cg_done) ops.check_err();
+        check_barriers(hs.err);
         *passes += 1;
         if (i == max_iter) break;
         if (o.verbose >= 1)
@@ -370,7 +370,7 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
 
     if (!mixed) {
         PlanCgLaunch L;
-        L.init(P, reg, S, ops.err_flag(), st);
+        L.init(P, reg, S, st);
         if (L.ok) {
             int niter = 0, len = 0;
             long long np = 0;
@@ -515,7 +515,7 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
         const double full = 1.0;
         try_steps(&full, 1);
         read_small(ctx, &hs, S, sizeof(hs), st);
-        if (!hs.cg_done) ops.check_err();
+        check_barriers(hs.err);
         if (L32.ok) passes += hs.cg_it;
         const double thresh = theta * hs.gtd;
         double step = 1.0, accepted = -1.0;
@@ -587,7 +587,7 @@ void erot_hess_solve_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, const do
     }
     if (!mixed) {
         PlanCgLaunch L;
-        L.init(P, reg, S, ops.err_flag(), st);
+        L.init(P, reg, S, st);
         if (L.ok) {
             L.p.rhs = rhs.get();
             L.p.cg_tol = tol;
@@ -596,7 +596,7 @@ void erot_hess_solve_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, const do
             L.solve(st);
             NewtonState hs{};
             read_small(ctx, &hs, S, sizeof(hs), st);
-            if (!hs.cg_done) ops.check_err();
+            check_barriers(hs.err);
             read_small(ctx, x_h, x.get(), (size_t)(n + m - 1) * sizeof(double), st);
             if (iters) *iters = hs.cg_it;
             return;
@@ -626,7 +626,7 @@ void erot_hess_solve_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, const do
         L32.solve(ops.rsplit(), ops.csplit(), rhs.get(), 1.0, hdiag.get(), tol, x.get(), st);
         NewtonState done{};
         read_small(ctx, &done, S, sizeof(done), st);
-        if (!done.cg_done) ops.check_err();
+        check_barriers(done.err);
         read_small(ctx, x_h, x.get(), (size_t)(n + m - 1) * sizeof(double), st);
         if (iters) *iters = done.cg_it;
         ops.check_err();

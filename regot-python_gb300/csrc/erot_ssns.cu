@@ -83,6 +83,7 @@ struct SsnState {
     int done;
     int it;
     int max_it;
+    int err;         // a barrier of a resident kernel gave up
     double shift;
     double absnew;   // r'z of the CG residual
     double alpha;
@@ -1497,10 +1498,11 @@ __global__ void k_ssns_grad(const Acc* rp, int nslabs, const Acc* cp, int nrb, i
     }
 }
 
-// The objective and gradient norm that the stored plan's gradient left.
+// The objective, gradient norm and barrier flag that the stored plan's gradient left.
 __global__ void k_ssns_take(const NewtonState* ns, SsnState* st) {
     st->f = ns->f;
     st->gnorm = ns->gnorm;
+    if (ns->err) st->err = ns->err;
 }
 
 __global__ void k_ssns_move(int N, double s, const double* d, double* gamma) {
@@ -1696,8 +1698,8 @@ public:
         if (!mixed_) {
             ns_.alloc(1, st_);
             ns_.zero();
-            plan_.init(P, reg, ns_.get(), ops_.err_flag(), st_);
-            schur_.init(S_, state_.get(), ops_.err_flag(), st_);
+            plan_.init(P, reg, ns_.get(), st_);
+            schur_.init(S_, state_.get(), st_);
         }
         if (mixed_) {
             u2_.alloc(n_, st_);
@@ -1721,6 +1723,7 @@ public:
     SsnState read_state() {
         SsnState hs;
         read_small(P_->ctx, &hs, state_.get(), sizeof(hs), st_);
+        check_barriers(hs.err);
         return hs;
     }
 
@@ -2233,7 +2236,6 @@ void run_ssns(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int max
         E.direction(shift);
         E.dir_dots();
         hs = E.read_state();
-        if (!hs.done) ops.check_err();  // the CG's launch gave up a wait
         const double gtd = hs.gtd, dhd = hs.dhd;
         // line_selection: first candidate below f, else the best. The full
         // step is evaluated alone first (one series per entry instead of
@@ -2387,7 +2389,7 @@ void run_sparse_newton(regot_ctx* ctx, regot_dproblem* P, double reg, double tol
             d2h(iy.data(), E.dir(), (size_t)N * sizeof(double), st);
             E.direction(shift, nullptr, 1);
             d2h(ir.data(), E.dir(), (size_t)N * sizeof(double), st);
-            sync(st);
+            E.read_state();  // synchronises, and checks the CG's barriers
             double rs = 0.0, yiy = 0.0, yir = 0.0;
             for (int q = 0; q < N1; ++q) {
                 rs -= sv[q] * g[q];
@@ -2402,7 +2404,7 @@ void run_sparse_newton(regot_ctx* ctx, regot_dproblem* P, double reg, double tol
         } else {
             E.direction(shift);
             d2h(dir.data(), E.dir(), (size_t)N * sizeof(double), st);
-            sync(st);
+            E.read_state();  // synchronises, and checks the CG's barriers
         }
         // Wolfe line search: one pass per trial
         const double g0d = dot(g, dir);

@@ -12,24 +12,24 @@
 
 namespace regot {
 
-// Polls of the grid barrier before it gives up (each a round trip to L2,
-// about a microsecond: some seconds in all).
-constexpr unsigned kGridSpins = 1u << 22;
-
 template <bool CLUSTER>
 struct GridBarrier;
 
 // count starts at 0 and only grows; generation g is complete at g * gridDim.x
-// arrivals. *err is set when a wait gives up; every later wait returns false
-// at once then, so all blocks leave within one limit.
+// arrivals. A wait gives up after `polls` of them (each a round trip to L2, about
+// a microsecond; grid_polls()) and sets *err. Its block leaves, so no later
+// generation completes, and the waits for one end within 1024 polls of seeing
+// *err; a wait whose generation was complete still returns true. The host looks at
+// *err after every launch.
 template <>
 struct GridBarrier<false> {
     unsigned* count;
     int* err;
-    unsigned target;
+    unsigned target, polls;
     int* s_ok;  // one int of shared memory
 
-    __device__ GridBarrier(unsigned* c, int* e, int* s) : count(c), err(e), target(0), s_ok(s) {}
+    __device__ GridBarrier(unsigned* c, int* e, unsigned p, int* s)
+        : count(c), err(e), target(0), polls(p), s_ok(s) {}
     __device__ void arrive() {
         __syncthreads();
         target += gridDim.x;
@@ -39,7 +39,7 @@ struct GridBarrier<false> {
     __device__ bool wait() {
         if (threadIdx.x == 0) {
             int ok = 0;
-            for (unsigned s = 0; s < kGridSpins; ++s) {
+            for (unsigned s = 0; s < polls; ++s) {
                 unsigned c;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
                 if ((int)(c - target) >= 0) {
@@ -58,7 +58,7 @@ struct GridBarrier<false> {
 
 template <>
 struct GridBarrier<true> {
-    __device__ GridBarrier(unsigned*, int*, int*) {}
+    __device__ GridBarrier(unsigned*, int*, unsigned, int*) {}
     __device__ void arrive() {
         __syncthreads();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

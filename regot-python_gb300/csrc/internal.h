@@ -144,6 +144,14 @@ constexpr long long kDefaultWaitSpins = 1LL << 14;
 // timeout path without a fault.
 long long wait_limit();
 long long set_wait_limit(long long spins);
+// Polls (of about a microsecond) of the resident kernels' barriers under the same
+// limit: 2^22, some seconds, by default.
+unsigned grid_polls();
+// Throws REGOT_ERR_TIMEOUT if the flag of a resident kernel's barriers is set.
+inline void check_barriers(int err) {
+    if (err)
+        throw Error(REGOT_ERR_TIMEOUT, "a resident kernel's blocks gave up waiting for one another");
+}
 
 struct PassShape {
     int nslabs, nrb, ntiles;

@@ -33,7 +33,8 @@ struct PlanCgParams {
     double* zbuf;     // [ldk]
     double* red;      // [3][G][2]: pairs of block sums
     unsigned* count;
-    int* err;
+    int* err;        // set when a barrier gives up
+    unsigned polls;  // before it does
     NewtonState* st;
     double *hobj, *hmar, *htime;  // gradient mode: this iterate's record (or null)
     double* hdiag;                // gradient alone: diag(H) [n + m] out, no solve
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg(const PlanCgParams p
     double* s_z = s_r + Im;
     double* s_y = s_z + Im;   // (T'p)_j of the own columns, at R + j
     double* s_w = s_y + Im;   // [2][kResWarps]
-    GridBarrier<CLUSTER> bar(p.count, p.err, &s_ok);
+    GridBarrier<CLUSTER> bar(p.count, p.err, p.polls, &s_ok);
     const double reg = p.reg;
     const int S = row_segments((int)(ldk >> 1), R);
     const int items = R + C, iwarps = (items + 31) / 32 < kResWarps ? (items + 31) / 32 : kResWarps;
@@ -338,7 +339,7 @@ struct PlanCgLaunch {
     PlanCgParams p{};
 
     // Room and launch for n x m, or ok = false.
-    void init(regot_dproblem* P, double reg, NewtonState* S, int* err, cudaStream_t st) {
+    void init(regot_dproblem* P, double reg, NewtonState* S, cudaStream_t st) {
         const int n = P->n, m = P->m;
         ldk = ((long long)m + 1) & ~1LL;
         if ((double)n * ldk * sizeof(double) > kPlanMaxBytes) return;
@@ -370,7 +371,8 @@ struct PlanCgLaunch {
         p.red = buf.get();
         p.zbuf = p.red + 8 * (size_t)blocks;
         p.count = reinterpret_cast<unsigned*>(p.zbuf + ldk);
-        p.err = err;
+        p.err = &S->err;
+        p.polls = grid_polls();
         p.st = S;
         ok = true;
     }

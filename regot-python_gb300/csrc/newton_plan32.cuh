@@ -45,7 +45,8 @@ struct PlanCg32Params {
     float *rowpart, *colpart;
     double *parts_a, *parts_b;  // sums of the 32-item and (two) of the 64-item groups
     unsigned* count;
-    int* err;
+    int* err;        // set when a barrier gives up
+    unsigned polls;  // before it does
     NewtonState* st;
 };
 
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_plan_cg32(const PlanCg32Para
     double* s_x = s_p + Im;
     double* s_r = s_x + Im;
     double* s_z = s_r + Im;
-    GridBarrier<CLUSTER> bar(p.count, p.err, &s_ok);
+    GridBarrier<CLUSTER> bar(p.count, p.err, p.polls, &s_ok);
     auto group_sync = [&]() {
         asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GT) : "memory");
     };
@@ -542,7 +543,8 @@ struct PlanCg32 {
         p.count = reinterpret_cast<unsigned*>(p.parts_a + cdiv(n, 32) + cdiv(m, 32));
         p.rowpart = reinterpret_cast<float*>(ops.buf().rowpart.get());
         p.colpart = reinterpret_cast<float*>(ops.buf().colpart.get());
-        p.err = ops.err_flag();
+        p.err = &S->err;
+        p.polls = grid_polls();
         p.st = S;
         ok = true;
     }

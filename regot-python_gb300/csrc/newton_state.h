@@ -7,6 +7,7 @@ struct NewtonState {
     int cg_done;
     int cg_it;
     int cg_max;
+    int err;  // a barrier of a resident kernel gave up
     unsigned counter;
     double rz;       // r' z of the current CG residual
     double alpha;    // CG step

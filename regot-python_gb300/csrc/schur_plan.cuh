@@ -29,7 +29,8 @@ struct SchurCgParams {
     double* zbuf;            // [m - 1]
     double* red;             // [2][G][2]
     unsigned* count;
-    int* err;
+    int* err;        // set when a barrier gives up
+    unsigned polls;  // before it does
     SsnState* st;
 };
 
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_schur_cg(const SchurCgParams
     double* s_z = s_r + Cm;
     double* s_c = s_z + Cm;   // column products
     double* s_v = s_c + Cm;   // [2][kResWarps]
-    GridBarrier<CLUSTER> bar(p.count, p.err, &s_ok);
+    GridBarrier<CLUSTER> bar(p.count, p.err, p.polls, &s_ok);
     const int items = R > C ? R : C;
     const int iwarps = (items + 31) / 32 < kResWarps ? (items + 31) / 32 : kResWarps;
     const double shift = p.shift, inv_reg = S.inv_reg;
@@ -313,7 +314,7 @@ struct SchurCg {
     DBuf<double> buf;
     SchurCgParams p{};
 
-    void init(const Sparse& S, SsnState* st, int* err, cudaStream_t stream) {
+    void init(const Sparse& S, SsnState* st, cudaStream_t stream) {
         if (S.m1 <= 0) return;
         blocks = 16;
         smem = schur_cg_smem(S.n, S.m1, blocks);
@@ -331,7 +332,8 @@ struct SchurCg {
         p.wbuf = p.ubuf + nn;
         p.zbuf = p.wbuf + nn;
         p.count = reinterpret_cast<unsigned*>(p.zbuf + mm);
-        p.err = err;
+        p.err = &st->err;
+        p.polls = grid_polls();
         p.st = st;
         ok = true;
     }
