@@ -458,7 +458,9 @@ long long regot_set_wait_limit(long long spins);
 /* ---- Autotuner of the dense passes (no counterpart in the reference,
  * whose passes are fixed Eigen loops, e.g. src/sinkhorn_problem_bcd.cpp:82-146
  * and src/sinkhorn_problem_obj.cpp:16-136) ----
- * Every dense pass has two launch configurations with the same tile shape:
+ * FP64 passes over up to 2^24 entries have tiles and a configuration of their
+ * own (2), which is neither tuned nor forced: regot_autotune does nothing there.
+ * Every other dense pass has two launch configurations with the same tile shape:
  * 0 = two CTAs per SM (128 registers a thread) with a 4-deep ring of row
  * buffers per warp, 1 = one CTA per SM (255 registers) with an 8-deep ring.
  * regot_autotune times every pass kind under both on a synthetic n x m
@@ -477,11 +479,12 @@ void regot_autotune_clear(void);
  * pass, size class, configuration, microseconds of each configuration);
  * copies at most len - 1 bytes and returns the full length. */
 size_t regot_autotune_entries(char* buf, size_t len);
-/* Force configuration cfg (0 or 1) for every pass; -1 restores the tuned
- * choices. Returns the previous forced value. */
+/* Force configuration cfg (0 or 1) for every pass that has the choice; -1
+ * restores the tuned choices. Returns the previous forced value. */
 int regot_force_pass_config(int cfg);
 /* The configuration a pass of `kind` (REGOT_PASS_*) would use now for an
- * n x m problem of `precision`; -1 on error. */
+ * n x m problem of `precision` (0 or 1, or 2 for FP64 up to 2^24 entries); -1
+ * on error. */
 int regot_pass_config(regot_ctx* ctx, int kind, int precision, int n, int m);
 
 /* ---- Allocation-free variant ----

@@ -882,6 +882,7 @@ extern "C" int regot_autotune(regot_ctx* ctx, int n, int m, int precision, int r
         require(reps > 0, "reps must be positive");
     });
     if (rc != REGOT_OK) return rc;
+    if (precision == REGOT_PREC_FP64 && tile_rows<double>(n, m) == kSmallRB) return rc;
     // A synthetic problem of the size: M uniform on [0, 1), uniform marginals.
     std::vector<float> M((size_t)n * m);
     unsigned long long x = 0x9E3779B97F4A7C15ULL;

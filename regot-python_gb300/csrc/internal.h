@@ -175,10 +175,11 @@ template <typename TM, int CFG>
 void launch_pass_cfg(int op, const PassParams& p, cudaStream_t st, int blocks);
 template <typename TM, int CFG>
 int occupancy_cfg(int op);
-// The configuration the passes use for (op, precision, n, m): a forced
-// choice (tests, the tuner), else the tuned one, else 0.
+// The configuration the passes use for (op, precision, n, m): kSmallCfg for FP64
+// problems of the small tiles, else a forced choice (tests, the tuner), else the
+// tuned one, else 0.
 int pass_config(int op, bool mixed, int n, int m);
-// Force one configuration for every pass (-1: back to the tuned choices);
+// Force one configuration for every pass that has the choice (-1: back to the tuned choices);
 // returns the previous forced value.
 int force_pass_config(int cfg);
 // The autotuner's table (passes.cu): record a measured choice for the
@@ -204,9 +205,10 @@ int pass_blocks(int op, bool mixed, int n, int m);
 // last round; beyond, their four times as many column partials (1/16 of M's
 // memory a sum) buy nothing. FP32 passes of small problems are bound by
 // latencies instead.
+constexpr long long kSmallEntries = 1LL << 24;
 template <typename TM>
 inline int tile_rows(int n, int m) {
-    return sizeof(TM) == 8 && (long long)n * m <= (1LL << 24) ? kSmallRB : kRB;
+    return sizeof(TM) == 8 && (long long)n * m <= kSmallEntries ? kSmallRB : kRB;
 }
 
 template <typename TM>

@@ -62,7 +62,10 @@ __global__ void k_split(const PassParams p, float4* rs, float4* cs, float* cds) 
 // Choices keyed by (device name, precision, pass, size class): the size
 // class of an n x m pass is floor(log2(n m)). A lookup without an entry for
 // its class takes the nearest tuned class of the same pass within two
-// classes, else configuration 0.
+// classes, else configuration 0. FP64 problems of the small tiles (tile_rows)
+// have one configuration: nothing is recorded for them, and a table's FP64
+// entries for the classes below kSmallEntries are passed over, as the passes
+// they were timed on no longer run there.
 struct TuneKey {
     std::string device;
     int mixed, op, bucket;
@@ -179,7 +182,8 @@ int force_pass_config(int cfg) {
     return g_force_cfg.exchange(cfg >= 0 && cfg < kPassConfigs ? cfg : -1);
 }
 
-int pass_config(int op, bool mixed, int n, int m) {
+// The tuned (or forced) choice among the kPassConfigs configurations.
+static int tuned_config(int op, bool mixed, int n, int m) {
     const int forced = g_force_cfg.load(std::memory_order_relaxed);
     if (forced >= 0) return forced;
     ensure_loaded();
@@ -195,11 +199,18 @@ int pass_config(int op, bool mixed, int n, int m) {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     for (int d = 0; d <= 2; ++d)
         for (int sgn = -1; sgn <= 1; sgn += 2) {
-            auto it = g_tune.find(TuneKey{dev_name, mixed ? 1 : 0, op, b + sgn * d});
-            if (it != g_tune.end()) return it->second.cfg;
+            const int c = b + sgn * d;
+            auto it = g_tune.find(TuneKey{dev_name, mixed ? 1 : 0, op, c});
+            if (it != g_tune.end() && (mixed || (1LL << c) >= kSmallEntries))
+                return it->second.cfg;
             if (d == 0) break;
         }
     return 0;
+}
+
+int pass_config(int op, bool mixed, int n, int m) {
+    if (!mixed && tile_rows<double>(n, m) == kSmallRB) return kSmallCfg;
+    return tuned_config(op, mixed, n, m);
 }
 
 void record_tuning(int op, bool mixed, int n, int m, int cfg, const double* us) {
@@ -273,12 +284,6 @@ int occupancy(int op, bool mixed, int cfg) {
     return occ;
 }
 
-// The configuration a pass runs in: the tuned one, or that of the small FP64 tiles.
-int run_config(int op, bool mixed, int n, int m) {
-    if (!mixed && tile_rows<double>(n, m) == kSmallRB) return kSmallCfg;
-    return pass_config(op, mixed, n, m);
-}
-
 int blocks_for(int op, bool mixed, int n, int m, int cfg) {
     const PassShape s = mixed ? pass_shape<float>(n, m) : pass_shape<double>(n, m);
     const int cap = device_sm_count() * occupancy(op, mixed, cfg);
@@ -297,7 +302,7 @@ void launch_pass(int op, const PassParams& p, cudaStream_t st) {
     q.inv_reg_d = 1.0 / p.reg;
     q.wait_limit = wait_limit();
     constexpr bool mixed = std::is_same<TM, float>::value;
-    const int cfg = run_config(op, mixed, p.n, p.m);
+    const int cfg = pass_config(op, mixed, p.n, p.m);
     const int blocks = blocks_for(op, mixed, p.n, p.m, cfg);
     if constexpr (!mixed) {
         if (cfg == kSmallCfg) {
@@ -310,7 +315,7 @@ void launch_pass(int op, const PassParams& p, cudaStream_t st) {
 }
 
 int pass_blocks(int op, bool mixed, int n, int m) {
-    return blocks_for(op, mixed, n, m, run_config(op, mixed, n, m));
+    return blocks_for(op, mixed, n, m, pass_config(op, mixed, n, m));
 }
 
 void launch_split(const PassParams& p, float4* rs, float4* cs, float* cds, cudaStream_t st) {
