@@ -454,6 +454,12 @@ long long regot_pass_bytes(regot_dproblem* prob, int kind);
  * Process-wide; for exercising the timeout path. No counterpart in the
  * reference. */
 long long regot_set_wait_limit(long long spins);
+/* Makes the k-th device allocation from now fail as if the memory were used up
+ * (k <= 0: none). Returns how many were still to come before the failing one of
+ * the call before (0: it has failed, or none was set). Process-wide; for
+ * exercising the out-of-memory paths without filling a GPU. No counterpart in
+ * the reference. */
+long long regot_fail_allocation(long long k);
 
 /* ---- Autotuner of the dense passes (no counterpart in the reference,
  * whose passes are fixed Eigen loops, e.g. src/sinkhorn_problem_bcd.cpp:82-146

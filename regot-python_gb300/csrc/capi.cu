@@ -5,6 +5,7 @@
 #include <sys/stat.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
@@ -102,7 +103,11 @@ namespace regot {
 static std::mutex g_pool_mutex;
 static std::unordered_map<int, cudaMemPool_t> g_pools;  // per device, kept for the process
 
+static std::atomic<long long> g_fail_alloc{0};  // allocations up to the one that fails
+
 void* dev_alloc(size_t bytes, cudaStream_t st) {
+    if (g_fail_alloc.load(std::memory_order_relaxed) > 0 && g_fail_alloc.fetch_sub(1) == 1)
+        throw Error(REGOT_ERR_CUDA, "out of memory (regot_fail_allocation)");
     int dev = 0;
     REGOT_CUDA(cudaGetDevice(&dev));
     cudaMemPool_t pool = nullptr;
@@ -824,6 +829,10 @@ static void drop_time_pass_state(regot_dproblem* P) {
 }
 
 extern "C" long long regot_set_wait_limit(long long spins) { return set_wait_limit(spins); }
+
+extern "C" long long regot_fail_allocation(long long k) {
+    return std::max(0LL, g_fail_alloc.exchange(std::max(0LL, k)));
+}
 
 extern "C" int regot_force_pass_config(int cfg) { return force_pass_config(cfg); }
 

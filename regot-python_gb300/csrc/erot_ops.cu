@@ -177,8 +177,9 @@ void launch_plan64(const double* M, long long ldm, int n, int m, const double* a
 ErotOps::ErotOps(regot_dproblem* P, double reg, cudaStream_t st)
     : P_(P), st_(st), n_(P->n), m_(P->m), mixed_(P->prec == REGOT_PREC_MIXED), reg_(reg) {
     if (!P->loga) {  // once per problem, kept with it
+        // both or none: a problem with one of them would be taken for complete
+        if (!P->logb) P->logb = static_cast<double*>(dev_alloc(m_ * sizeof(double), st_));
         P->loga = static_cast<double*>(dev_alloc(n_ * sizeof(double), st_));
-        P->logb = static_cast<double*>(dev_alloc(m_ * sizeof(double), st_));
         k_log<<<cdiv(n_, 256), 256, 0, st_>>>(P->a, n_, P->loga);
         k_log<<<cdiv(m_, 256), 256, 0, st_>>>(P->b, m_, P->logb);
         count_launch(2);

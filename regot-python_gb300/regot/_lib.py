@@ -149,7 +149,7 @@ EXPORTS = [
     "regot_qrot_dual_obj_grad",
     "regot_qrot_optimal_beta",
     "regot_qrot_primal_val", "regot_qrot_plan", "regot_time_pass", "regot_pass_bytes",
-    "regot_set_wait_limit", "regot_autotune", "regot_autotune_save", "regot_autotune_load",
+    "regot_set_wait_limit", "regot_fail_allocation", "regot_autotune", "regot_autotune_save", "regot_autotune_load",
     "regot_autotune_clear", "regot_autotune_entries", "regot_force_pass_config",
     "regot_pass_config", "regot_force_batch_variant", "regot_batch_variants",
     "regot_force_sparsify_path",
@@ -220,6 +220,8 @@ def load() -> C.CDLL:
         lib.regot_pass_bytes.restype = C.c_longlong
         lib.regot_set_wait_limit.argtypes = [C.c_longlong]
         lib.regot_set_wait_limit.restype = C.c_longlong
+        lib.regot_fail_allocation.argtypes = [C.c_longlong]
+        lib.regot_fail_allocation.restype = C.c_longlong
         lib.regot_autotune.argtypes = [vp, C.c_int, C.c_int, C.c_int, C.c_int]
         lib.regot_autotune_save.argtypes = [C.c_char_p]
         lib.regot_autotune_load.argtypes = [C.c_char_p]
