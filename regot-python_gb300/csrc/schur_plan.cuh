@@ -325,7 +325,12 @@ struct SchurCg {
             if (!resident_grid(k_schur_cg<false>, smem)) return;
         }
         const size_t nn = ((size_t)S.n + 1) & ~(size_t)1, mm = ((size_t)S.m1 + 1) & ~(size_t)1;
-        buf.alloc(4 * (size_t)blocks + 2 * nn + mm + 2, stream);
+        try {
+            buf.alloc(4 * (size_t)blocks + 2 * nn + mm + 2, stream);
+        } catch (const Error&) {  // no room: the captured steps
+            cudaGetLastError();
+            return;
+        }
         p.S = S;
         p.red = buf.get();  // first: read in pairs
         p.ubuf = p.red + 4 * (size_t)blocks;

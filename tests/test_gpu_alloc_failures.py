@@ -47,12 +47,12 @@ def _scan(make, solve, check):
 
 # problem, solver, its options, how far results may be off, fallbacks at least
 ENTROPIC = [
-    # a matrix (K or T) and its buffers
+    # a matrix (K or T) and its buffers; of SSNS also those of the Schur CG
     ("points", "fp64", "sinkhorn_bcd", dict(reg=0.05, tol=1e-9, max_iter=400), 1e-8, 3),
     ("readme", "fp64", "sinkhorn_bcd", dict(reg=0.05, tol=1e-9, max_iter=3000, x0=DEAD), 1e-7, 3),
     ("points", "fp64", "sinkhorn_newton", dict(reg=0.05, tol=1e-9, max_iter=50), 1e-8, 4),
     ("points", "mixed", "sinkhorn_newton", dict(reg=0.05, tol=1e-6, max_iter=50), 1e-4, 2),
-    ("points", "fp64", "sinkhorn_ssns", dict(reg=0.05, tol=1e-9, max_iter=200), 1e-7, 4),
+    ("points", "fp64", "sinkhorn_ssns", dict(reg=0.05, tol=1e-9, max_iter=200), 1e-7, 5),
     ("points", "mixed", "sinkhorn_bcd", dict(reg=0.05, tol=1e-6, max_iter=400), 1e-4, 0),
 ]
 
