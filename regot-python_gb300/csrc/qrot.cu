@@ -2590,6 +2590,16 @@ struct SideStream {
     }
 };
 
+// An engine on stream s beside another, or null where there is no room for one.
+std::unique_ptr<QrotEngine> second_engine(regot_dproblem* P, double reg, cudaStream_t s) {
+    try {
+        return std::unique_ptr<QrotEngine>(new QrotEngine(P, reg, 0.0, s));
+    } catch (const Error&) {
+        cudaGetLastError();
+        return nullptr;
+    }
+}
+
 // The host side of the pair ring: Gram matrices of the stored pairs in ring
 // slots (logical order of BFGSMat), s'y of each, theta, and the maps of the
 // device buffers.
@@ -2891,7 +2901,8 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
     // neither the iterate it starts from nor that iterate's max and row
     // scalings; what it may overwrite belongs to the iterate before, whose
     // primal value `st` therefore waits for. So the value of iterate q is
-    // complete once the line search from q + 1 has been waited for.
+    // complete once the line search from q + 1 has been waited for. Without room
+    // for a second engine they run on `st` in between, where that holds as well.
     struct PrimSlots {
         PrimRaw s[2];
     };
@@ -2902,19 +2913,21 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
         side.create();
         REGOT_CUDA(cudaEventRecord(side.done[0], st));
         REGOT_CUDA(cudaStreamWaitEvent(side.s, side.done[0], 0));
-        EP.reset(new QrotEngine(P, reg, 0.0, side.s));
+        EP = second_engine(P, reg, side.s);
     }
     auto prim_read = [&](int q) {
-        if (q >= 0) hprim[q] = EP->primal_value(pslots.p->s[q & 1]);
+        if (q >= 0) hprim[q] = E.primal_value(pslots.p->s[q & 1]);
     };
     auto iterate = [&](int xi, int gi, double gnorm) {
         stamp();
         if (o.prim_vals) {
             prim_read(it - 2);
             // the caller has synchronised st: x, its max and row scalings are there
-            EP->primal_launch(xbuf(xi), xmax.get() + xi, &pslots.p->s[it & 1], xrbuf(gi));
-            REGOT_CUDA(cudaEventRecord(side.done[it & 1], side.s));
-            if (it > 0) REGOT_CUDA(cudaStreamWaitEvent(st, side.done[(it - 1) & 1], 0));
+            (EP ? *EP : E).primal_launch(xbuf(xi), xmax.get() + xi, &pslots.p->s[it & 1], xrbuf(gi));
+            if (EP) {
+                REGOT_CUDA(cudaEventRecord(side.done[it & 1], side.s));
+                if (it > 0) REGOT_CUDA(cudaStreamWaitEvent(st, side.done[(it - 1) & 1], 0));
+            }
         }
         hobj.push_back(last_obj);
         hmar.push_back(gnorm / reg);
@@ -3116,10 +3129,12 @@ void qrot_lbfgs_dual_device(regot_ctx* ctx, regot_dproblem* P, double reg, doubl
     std::vector<unsigned long long> hst(nstamp);
     d2h(hst.data(), stamps.get(), nstamp * sizeof(unsigned long long), st);
     sync(st);
-    if (EP) {
+    if (o.prim_vals) {
         sync(side.s);
         prim_read(it - 2);
         prim_read(it - 1);
+    }
+    if (EP) {
         EP->ops().check_err();
         E.add_passes(EP->passes());
     }
@@ -3239,7 +3254,8 @@ namespace {
 
 // Primal values on a stream and an engine of their own, beside the next Newton
 // system (whose CG runs on 16 SMs): at each launch the point of the last eval()
-// and its row scalings are copied, then the passes run at their own pace.
+// and its row scalings are copied, then the passes run at their own pace. Without
+// room for a second engine the passes run on the main stream, by the main engine.
 class SidePrimal {
 public:
     SidePrimal(regot_dproblem* P, double reg, cudaStream_t main) : main_(main) {
@@ -3247,8 +3263,14 @@ public:
         REGOT_CUDA(cudaEventCreateWithFlags(&copied_.e, cudaEventDisableTiming));
         REGOT_CUDA(cudaEventRecord(copied_.e, main_));
         REGOT_CUDA(cudaStreamWaitEvent(side_.s, copied_.e, 0));
-        x_.alloc(P->n, side_.s);
-        E_.reset(new QrotEngine(P, reg, 0.0, side_.s));
+        E_ = second_engine(P, reg, side_.s);
+        if (!E_) return;
+        try {
+            x_.alloc(P->n, side_.s);
+        } catch (const Error&) {
+            cudaGetLastError();
+            E_.reset();
+        }
     }
     // Appends the value at the point of E's last eval() to out, where it arrives
     // by finish() at the latest. The caller has synchronised the main stream.
@@ -3256,9 +3278,14 @@ public:
         const int q = (int)out.size();
         if (q >= 2) {
             REGOT_CUDA(cudaEventSynchronize(side_.done[q & 1]));
-            out[q - 2] = E_->primal_value(slots_.p->s[q & 1]);
+            out[q - 2] = E.primal_value(slots_.p->s[q & 1]);
         }
         out.push_back(0.0);
+        if (!E_) {
+            E.primal_launch(E.gamma(), nullptr, &slots_.p->s[q & 1], E.row_scalings());
+            REGOT_CUDA(cudaEventRecord(side_.done[q & 1], main_));
+            return;
+        }
         const size_t n = E.n(), N = n + E.m();
         d2d(E_->gamma(), E.gamma(), N * sizeof(double), side_.s);
         d2d(x_.get(), E.row_scalings(), n * sizeof(double), side_.s);
@@ -3268,9 +3295,10 @@ public:
         REGOT_CUDA(cudaEventRecord(side_.done[q & 1], side_.s));
     }
     void finish(QrotEngine& E, std::vector<double>& out) {
-        sync(side_.s);
+        sync(E_ ? side_.s : main_);
         const int L = (int)out.size();
-        for (int q = L > 1 ? L - 2 : 0; q < L; ++q) out[q] = E_->primal_value(slots_.p->s[q & 1]);
+        for (int q = L > 1 ? L - 2 : 0; q < L; ++q) out[q] = E.primal_value(slots_.p->s[q & 1]);
+        if (!E_) return;
         E_->ops().check_err();
         E.add_passes(E_->passes());
     }

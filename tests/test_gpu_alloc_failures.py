@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import regot_oracle as O
-from problems import erot_points, readme_example
+from problems import erot_points, qrot_points, readme_example
 
 pytestmark = pytest.mark.gpu
 
@@ -78,3 +78,24 @@ def test_entropic_solves(problem, precision, solver, options, atol, fallbacks):
     outcomes = _scan(lambda: regot.Problem(M, a, b, precision=precision),
                      lambda P: getattr(P, solver)(**options), check)
     assert sum(outcomes) >= fallbacks and outcomes.count(False) >= 5
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("solver", ["qrot_lbfgs_dual", "qrot_assn", "qrot_grssn"])
+def test_quadratic_solves(solver, precision):
+    # the primal values' second engine is left out where it has no room: the same
+    # kernels then run one after another, so every value has the same bits
+    M, a, b = qrot_points(150, 130, seed=2)
+    P = regot.Problem(M, a, b, precision=precision)
+    want = getattr(P, solver)(0.1, tol=1e-6, max_iter=8)
+    P.close()
+    assert len(want.prim_vals) >= 4
+
+    def check(r):
+        assert np.array_equal(r.prim_vals, want.prim_vals)
+        assert np.array_equal(r.obj_vals, want.obj_vals)
+        assert np.array_equal(r.dual, want.dual)
+
+    outcomes = _scan(lambda: regot.Problem(M, a, b, precision=precision),
+                     lambda P: getattr(P, solver)(0.1, tol=1e-6, max_iter=8), check)
+    assert sum(outcomes) >= 5 and outcomes.count(False) >= 5
