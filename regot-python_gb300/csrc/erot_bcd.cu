@@ -691,6 +691,10 @@ void sinkhorn_bcd_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double tol,
         cudaGraphDestroy(graph);
     }
     const long long passes = 2LL * hs.hist_len;
+    // the plan's output may need their room
+    K.release();
+    spart.release();
+    sbuf.release();
 
     // Results: gauge-fixed dual, plan, histories.
     DBuf<double> gamma(n + m, st);

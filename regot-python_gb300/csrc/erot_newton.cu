@@ -376,6 +376,7 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
             long long np = 0;
             newton_on_plan(ctx, P, ops, L, tol, max_iter, cg_tol, gamma.get(), o, hist.get(),
                            hist_cap, parts.get(), S, &niter, &len, &np);
+            L.release();
             finish_erot_result(ops, gamma.get(), hobj, hmar, htime, nullptr, len, hist_cap, niter, np,
                                o, res);
             return;
@@ -552,6 +553,7 @@ void sinkhorn_newton_gpu(regot_ctx* ctx, regot_dproblem* P, double reg, double t
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
+    L32.release();
     finish_erot_result(ops, gamma.get(), hobj, hmar, htime, nullptr, hist_len, hist_cap, i,
                        passes, o, res);
 }

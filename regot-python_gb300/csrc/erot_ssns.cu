@@ -1720,6 +1720,9 @@ public:
     SsnState* state() { return state_.get(); }
     long long passes() const { return passes_; }
 
+    // Gives the stored plan's memory back, for the plan's output.
+    void release_plan() { plan_.release(); }
+
     SsnState read_state() {
         SsnState hs;
         read_small(P_->ctx, &hs, state_.get(), sizeof(hs), st_);
@@ -2281,6 +2284,7 @@ void run_ssns(regot_ctx* ctx, regot_dproblem* P, double reg, double tol, int max
     h2d(hist.get() + L, hmar.data(), L * sizeof(double), st);
     h2d(hist.get() + 2 * L, htime.data(), L * sizeof(double), st);
     h2d(hist.get() + 3 * L, hdens.data(), L * sizeof(double), st);
+    E.release_plan();
     finish_erot_result(ops, E.gamma(), hist.get(), hist.get() + L, hist.get() + 2 * L,
                        hist.get() + 3 * L, L, L, i, E.passes(), o, res);
 }
@@ -2458,6 +2462,7 @@ void run_sparse_newton(regot_ctx* ctx, regot_dproblem* P, double reg, double tol
     h2d(hist.get() + L, hmar.data(), L * sizeof(double), st);
     h2d(hist.get() + 2 * L, htime.data(), L * sizeof(double), st);
     h2d(hist.get() + 3 * L, hdens.data(), L * sizeof(double), st);
+    E.release_plan();
     finish_erot_result(ops, E.gamma(), hist.get(), hist.get() + L, hist.get() + 2 * L,
                        hist.get() + 3 * L, L, L, i, E.passes(), o, res);
 }

@@ -376,6 +376,12 @@ struct PlanCgLaunch {
         p.st = S;
         ok = true;
     }
+    // Gives the memory back, for the plan's output; nothing can be solved any more.
+    void release() {
+        T.release();
+        part.release();
+        ok = false;
+    }
     // Blocks of the line search: at most eight an SM, with the items dealt out
     // evenly over their rounds.
     int ls_blocks() const {

@@ -548,6 +548,11 @@ struct PlanCg32 {
         p.st = S;
         ok = true;
     }
+    // Gives the memory back, for the plan's output; nothing can be solved any more.
+    void release() {
+        T.release();
+        ok = false;
+    }
     // H x = sign rhs at the duals split in rs, cs (H's diagonal given).
     void solve(const float4* rs, const float4* cs, const double* rhs, double sign,
                const double* hdiag, double tol, double* x, cudaStream_t st) {
