@@ -414,6 +414,28 @@ inline double largest_square_below(double tol) {
     return std::sqrt(x) < tol ? x : -1.0;
 }
 
+// part[k] += block_parts[b][k] over the blocks b = lane, lane + 32, ... in order, U
+// rounds of loads under way together.
+template <int K, unsigned U>
+__device__ __forceinline__ void gather_parts(const double* block_parts, unsigned blocks, int lane,
+                                             double (&part)[K]) {
+    for (unsigned b = lane; b < blocks; b += 32 * U) {
+        double v[U][K];
+#pragma unroll
+        for (unsigned u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                v[u][k] = b + 32 * u < blocks ? __ldcg(&block_parts[(size_t)(b + 32 * u) * K + k]) : 0.0;
+#pragma unroll
+        for (unsigned u = 0; u < U; ++u) {
+            if (b + 32 * u < blocks) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) part[k] += v[u][k];
+            }
+        }
+    }
+}
+
 // Grid-wide sum of K values when one full warp of each of the grid's first
 // `blocks` blocks (0: all) holds them (the other warps take no part). Returns true in every lane of that
 // warp of the last block to finish, with the totals in out[]. The last warp
@@ -442,23 +464,15 @@ __device__ bool warp_grid_reduce(const double (&vals)[K], double* block_parts, u
 #pragma unroll
     for (int k = 0; k < K; ++k) part[k] = 0.0;
     // up to 24 loads a lane under way together: one after another, the sums of
-    // 256 blocks took eight L2 latencies
-    constexpr unsigned U = K <= 3 ? 8 : 4;
-    for (unsigned b = lane; b < blocks; b += 32 * U) {
-        double v[U][K];
-#pragma unroll
-        for (unsigned u = 0; u < U; ++u)
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                v[u][k] = b + 32 * u < blocks ? __ldcg(&block_parts[(size_t)(b + 32 * u) * K + k]) : 0.0;
-#pragma unroll
-        for (unsigned u = 0; u < U; ++u) {
-            if (b + 32 * u < blocks) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) part[k] += v[u][k];
-            }
-        }
-    }
+    // 256 blocks took eight L2 latencies. Grids of up to 32 and 64 blocks (1024 and
+    // 2048 rows or columns) have rounds of their own size: an FP64 addition that no
+    // lane takes part in still holds its place, and the seven rounds too many cost
+    // mixed BCD 811 against 781 us at 300 x 260 (22 sweeps), 765 against 741 at
+    // 1000 x 800. From 65 blocks on the large rounds are the faster ones (a break
+    // between the additions cost 7 % at 8192 x 300).
+    if (blocks <= 32) gather_parts<K, 1>(block_parts, blocks, lane, part);
+    else if (blocks <= 64) gather_parts<K, 2>(block_parts, blocks, lane, part);
+    else gather_parts<K, (K <= 3 ? 8 : 4)>(block_parts, blocks, lane, part);
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < K; ++k) out[k] = warp_sum_d(part[k]);
