@@ -277,8 +277,13 @@ __device__ __forceinline__ void merge_columns(const double* part, long long ldk,
 
 // ---- launches: one cluster of 16 blocks for small problems, else a block an SM ----
 
-// Problems of at most this many entries run in one cluster.
-constexpr long long kClusterEntries = 64 * 1024;
+// Problems of at most this many entries run in one cluster: its barrier takes a
+// third of the grid's, its 16 SMs nine times the products. FP64, cluster against
+// grid, us (sinkhorn_bcd / newton / ssns): 64 x 64 508 / 3210 / 1642 against 570 /
+// 3457 / 1760, 128 x 128 500 / 3750 / 1778 against 490 / 3689 / 1845, 160 x 150
+// 500 / 3735 / 1824 against 500 / 3798 / 1837, 250 x 250 508 / 4456 / 2036 against
+// 413 / 3956 / 1837.
+constexpr long long kClusterEntries = 24 * 1024;
 // A stored plan doubles the memory of the cost matrix; beyond this size the
 // solvers keep to the dense passes.
 constexpr double kPlanMaxBytes = 32.0 * (1ULL << 30);

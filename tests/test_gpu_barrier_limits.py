@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 regot = pytest.importorskip("regot")
 from regot import _lib  # noqa: E402
 
-N, M = 300, 260  # more than 65536 entries: a block on every SM, not one cluster
+N, M = 300, 260  # a block on every SM, not one cluster
 
 
 @pytest.fixture

@@ -1,7 +1,8 @@
 """The resident kernels' records and results do not depend on which warp or
 block is first: the same bits from run to run, and the oracle's values, at
 shapes whose products need no barrier of the block of their own (one cluster
-of 16 blocks, wide matrices) and at shapes with a block on every SM."""
+of 16 blocks up to 24576 entries, wide matrices) and at shapes with a block on
+every SM."""
 import numpy as np
 import pytest
 
@@ -13,8 +14,8 @@ pytestmark = pytest.mark.gpu
 regot = pytest.importorskip("regot")
 
 
-@pytest.mark.parametrize("n,m", [(80, 700), (15, 4000), (60, 1024), (9, 513)])
-def test_bcd_records_in_one_cluster(n, m):
+@pytest.mark.parametrize("n,m", [(35, 700), (6, 4000), (20, 1024), (9, 513), (15, 4000)])
+def test_bcd_records(n, m):
     # errors of z = (alpha + beta - M) / reg as in test_gpu_bcd_scaled.py
     M, a, b = erot_points(n, m, seed=n, dtype=np.float64)
     o = O.sinkhorn_bcd(M, a, b, 0.05, tol=1e-13, max_iter=40)
@@ -30,7 +31,7 @@ def test_bcd_records_in_one_cluster(n, m):
     P.close()
 
 
-@pytest.mark.parametrize("n,m", [(40, 30), (90, 700), (300, 260), (1000, 803)])
+@pytest.mark.parametrize("n,m", [(40, 30), (30, 700), (128, 192), (193, 128), (300, 260), (1000, 803)])
 def test_newton_is_the_same_from_run_to_run(n, m):
     M, a, b = erot_points(n, m, seed=m, dtype=np.float64)
     P = regot.Problem(M, a, b, precision="fp64")
@@ -68,3 +69,15 @@ def test_first_record_from_a_dual_off_the_split_grid(n, m, reg):
         assert np.array_equal(r.obj_vals, first.obj_vals)
         assert np.array_equal(r.dual, first.dual)
     P.close()
+
+
+@pytest.mark.parametrize("n,m", [(128, 192), (193, 128), (24576, 1), (1, 24577), (24577, 1)])
+def test_the_edge_of_one_cluster(n, m):
+    # 24576 entries run in one cluster, more in a block an SM (errors as above)
+    M, a, b = erot_points(n, m, seed=7, dtype=np.float64)
+    o = O.sinkhorn_bcd(M, a, b, 0.05, tol=1e-13, max_iter=20)
+    r = regot.sinkhorn_bcd(M, a, b, 0.05, tol=1e-13, max_iter=20)
+    k = min(len(r.obj_vals), len(o.obj_vals))
+    assert abs(r.niter - o.niter) <= 1
+    np.testing.assert_allclose(r.obj_vals[:k], o.obj_vals[:k], rtol=0, atol=1e-12)
+    np.testing.assert_allclose(r.dual, o.dual, rtol=0, atol=1e-11)
