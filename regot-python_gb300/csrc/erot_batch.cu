@@ -1132,8 +1132,12 @@ int tail_cluster_size() {
 // Bodies (pairs of sweeps) of a k_bteam launch of several problems: some
 // milliseconds, against some 40 us for the launch and the reads around it.
 constexpr int kTeamBodies = 16;
-// Problems up to which the tail runs in clusters, where these have the CTAs.
-constexpr int kTailClusters = 4;
+// Problems up to which the tail runs in clusters, where these have the CTAs. Whole
+// calls, clusters against teams, ms: 5 problems of 64 to 500 points 4.81 against
+// 5.89, 6 of 200 to 500 5.90 against 7.27, 7 of 64 to 300 3.71 against 4.23, 8 of 64
+// to 500 3.75 against 3.42, 12 of 64 to 300 4.84 against 4.62, 16 of 64 to 500 7.79
+// against 6.05 (the clusters run in rounds then).
+constexpr int kTailClusters = 7;
 
 // CTAs of k_bteam that the device holds at once, 0 without cooperative launches.
 int team_slots() {
