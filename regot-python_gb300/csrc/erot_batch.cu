@@ -1129,13 +1129,9 @@ int tail_cluster_size() {
     return size;
 }
 
-// Bodies (pairs of sweeps) of a k_bteam launch of several problems, after which
-// those that still run share the CTAs out anew: a launch and the reads around it
-// take some 40 us. Whole calls with 4 / 16 / 64 / 128 bodies and with all, ms: 64
-// problems of 64 to 2048 points 22.5 / 21.0 / 18.9 / 19.6 / 26.7, 24 of 64 to 500
-// - / 5.8 / 5.2 / 4.4 / -, 32 of 64 to 1000 16.7 / 15.7 / 14.6 / 15.1 / 15.0, 16 of
-// 64 to 2048 11.6 / 11.2 / 11.3 / 10.7 / 10.4.
-constexpr int kTeamBodies = 64;
+// Bodies (pairs of sweeps) of a k_bteam launch of several problems: some
+// milliseconds, against some 40 us for the launch and the reads around it.
+constexpr int kTeamBodies = 16;
 // Problems up to which the tail runs in clusters, where these have the CTAs. Whole
 // calls, clusters against teams, ms: 5 problems of 64 to 500 points 4.81 against
 // 5.89, 6 of 200 to 500 5.90 against 7.27, 7 of 64 to 300 3.71 against 4.23, 8 of 64
@@ -1154,8 +1150,7 @@ int team_slots() {
 }
 
 // The teams of the running problems (at most `slots`), CTA by CTA. A sweep in C
-// CTAs takes about a fixed time (barriers, reductions: kFixed points a half; with 94
-// or 1500 instead, thirteen batches of 1 to 64 problems change by less than 0.5 %) and
+// CTAs takes about a fixed time (barriers, reductions: kFixed points a half) and
 // ceil(row blocks / C) m + ceil(column blocks / C) n points a CTA; the CTAs are
 // dealt out to the problem that is slowest by that, as long as one more block
 // less a CTA makes it faster.
