@@ -1130,12 +1130,17 @@ int tail_cluster_size() {
 }
 
 // Bodies (pairs of sweeps) of a k_bteam launch of several problems: some
-// milliseconds, against some 40 us for the launch and the reads around it.
+// milliseconds, against some 40 us for the launch and the reads around it. Whole
+// calls over eight seeds of nine batches of 12 to 200 problems: with 32 bodies 0.97
+// to 1.00 of the time by geometric mean (single seeds 0.92 to 1.03), with 64 0.96 to
+// 1.03 (0.86 to 1.15, the longer the more it hangs on when problems end); all
+// bodies in one launch 26.7 against 21.0 ms for 64 problems of 64 to 2048 points.
 constexpr int kTeamBodies = 16;
 // Problems up to which the tail runs in clusters, where these have the CTAs. Whole
-// calls, clusters against teams, ms: 5 problems of 64 to 500 points 4.81 against
-// 5.89, 6 of 200 to 500 5.90 against 7.27, 7 of 64 to 300 3.71 against 4.23, 8 of 64
-// to 500 3.75 against 3.42, 12 of 64 to 300 4.84 against 4.62, 16 of 64 to 500 7.79
+// calls of batches, with this line instead of four, by geometric mean over eight
+// seeds: 5 problems of 64 to 500 points 0.79 of the time, 6 of 200 to 500 0.79, 7 of
+// 64 to 300 0.86, 10 of 64 to 500 0.96, none of fourteen batches slower. With the
+// line at 16: 8 of 64 to 500 3.77 against 3.43 ms in teams, 16 of 64 to 500 7.79
 // against 6.05 (the clusters run in rounds then).
 constexpr int kTailClusters = 7;
 
@@ -1150,7 +1155,8 @@ int team_slots() {
 }
 
 // The teams of the running problems (at most `slots`), CTA by CTA. A sweep in C
-// CTAs takes about a fixed time (barriers, reductions: kFixed points a half) and
+// CTAs takes about a fixed time (barriers, reductions: kFixed points a half; with 94
+// or 1500 instead, thirteen batches of 1 to 64 problems change by less than 0.5 %) and
 // ceil(row blocks / C) m + ceil(column blocks / C) n points a CTA; the CTAs are
 // dealt out to the problem that is slowest by that, as long as one more block
 // less a CTA makes it faster.
