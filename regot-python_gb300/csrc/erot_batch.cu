@@ -1136,13 +1136,14 @@ int tail_cluster_size() {
 // 1.03 (0.86 to 1.15, the longer the more it hangs on when problems end); all
 // bodies in one launch 26.7 against 21.0 ms for 64 problems of 64 to 2048 points.
 constexpr int kTeamBodies = 16;
-// Problems up to which the tail runs in clusters, where these have the CTAs. Whole
-// calls of batches, with this line instead of four, by geometric mean over eight
-// seeds: 5 problems of 64 to 500 points 0.79 of the time, 6 of 200 to 500 0.79, 7 of
-// 64 to 300 0.86, 10 of 64 to 500 0.96, none of fourteen batches slower. With the
-// line at 16: 8 of 64 to 500 3.77 against 3.43 ms in teams, 16 of 64 to 500 7.79
-// against 6.05 (the clusters run in rounds then).
-constexpr int kTailClusters = 7;
+// Problems up to which the tail runs in clusters, where these have the CTAs (a
+// device holds fourteen such clusters, of 152 SMs). Whole calls of batches, by
+// geometric mean over eight to twelve seeds: a line of 7 instead of 4 takes 0.79 of
+// the time for 5 problems of 64 to 500 points and for 6 of 200 to 500, 0.86 for 7 of
+// 64 to 300; a line of 10 instead of 7 takes 0.94 for 8 of 64 to 500, 0.96 for 10 of
+// 64 to 300, 0.99 for 12 and 14 of up to 500; a line of 14 instead of 10 1.10 for 14
+// of 200 to 500.
+constexpr int kTailClusters = 10;
 
 // CTAs of k_bteam that the device holds at once, 0 without cooperative launches.
 int team_slots() {

@@ -38,7 +38,8 @@ namespace {
 // sums (warp_grid_reduce) need one thread per row or column, and keeping
 // FP64 instructions to that one warp matters on a part whose FP64 rate is a
 // small fraction of its FP32 rate. (In the row finalize warp 1 forms the sums
-// while warp 0 takes the logarithms.)
+// while warp 0 takes the logarithms, and waits for its flags: all in one warp
+// takes 0 to 1.3 % longer a solve, over eight sizes from 100 x 80 to 8192^2.)
 constexpr int kFinItems = 32;
 const dim3 kFinBlock(32, 8);
 

@@ -1,4 +1,4 @@
-"""The batched tail on both sides of its rule (clusters for up to seven problems
+"""The batched tail on both sides of its rule (clusters for up to ten problems
 of at most sixteen blocks, teams of CTAs beyond, several launches of a team) gives
 the bits of the per-sweep kernels."""
 import numpy as np
@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 regot = pytest.importorskip("regot")
 
 
-@pytest.mark.parametrize("count,largest", [(7, 512), (7, 513), (8, 300), (9, 512)])
+@pytest.mark.parametrize("count,largest", [(7, 512), (10, 512), (10, 513), (11, 300)])
 def test_same_bits_as_the_sweep_kernels(count, largest):
     from regot import _lib
 
@@ -17,7 +17,7 @@ def test_same_bits_as_the_sweep_kernels(count, largest):
     rng = np.random.default_rng(count)
     xs, ys, aa, bb = [], [], [], []
     for k in range(count):
-        n, m, d = (largest if k == 0 else 40 + 29 * k), 330 - 31 * k, (2, 3, 8, 16)[k % 4]
+        n, m, d = (largest if k == 0 else 40 + 29 * k), 330 - 28 * k, (2, 3, 8, 16)[k % 4]
         xs.append(rng.standard_normal((n, d), dtype=np.float32))
         ys.append(rng.standard_normal((m, d), dtype=np.float32) + np.float32(0.3))
         aa.append(np.full(n, 1.0 / n))
