@@ -447,7 +447,7 @@ long long regot_pass_bytes(regot_dproblem* prob, int kind);
 /* Limit (polls of about 200 us) of the dense passes' bounded waits on their
  * parameter copies, and (256 polls of about a microsecond for each) of the
  * barriers between the blocks of the kernels that run many sweeps or CG steps
- * in one launch; returns the previous limit, and a negative value
+ * in one launch, these at most under the default; returns the previous limit, and a negative value
  * restores the default (16384). A pass whose wait gives up drains the copy
  * under the default limit, a block whose barrier gives up leaves, and the call
  * returns REGOT_ERR_TIMEOUT; 0 makes every such wait give up at once. (The

@@ -765,16 +765,7 @@ struct GridTeam {
         target += (unsigned)size;
         if (threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-            int ok = 0;
-            for (unsigned s = 0; s < polls; ++s) {
-                unsigned c;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-                if ((int)(c - target) >= 0) {
-                    ok = 1;
-                    break;
-                }
-                if ((s & 1023u) == 1023u && *(volatile int*)&st->err) break;
-            }
+            const bool ok = poll_count(count, target, polls, &st->err);
             if (!ok) atomicOr(&st->err, 2);
             s_ok = ok;
         }
@@ -873,7 +864,7 @@ __global__ void __launch_bounds__(kBWarps * 32, 2) k_bteam(const TailArgs a) {
     const int p = t.x;
     float2* spts = tail_smem;
     float2* spar = tail_smem + kBTile * (kBClassDim[kBClasses - 1] + 1);
-    const GridTeam team{a.count + p, a.st, t.z, 0u, a.polls};
+    const GridTeam team{a.count + p, a.st, t.z, first_target(a.polls), a.polls};
     switch (a.pcls[p]) {
         case 0: tail_solve<4>(a, p, t.y, t.z, team, spts, spar); break;
         case 1: tail_solve<8>(a, p, t.y, t.z, team, spts, spar); break;

@@ -145,7 +145,7 @@ constexpr long long kDefaultWaitSpins = 1LL << 14;
 long long wait_limit();
 long long set_wait_limit(long long spins);
 // Polls (of about a microsecond) of the resident kernels' barriers under the same
-// limit: 2^22, some seconds, by default.
+// limit: 2^22, some seconds, by default and at most.
 unsigned grid_polls();
 // Throws REGOT_ERR_TIMEOUT if the flag of a resident kernel's barriers is set.
 inline void check_barriers(int err) {

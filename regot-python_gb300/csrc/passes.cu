@@ -173,7 +173,9 @@ Exp64 exp64_for(double reg) {
 }
 
 long long wait_limit() { return g_wait_limit.load(std::memory_order_relaxed); }
-unsigned grid_polls() { return (unsigned)std::min<long long>(wait_limit(), 1LL << 22) * 256u; }
+unsigned grid_polls() {
+    return (unsigned)std::min(wait_limit(), kDefaultWaitSpins) * 256u;
+}
 long long set_wait_limit(long long spins) {
     return g_wait_limit.exchange(spins < 0 ? kDefaultWaitSpins : spins);
 }
